@@ -69,6 +69,11 @@ bool ctx_alive(const Ctx *c) {
 
 void Ctx::stage_upload(void *dst, const void *src, size_t bytes) {
   if (!bytes) return;
+  std::memcpy(stage_reserve(bytes), src, bytes);
+  stage_commit(dst, bytes);
+}
+
+char *Ctx::stage_reserve(size_t bytes) {
   const int64_t n = (int64_t)((bytes + 255) & ~size_t(255));
   if ((size_t)n > stage_cap / 2) {
     // grow: wait for every staged copy, then replace the buffer
@@ -101,7 +106,12 @@ void Ctx::stage_upload(void *dst, const void *src, size_t bytes) {
     stage_ev.push_back(stage_q.front().ev);
     stage_q.pop_front();
   }
-  std::memcpy(stage_buf + h % cap, src, bytes);
+  stage_head = h;
+  return stage_buf + h % cap;
+}
+
+void Ctx::stage_commit(void *dst, size_t bytes) {
+  const int64_t h = stage_head, cap = (int64_t)stage_cap;
   launch_stage_copy(this, stage_dev + h % cap, dst, bytes);
   cudaEvent_t ev;
   if (stage_ev.empty()) {
@@ -112,7 +122,19 @@ void Ctx::stage_upload(void *dst, const void *src, size_t bytes) {
   }
   QS_CUDA(cudaEventRecord(ev, stream));
   stage_q.push_back({ev, h});
-  stage_head = h + n;
+  stage_head = h + (int64_t)((bytes + 255) & ~size_t(255));
+}
+
+void DevLists::commit(Ctx *ctx) {
+  ctx_ = ctx;
+  base_ = dev_alloc<char>(ctx, sent_ + scratch_);
+  if (!sent_) return;
+  char *h = ctx->stage_reserve(sent_);
+  for (const Span &s : spans_) {
+    if (s.src) std::memcpy(h + s.off, s.src, s.bytes);
+    else std::memset(h + s.off, 0, s.bytes);
+  }
+  ctx->stage_commit(base_, sent_);
 }
 
 void Ctx::destroy_staging() {

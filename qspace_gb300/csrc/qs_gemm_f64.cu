@@ -71,7 +71,8 @@ __device__ __forceinline__ void panel_fma(typename E::T (&acc)[4][4], const type
 template <bool CPLX>
 __global__ void __launch_bounds__(256)
 gemm_f64_kernel(const PairDesc *__restrict__ pairs, const TileDesc *__restrict__ tiles,
-                const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C) {
+                const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C,
+                const int *__restrict__ flags) {
   using E = Elem<CPLX>;
   using T = typename E::T;
   constexpr int KC = E::KC;
@@ -79,6 +80,7 @@ gemm_f64_kernel(const PairDesc *__restrict__ pairs, const TileDesc *__restrict__
   __shared__ T Bs[KC][TN + 1];
 
   const TileDesc t = tiles[blockIdx.x];
+  if (t.flag >= 0 && !flags[t.flag]) return;  // the tensor-core launch has computed this tile
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
   const int shape = (min(4, (t.M - t.m0 + 15) / 16) - 1) * 4 + (min(4, (t.N - t.n0 + 15) / 16) - 1);
@@ -165,15 +167,17 @@ int gemm_f64_tile_n() { return TN; }
 
 void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles,
                      int64_t ntiles, const double *A, const double *B, double *C,
-                     int is_complex) {
+                     int is_complex, const int *d_flags) {
   if (ntiles <= 0) return;
   if (ntiles > 0x7fffffff) fail(QS_ERR_SHAPE, "gemm_f64: too many tiles");
-  ctx->mark(0);
-  ctx->mark(1);
+  if (!d_flags) {  // else the marks of the tensor-core launch before it stand
+    ctx->mark(0);
+    ctx->mark(1);
+  }
   if (is_complex)
-    gemm_f64_kernel<true><<<(unsigned)ntiles, 256, 0, ctx->stream>>>(d_pairs, d_tiles, A, B, C);
+    gemm_f64_kernel<true><<<(unsigned)ntiles, 256, 0, ctx->stream>>>(d_pairs, d_tiles, A, B, C, d_flags);
   else
-    gemm_f64_kernel<false><<<(unsigned)ntiles, 256, 0, ctx->stream>>>(d_pairs, d_tiles, A, B, C);
+    gemm_f64_kernel<false><<<(unsigned)ntiles, 256, 0, ctx->stream>>>(d_pairs, d_tiles, A, B, C, d_flags);
   QS_LAUNCHED(ctx);
   ctx->mark(2);
 }

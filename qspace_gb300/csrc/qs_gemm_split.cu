@@ -71,6 +71,7 @@ constexpr int A_DIGIT_BYTES = TMS * TKS * 2;  // 8 KB
 constexpr int B_DIGIT_BYTES = TNS * TKS * 2;  // 2 KB
 constexpr int MAX_STAGES = 8;
 constexpr int EMPTY_EXP = -30000;
+constexpr int NONFINITE_EXP = 20000;  // lines with an infinity or NaN (FP64-grade launches)
 constexpr int SMEM_HDR = 2048;   // barriers, TMEM slot, abort flag; tile-descriptor slots at 1024
 constexpr int SMEM_LIMIT = 227 * 1024;
 constexpr uint32_t WAIT_LIMIT = 1u << 22;  // bounded mbarrier polls (seconds)
@@ -110,11 +111,14 @@ struct SplitTile {
   int32_t rshift;          // bits dropped below the lowest group (int64 headroom)
   // output address of tile row r, column j (doubles from c_off):
   // (r >> rsplit) * rs + (r & rsplit) + (j >> csplit) * ldc + (j & csplit),
-  // splits = rsplit | csplit << 1; rsplit = 1 for a complex block computed
-  // transposed in the A-duplicated form (its rows interleave Re/Im of C's
-  // columns), csplit = 1 for one in the B-duplicated form, not transposed
-  // (its columns interleave Re/Im of C's columns)
+  // splits = rsplit | csplit << 1 | swapped << 2 | rdup << 3 | cdup << 4;
+  // rsplit = 1 for a complex block computed transposed in the A-duplicated
+  // form (its rows interleave Re/Im of C's columns), csplit = 1 for one in
+  // the B-duplicated form, not transposed (its columns interleave Re/Im of
+  // C's columns); swapped: the block is computed as C^T; rdup / cdup: two
+  // tile rows / columns per row / column of the computed block
   int32_t rs, splits;
+  int32_t fbase;           // FP64-grade launches: first FP64 tile flag of the block
 };
 constexpr int TILE_WORDS = (int)(sizeof(SplitTile) / 4);
 static_assert(sizeof(SplitTile) % 8 == 0 && TILE_WORDS <= 16, "tile descriptor fits one 64-byte slot");
@@ -295,7 +299,7 @@ constexpr int STRIP_THREADS = 128;
 // Phase 1 for the lines l0 .. l0+nl-1 of op(X) (X = A role: rows, line m at
 // m + k*ld (contig: k + m*ld); X = B role: columns, line n at k + n*ld
 // (contig) or n + k*ld), max over the pairs p0..p1-1 into smax[line].
-template <bool CPLX, bool ROLE_B>
+template <bool CPLX, bool ROLE_B, bool HP>
 __device__ __forceinline__ void strip_maxima(const SplitPair *__restrict__ pairs, const OperandView *views, int p0,
                                              int p1, int l0, int nl, const double *__restrict__ Aarena,
                                              const double *__restrict__ Barena, int *smax) {
@@ -342,23 +346,26 @@ __device__ __forceinline__ void strip_maxima(const SplitPair *__restrict__ pairs
         }
       }
     }
+    // an infinity or NaN: no scale; every tile that reads the line goes to the FP64 kernel
+    if (HP && key == 0x7ff) key = NONFINITE_EXP + 1022 - (ROLE_B ? 0 : P.e_afac);
     if (key) atomicMax(&smax[line], key - 1022 + (ROLE_B ? 0 : P.e_afac));
   }
   __syncthreads();
 }
 
 // A role.  Task = (first pair, end pair, first real row r0 of the strip).
-template <bool CPLX, int S, int B>
+template <bool CPLX, int S, int B, bool HP>
 __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, const OperandView *views, int4 tk,
                                         const double *__restrict__ Aarena, const double *__restrict__ Barena,
                                         int *__restrict__ E, uint8_t *__restrict__ arena) {
+  constexpr int NP = S + (HP ? 1 : 0);  // digit planes, and the magnitudes of the leading one
   __shared__ int smax[STRIP];
   const int p0 = tk.x, p1 = tk.y, r0 = tk.z;
   const SplitPair &Q = pairs[p0];
   const bool dup = CPLX && Q.dupb == 0;  // two real rows per row of op(A)
   const int l0 = dup ? r0 / 2 : r0;
   const int nl = min(dup ? STRIP / 2 : STRIP, Q.M - l0);
-  strip_maxima<CPLX, false>(pairs, views, p0, p1, l0, nl, Aarena, Barena, smax);
+  strip_maxima<CPLX, false, HP>(pairs, views, p0, p1, l0, nl, Aarena, Barena, smax);
   if (threadIdx.x < nl) {
     const int e = smax[threadIdx.x];
     if (dup) {
@@ -376,7 +383,7 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
     const bool ca = P.trans & 4;
     const OpAddr ad = addr_a(P, views, p);
     const Factor Fa{P.fm, P.fe, P.fneg != 0};
-    uint8_t *tiles = arena + P.as_off + (int64_t)mt * P.KB * S * A_DIGIT_BYTES;
+    uint8_t *tiles = arena + P.as_off + (int64_t)mt * P.KB * NP * A_DIGIT_BYTES;
     if (dup) {
       // item = one row of op(A) (real rows 2m, 2m+1) x 4 complex k
       const int items = (STRIP / 2) * KCM * P.KB;
@@ -393,26 +400,32 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
           a[j] = make_double2(0.0, 0.0);
           if (k < P.K) a[j] = ld_pol(reinterpret_cast<const double2 *>(A) + lo + ad.depth(k), last);
         }
-        uint32_t p0w[S][4], p1w[S][4];
+        // row 2m: ( re, -im ); row 2m+1 is formed from it at the store, which
+        // saves half of the digit registers (72 -> 54, two more CTAs per SM;
+        // the strips of the 2000-product batch 1.98 -> 1.89 ms)
+        uint32_t pw[NP][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           float dr[S], di[S];
           digits_f<S, B>(scaled_int(a[j].x, Ei, B * S, Fa), dr);
           digits_f<S, B>(scaled_int(ca ? -a[j].y : a[j].y, Ei, B * S, Fa), di);
 #pragma unroll
-          for (int t = 0; t < S; ++t) {
-            p0w[t][j] = pack2(dr[t], -di[t]);  // ( re, -im )
-            p1w[t][j] = pack2(di[t], dr[t]);   // ( im,  re )
-          }
+          for (int t = 0; t < S; ++t) pw[t][j] = pack2(dr[t], -di[t]);
+          if constexpr (HP) pw[S][j] = pw[0][j] & 0x7FFF7FFFu;
         }
         const int rr0 = rl + 2 * ml, rr1 = rr0 + 1;
-        uint8_t *tile = tiles + (int64_t)kb * S * A_DIGIT_BYTES;
+        uint8_t *tile = tiles + (int64_t)kb * NP * A_DIGIT_BYTES;
         uint8_t *d0 = tile + ((rr0 >> 3) * KCM + q) * 128 + (rr0 & 7) * 16;
         uint8_t *d1 = tile + ((rr1 >> 3) * KCM + q) * 128 + (rr1 & 7) * 16;
 #pragma unroll
-        for (int t = 0; t < S; ++t) {
-          st_pol(d0 + t * A_DIGIT_BYTES, make_uint4(p0w[t][0], p0w[t][1], p0w[t][2], p0w[t][3]), last);
-          st_pol(d1 + t * A_DIGIT_BYTES, make_uint4(p1w[t][0], p1w[t][1], p1w[t][2], p1w[t][3]), last);
+        for (int t = 0; t < NP; ++t) {
+          st_pol(d0 + t * A_DIGIT_BYTES, make_uint4(pw[t][0], pw[t][1], pw[t][2], pw[t][3]), last);
+          // row 2m+1: ( im, re ) = the halves of row 2m exchanged, the sign of im flipped back
+          const uint32_t flip = t < S ? 0x8000u : 0u;
+          st_pol(d1 + t * A_DIGIT_BYTES,
+                 make_uint4(__byte_perm(pw[t][0], 0, 0x1032) ^ flip, __byte_perm(pw[t][1], 0, 0x1032) ^ flip,
+                            __byte_perm(pw[t][2], 0, 0x1032) ^ flip, __byte_perm(pw[t][3], 0, 0x1032) ^ flip),
+                 last);
         }
       }
     } else {
@@ -424,7 +437,7 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
         if (rloc >= nl) continue;
         const int64_t lo = P.a_off + ad.line(l0 + rloc);
         const int Ei = smax[rloc];
-        uint32_t pk[S][4];
+        uint32_t pk[NP][4];
         if constexpr (CPLX) {
           double2 a[4];
 #pragma unroll
@@ -458,10 +471,14 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
             for (int t = 0; t < S; ++t) pk[t][e >> 1] = pack2(d0[t], d1[t]);
           }
         }
-        const int rr = rl + rloc;
-        uint8_t *dst = tiles + (int64_t)kb * S * A_DIGIT_BYTES + ((rr >> 3) * KCM + q) * 128 + (rr & 7) * 16;
+        if constexpr (HP) {
 #pragma unroll
-        for (int t = 0; t < S; ++t)
+          for (int j = 0; j < 4; ++j) pk[S][j] = pk[0][j] & 0x7FFF7FFFu;
+        }
+        const int rr = rl + rloc;
+        uint8_t *dst = tiles + (int64_t)kb * NP * A_DIGIT_BYTES + ((rr >> 3) * KCM + q) * 128 + (rr & 7) * 16;
+#pragma unroll
+        for (int t = 0; t < NP; ++t)
           st_pol(dst + t * A_DIGIT_BYTES, make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]), last);
       }
     }
@@ -469,17 +486,18 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
 }
 
 // B role.  Task = (first pair, end pair, first real column c0 of the strip).
-template <bool CPLX, int S, int B>
+template <bool CPLX, int S, int B, bool HP>
 __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, const OperandView *views, int4 tk,
                                         const double *__restrict__ Aarena, const double *__restrict__ Barena,
                                         int *__restrict__ F, uint8_t *__restrict__ arena) {
+  constexpr int NP = S + (HP ? 1 : 0);
   __shared__ int smax[STRIP];
   const int p0 = tk.x, p1 = tk.y, c0 = tk.z;
   const SplitPair &Q = pairs[p0];
   const bool dup = CPLX && Q.dupb != 0;  // two real columns per column of op(B)
   const int l0 = dup ? c0 / 2 : c0;
   const int nl = min(dup ? STRIP / 2 : STRIP, Q.N - l0);
-  strip_maxima<CPLX, true>(pairs, views, p0, p1, l0, nl, Aarena, Barena, smax);
+  strip_maxima<CPLX, true, HP>(pairs, views, p0, p1, l0, nl, Aarena, Barena, smax);
   if (threadIdx.x < nl) {
     const int e = smax[threadIdx.x];
     if (dup) {
@@ -498,7 +516,7 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
     const double *__restrict__ Bm = P.swap ? Aarena : Barena;
     const bool cb = P.trans & 8;
     const OpAddr ad = addr_b(P, views, p);
-    uint8_t *tiles = arena + P.bs_off + (int64_t)nt * P.KB * S * B_DIGIT_BYTES;
+    uint8_t *tiles = arena + P.bs_off + (int64_t)nt * P.KB * NP * B_DIGIT_BYTES;
     // item = one real column x 8 real k
     const int items = STRIP * KCM * P.KB;
     for (int w = threadIdx.x; w < items; w += blockDim.x) {
@@ -507,7 +525,7 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
       if (cloc >= ncols) continue;  // columns past the block feed discarded outputs only
       const int c = cl + cloc;
       const int Fj = smax[dup ? cloc >> 1 : cloc];
-      uint32_t pk[S][4];
+      uint32_t pk[NP][4];
       if constexpr (CPLX) {
         const int64_t lo = P.b_off + ad.line(dup ? l0 + (cloc >> 1) : l0 + cloc);
         double2 x[4];
@@ -547,9 +565,13 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
           for (int t = 0; t < S; ++t) pk[t][e >> 1] = pack2(d0[t], d1[t]);
         }
       }
-      uint8_t *dst = tiles + (int64_t)kb * S * B_DIGIT_BYTES + ((c >> 3) * KCM + q) * 128 + (c & 7) * 16;
+      if constexpr (HP) {
 #pragma unroll
-      for (int t = 0; t < S; ++t)
+        for (int j = 0; j < 4; ++j) pk[S][j] = pk[0][j] & 0x7FFF7FFFu;
+      }
+      uint8_t *dst = tiles + (int64_t)kb * NP * B_DIGIT_BYTES + ((c >> 3) * KCM + q) * 128 + (c & 7) * 16;
+#pragma unroll
+      for (int t = 0; t < NP; ++t)
         st_pol(dst + t * B_DIGIT_BYTES, make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]), last);
     }
   }
@@ -557,35 +579,43 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
 
 // VIEWS = false: no pair of the launch reads its operand through a view, and
 // the view addressing is compiled out
-template <bool CPLX, int S, bool VIEWS>
+template <bool CPLX, int S, bool VIEWS, bool HP>
 __global__ void __launch_bounds__(STRIP_THREADS)
 strip_a_kernel(const SplitPair *__restrict__ pairs, const OperandView *__restrict__ views_in,
                const int4 *__restrict__ tasks, const double *__restrict__ A, const double *__restrict__ B,
                int *__restrict__ E, uint8_t *__restrict__ arena, int b) {
   const OperandView *views = VIEWS ? views_in : nullptr;
   const int4 tk = tasks[blockIdx.x];
-  switch (b) {  // the host admits b = 5..8 only
-    case 5: strip_a<CPLX, S, 5>(pairs, views, tk, A, B, E, arena); break;
-    case 6: strip_a<CPLX, S, 6>(pairs, views, tk, A, B, E, arena); break;
-    case 7: strip_a<CPLX, S, 7>(pairs, views, tk, A, B, E, arena); break;
-    default: strip_a<CPLX, S, 8>(pairs, views, tk, A, B, E, arena); break;
+  if constexpr (HP) {  // FP64-grade launches: always 8-bit digits
+    strip_a<CPLX, S, 8, true>(pairs, views, tk, A, B, E, arena);
+  } else {
+    switch (b) {  // the host admits b = 5..8 only
+      case 5: strip_a<CPLX, S, 5, false>(pairs, views, tk, A, B, E, arena); break;
+      case 6: strip_a<CPLX, S, 6, false>(pairs, views, tk, A, B, E, arena); break;
+      case 7: strip_a<CPLX, S, 7, false>(pairs, views, tk, A, B, E, arena); break;
+      default: strip_a<CPLX, S, 8, false>(pairs, views, tk, A, B, E, arena); break;
+    }
   }
 }
 
 // VIEWS = false: no pair of the launch reads its operand through a view, and
 // the view addressing is compiled out
-template <bool CPLX, int S, bool VIEWS>
+template <bool CPLX, int S, bool VIEWS, bool HP>
 __global__ void __launch_bounds__(STRIP_THREADS)
 strip_b_kernel(const SplitPair *__restrict__ pairs, const OperandView *__restrict__ views_in,
                const int4 *__restrict__ tasks, const double *__restrict__ A, const double *__restrict__ B,
                int *__restrict__ F, uint8_t *__restrict__ arena, int b) {
   const OperandView *views = VIEWS ? views_in : nullptr;
   const int4 tk = tasks[blockIdx.x];
-  switch (b) {
-    case 5: strip_b<CPLX, S, 5>(pairs, views, tk, A, B, F, arena); break;
-    case 6: strip_b<CPLX, S, 6>(pairs, views, tk, A, B, F, arena); break;
-    case 7: strip_b<CPLX, S, 7>(pairs, views, tk, A, B, F, arena); break;
-    default: strip_b<CPLX, S, 8>(pairs, views, tk, A, B, F, arena); break;
+  if constexpr (HP) {  // FP64-grade launches: always 8-bit digits
+    strip_b<CPLX, S, 8, true>(pairs, views, tk, A, B, F, arena);
+  } else {
+    switch (b) {  // the host admits b = 5..8 only
+      case 5: strip_b<CPLX, S, 5, false>(pairs, views, tk, A, B, F, arena); break;
+      case 6: strip_b<CPLX, S, 6, false>(pairs, views, tk, A, B, F, arena); break;
+      case 7: strip_b<CPLX, S, 7, false>(pairs, views, tk, A, B, F, arena); break;
+      default: strip_b<CPLX, S, 8, false>(pairs, views, tk, A, B, F, arena); break;
+    }
   }
 }
 
@@ -751,6 +781,59 @@ __device__ __forceinline__ void fold_groups(uint32_t set_base, int cbase, int b,
   }
 }
 
+// Smallest certificate of an output: sum_k |d_0(ik)| |d_0(kj)| in units of
+// 2^(E_i+F_j-2b), where 2^(2b) is the product of two full-scale entries.  The
+// truncations -- 2^-57 of full scale per operand entry and at most 6 2^-58 for
+// the digit products left out -- are below K 2^(E_i+F_j) 2^-54.9, so a sum of
+// at least full scale / 16 keeps them within 4.3 K u sum_k |a_ik b_kj|
+// (u = 2^-53; an FP64 dot product is bounded by K u of the same sum).
+// Normally distributed entries pass for sums of about 48 terms on.
+constexpr float CERT_MIN = 65536.0f / 16.0f;
+
+// FP64-grade fold (S digits, two 64-bit words): the groups 0..HG-1 into Vh
+// with weights 2^(b(HG-1-g)), the others into Vl with 2^(b(S-1-g)), so that
+// V = Vh 2^(b(S-HG)) + Vl exactly (no bit of any group is dropped; the words
+// hold 25 + b(HG-1) resp. 25 + b(S-HG-1) bits and the chunk count's).  The
+// certificate group S (products of the leading digits' magnitudes) is summed
+// in FP32: it is compared with a threshold only.
+constexpr int HG = 4;
+template <int S, int G0, int NG>
+__device__ __forceinline__ void fold_groups_hp(uint32_t set_base, int cbase, int b, unsigned long long (&Vl)[8],
+                                               unsigned long long (&Vh)[8], float (&cert)[8]) {
+  float acc[NG][8];
+#pragma unroll
+  for (int g = 0; g < NG; ++g) tmem_ld8(set_base + (uint32_t)((G0 + g) * TNS + cbase), acc[g]);
+  tmem_wait_ld();
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    const int gg = G0 + g;
+    if (gg == S) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) cert[c] += acc[g][c];
+    } else if (gg < HG) {
+      const int m = 1 << (b * (HG - 1 - gg));
+#pragma unroll
+      for (int c = 0; c < 8; ++c) Vh[c] = mad_wide(__float2int_rn(acc[g][c]), m, Vh[c]);
+    } else {
+      const int m = 1 << (b * (S - 1 - gg));
+#pragma unroll
+      for (int c = 0; c < 8; ++c) Vl[c] = mad_wide(__float2int_rn(acc[g][c]), m, Vl[c]);
+    }
+  }
+}
+
+// (Vh 2^lb + Vl) 2^scale rounded once to FP64: the sum is normalised into 62
+// bits with a sticky bit below (24 <= lb <= 31).
+__device__ __forceinline__ double wide_to_double(long long Vh, long long Vl, int lb, int scale) {
+  const long long T = Vh + (Vl >> lb);                       // floor of the sum / 2^lb
+  const unsigned long long rem = (unsigned long long)Vl & ((1ull << lb) - 1);
+  const int room = __clzll(T < 0 ? ~T : T) - 2;              // left shifts that keep a spare bit
+  const int k = min(max(room, 0), lb);
+  long long V = (long long)((unsigned long long)T << k) | (long long)(rem >> (lb - k));
+  if (rem & ((1ull << (lb - k)) - 1)) V |= 1;                // sticky
+  return fixed_to_double(V, scale + lb - k);
+}
+
 // Chunking rule shared by the host and the MMA issuer: a new chunk starts
 // when adding the next K block would push the summed (real) depth of the
 // current chunk above kchunk.
@@ -765,12 +848,19 @@ __device__ __forceinline__ int kblock_depth(int Kr, int kb) { return min(TKS, Kr
 // fills the other.
 __device__ __forceinline__ int tile_of(int r, int c, int G) { return r * G + ((r & 1) ? (G - 1 - c) : c); }
 
-template <int S>
+//
+// HP: the FP64-grade launch of the plain path (see split_f64_eligible): S
+// digits plus one plane of the leading digits' magnitudes per operand, whose
+// product (accumulator group S) bounds sum_k |a_ik b_kj| from below.  An
+// output whose bound is too small for the digits' truncation to stay at the
+// level of an FP64 sum, or whose row or column holds an infinity or NaN,
+// raises the flag of its FP64 tile, which the FP64 kernel then recomputes.
+template <int S, bool HP>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPair *__restrict__ pairs,
                   const uint8_t *__restrict__ arena, const int *__restrict__ E,
                   const int *__restrict__ F, double *__restrict__ C, int b, int nstages,
-                  int kchunk, int *err) {
+                  int kchunk, int *err, int *__restrict__ flags) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);       // [MAX_STAGES]
   uint64_t *empty = full + MAX_STAGES;                        // [MAX_STAGES]
@@ -779,9 +869,10 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 516);
   uint8_t *stages = smem + SMEM_HDR;
-  constexpr uint32_t A_BYTES = S * A_DIGIT_BYTES, B_BYTES = S * B_DIGIT_BYTES;
+  constexpr int NP = S + (HP ? 1 : 0);
+  constexpr uint32_t A_BYTES = NP * A_DIGIT_BYTES, B_BYTES = NP * B_DIGIT_BYTES;
   constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  constexpr uint32_t SET_COLS = S * TNS;  // columns of one accumulator set
+  constexpr uint32_t SET_COLS = NP * TNS;  // columns of one accumulator set
   constexpr uint32_t NCOLS = (2 * SET_COLS <= 256) ? 256 : 512;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -913,6 +1004,11 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
                 const uint32_t acc = (fresh && ks == 0 && t == 0) ? 0u : 1u;
                 umma_bf16(dset + (uint32_t)(t * TNS), ad, bd, idesc[S - 1 - t], acc);
               }
+              if constexpr (HP) {
+                const uint64_t ad = dst0 + (uint64_t)((S * A_DIGIT_BYTES + ks * 256) >> 4);
+                const uint64_t bd = dst0 + (uint64_t)((A_BYTES + S * B_DIGIT_BYTES + ks * 256) >> 4);
+                umma_bf16(dset + (uint32_t)(S * TNS), ad, bd, idesc[0], (fresh && ks == 0) ? 0u : 1u);
+              }
             }
             fresh = false;
             umma_commit(&empty[st]);
@@ -975,11 +1071,13 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
       const int Ei = rv ? E[T.eoff + i_glob] : 0;
       const int rsh = T.rshift;
       unsigned long long Vl[CW];
-      unsigned int Vh[CW];
+      std::conditional_t<HP, unsigned long long, unsigned int> Vh[CW];
+      float cert[CW];
 #pragma unroll
       for (int jj = 0; jj < CW; ++jj) {
         Vl[jj] = 0;
         Vh[jj] = 0;
+        cert[jj] = 0.0f;
       }
       for (int ch = 0; ch < T.nchunk; ++ch, ++u) {
         // one lane polls; the warp proceeds together (tcgen05.ld is .aligned)
@@ -991,7 +1089,10 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
         const uint32_t set_base = lane_base + (uint32_t)((u & 1) * SET_COLS);
         // the groups' columns are in flight together (one wait per batch of up
         // to six): the drain is bound by TMEM load latency otherwise
-        if constexpr (S <= 6) {
+        if constexpr (HP) {
+          fold_groups_hp<S, 0, 4>(set_base, cbase, b, Vl, Vh, cert);
+          fold_groups_hp<S, 4, NP - 4>(set_base, cbase, b, Vl, Vh, cert);
+        } else if constexpr (S <= 6) {
           fold_groups<S, 0, S>(set_base, cbase, b, rsh, Vl, Vh);
         } else {
           fold_groups<S, 0, 4>(set_base, cbase, b, rsh, Vl, Vh);
@@ -1003,15 +1104,28 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
       }
       if (!ok) break;
       if (rv) {
-        const int rsplit = T.splits & 1, csplit = T.splits >> 1;
+        const int rsplit = T.splits & 1, csplit = (T.splits >> 1) & 1;
         double *crow = C + T.c_off + (int64_t)(i_glob >> rsplit) * T.rs + (i_glob & rsplit);
 #pragma unroll
         for (int jj = 0; jj < CW; ++jj) {
           const int j = j0 + jj;
           if (j < T.N) {
-            const long long V = (long long)(((unsigned long long)Vh[jj] << 32) + Vl[jj]);
-            crow[(int64_t)(j >> csplit) * T.ldc + (j & csplit)] =
-                fixed_to_double(V, Ei + F[T.foff + j] + rsh + scale_b);
+            double *out = crow + (int64_t)(j >> csplit) * T.ldc + (j & csplit);
+            if constexpr (HP) {
+              const int Fj = F[T.foff + j];
+              *out = wide_to_double((long long)Vh[jj], (long long)Vl[jj], b * (S - HG), Ei + Fj + scale_b);
+              // a row or column of zeros (EMPTY_EXP) is exact
+              if (max(Ei, Fj) >= NONFINITE_EXP || (min(Ei, Fj) > EMPTY_EXP && cert[jj] < CERT_MIN)) {
+                const int rdup = (T.splits >> 3) & 1, cdup = (T.splits >> 4) & 1;
+                const int lr = i_glob >> rdup, lc = j >> cdup;
+                const bool sw = T.splits & 4;
+                const int rows = sw ? T.N >> cdup : T.Mr >> rdup;  // of C
+                flags[T.fbase + ((sw ? lc : lr) >> 6) + ((sw ? lr : lc) >> 6) * ((rows + 63) >> 6)] = 1;
+              }
+            } else {
+              const long long V = (long long)(((unsigned long long)Vh[jj] << 32) + Vl[jj]);
+              *out = fixed_to_double(V, Ei + F[T.foff + j] + rsh + scale_b);
+            }
           }
         }
       }
@@ -1026,26 +1140,26 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
   }
 }
 
-template <int S>
+template <int NP>
 size_t smem_bytes(int nstages) {
-  return SMEM_HDR + (size_t)nstages * S * (A_DIGIT_BYTES + B_DIGIT_BYTES);
+  return SMEM_HDR + (size_t)nstages * NP * (A_DIGIT_BYTES + B_DIGIT_BYTES);
 }
 
-template <int S>
+template <int NP>
 int pick_stages() {
-  const size_t per = (size_t)S * (A_DIGIT_BYTES + B_DIGIT_BYTES);
+  const size_t per = (size_t)NP * (A_DIGIT_BYTES + B_DIGIT_BYTES);
   int n = (int)((SMEM_LIMIT - SMEM_HDR) / per);
   return std::max(1, std::min(n, MAX_STAGES));
 }
 
-template <int S>
+template <int S, bool HP>
 void launch_split_s(Ctx *ctx, bool cplx, const SplitPair *d_pairs, const OperandView *d_va, const OperandView *d_vb,
                     const int4 *d_sa, int nsa, const int4 *d_sb, int nsb, const SplitTile *d_tiles, int ntiles,
                     const double *A, const double *B, double *C, int *dE, int *dF, uint8_t *arena, int b,
-                    int kchunk, int *err, bool may_fork) {
-  if (b < 5 || b > 8 || b * S > 62) fail(QS_ERR_INTERNAL, "split: unsupported digit plan b=%d S=%d", b, S);
+                    int kchunk, int *err, bool may_fork, int *flags, bool marks) {
+  if (b < 5 || b > 8 || b * S > 62 || (HP && (b != 8 || d_va || d_vb))) fail(QS_ERR_INTERNAL, "split: unsupported digit plan b=%d S=%d", b, S);
   cudaStream_t st = ctx->stream;
-  ctx->mark(0);
+  if (marks) ctx->mark(0);
   // the two roles' strips are independent: the B role runs on the
   // context's second stream beside the A role, so that neither launch's
   // last partial wave leaves SMs idle; the GEMM waits for both (not on the
@@ -1061,13 +1175,17 @@ void launch_split_s(Ctx *ctx, bool cplx, const SplitPair *d_pairs, const Operand
   auto strips = [&](auto cx) {
     constexpr bool CX = decltype(cx)::value;
     if (nsb) {
-      if (d_vb) strip_b_kernel<CX, S, true><<<nsb, STRIP_THREADS, 0, sb>>>(d_pairs, d_vb, d_sb, A, B, dF, arena, b);
-      else strip_b_kernel<CX, S, false><<<nsb, STRIP_THREADS, 0, sb>>>(d_pairs, nullptr, d_sb, A, B, dF, arena, b);
+      if (!HP && d_vb)
+        strip_b_kernel<CX, S, !HP, HP><<<nsb, STRIP_THREADS, 0, sb>>>(d_pairs, d_vb, d_sb, A, B, dF, arena, b);
+      else
+        strip_b_kernel<CX, S, false, HP><<<nsb, STRIP_THREADS, 0, sb>>>(d_pairs, nullptr, d_sb, A, B, dF, arena, b);
       QS_LAUNCHED(ctx);
     }
     if (nsa) {
-      if (d_va) strip_a_kernel<CX, S, true><<<nsa, STRIP_THREADS, 0, st>>>(d_pairs, d_va, d_sa, A, B, dE, arena, b);
-      else strip_a_kernel<CX, S, false><<<nsa, STRIP_THREADS, 0, st>>>(d_pairs, nullptr, d_sa, A, B, dE, arena, b);
+      if (!HP && d_va)
+        strip_a_kernel<CX, S, !HP, HP><<<nsa, STRIP_THREADS, 0, st>>>(d_pairs, d_va, d_sa, A, B, dE, arena, b);
+      else
+        strip_a_kernel<CX, S, false, HP><<<nsa, STRIP_THREADS, 0, st>>>(d_pairs, nullptr, d_sa, A, B, dE, arena, b);
       QS_LAUNCHED(ctx);
     }
   };
@@ -1077,15 +1195,16 @@ void launch_split_s(Ctx *ctx, bool cplx, const SplitPair *d_pairs, const Operand
     QS_CUDA(cudaEventRecord(ctx->aux_join, ctx->aux));
     QS_CUDA(cudaStreamWaitEvent(st, ctx->aux_join, 0));
   }
-  const int nst = pick_stages<S>();
-  const size_t sm = smem_bytes<S>(nst);
-  QS_CUDA(cudaFuncSetAttribute(gemm_split_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  ctx->mark(1);
+  constexpr int NP = S + (HP ? 1 : 0);
+  const int nst = pick_stages<NP>();
+  const size_t sm = smem_bytes<NP>(nst);
+  QS_CUDA(cudaFuncSetAttribute(gemm_split_kernel<S, HP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (marks) ctx->mark(1);
   const int grid = std::min(ntiles, std::max(ctx->num_sms, 1));
-  gemm_split_kernel<S><<<grid, GEMM_THREADS, sm, st>>>(d_tiles, ntiles, d_pairs, arena, dE, dF, C, b, nst, kchunk,
-                                              err);
+  gemm_split_kernel<S, HP><<<grid, GEMM_THREADS, sm, st>>>(d_tiles, ntiles, d_pairs, arena, dE, dF, C, b, nst, kchunk,
+                                                           err, flags);
   QS_LAUNCHED(ctx);
-  ctx->mark(2);
+  if (marks) ctx->mark(2);
 }
 
 }  // namespace
@@ -1176,9 +1295,14 @@ DigitPlan choose_digits(int64_t kreal, double tol, int forced_slices) {
   return choose_digits_for(one, {0, 1}, {TMS}, {TNS}, 1, tol, forced_slices);
 }
 
+// Digits of the FP64-grade launches: 7 x 8 bits and the magnitude plane fill
+// the two accumulator sets of TMEM (8 groups x 32 columns x 2).
+constexpr int HP_BITS = 8, HP_DIGITS = 7;
+
 // Host-side work lists of one planned split product.
 struct SplitWork {
   int S = 0, b = 0, kchunk = 0;
+  bool hp = false;  // FP64-grade: one more plane per operand, tile flags
   int64_t nE = 0, nF = 0, arena = 0;
   std::vector<SplitPair> sp;
   // strips of STRIP real lines: (first pair, end pair, first line, 0) of the
@@ -1197,6 +1321,7 @@ struct SplitDev {
   OperandView *va = nullptr, *vb = nullptr;
   int *E = nullptr, *F = nullptr;
   uint8_t *arena = nullptr;
+  int *flags = nullptr;  // FP64-grade: one flag per FP64 tile
 };
 
 // Host half of the split path: digit plan, per-pair digit geometry and arena
@@ -1264,7 +1389,8 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
                               const std::vector<int64_t> &c_off, bool cplx, int forced_slices, double tol,
                               const std::vector<int32_t> *blk_ldc, SplitWork &w, int forced_bits = 0,
                               const std::vector<OperandView> *va = nullptr,
-                              const std::vector<OperandView> *vb = nullptr) {
+                              const std::vector<OperandView> *vb = nullptr,
+                              const std::vector<int32_t> *fbase = nullptr) {
   SplitResult res;
   const int64_t nb = (int64_t)blk_M_in.size();
   const int cm = cplx ? 2 : 1;
@@ -1291,8 +1417,11 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
         }
       }
   }
-  DigitPlan dp = choose_digits_for(pairs, grp, blk_M, blk_N, cm, tol, forced_slices, forced_bits);
+  w.hp = fbase != nullptr;
+  DigitPlan dp = w.hp ? DigitPlan{HP_BITS, HP_DIGITS, (HP_DIGITS + 2) * std::ldexp(1.0, -HP_BITS * HP_DIGITS)}
+                      : choose_digits_for(pairs, grp, blk_M, blk_N, cm, tol, forced_slices, forced_bits);
   const int S = dp.nslices, b = dp.bits;
+  const int NP = S + (w.hp ? 1 : 0);
   const int kchunk = kchunk_of(b, S);
   w.S = S;
   w.b = b;
@@ -1355,9 +1484,9 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
       s.e_afac = e;
       s.swap = mode[g] & 1;
       s.as_off = arena;
-      arena += (int64_t)s.MT * s.KB * S * A_DIGIT_BYTES;
+      arena += (int64_t)s.MT * s.KB * NP * A_DIGIT_BYTES;
       s.bs_off = arena;
-      arena += (int64_t)s.NT * s.KB * S * B_DIGIT_BYTES;
+      arena += (int64_t)s.NT * s.KB * NP * B_DIGIT_BYTES;
     }
     // exponent + slicing strips over all pairs of the block
     if (grp[g + 1] > grp[g]) {
@@ -1415,6 +1544,9 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
           t.ldc = 1;
           t.splits = 0;
         }
+        if (swp) t.splits |= 4;
+        if (cm == 2) t.splits |= dupb ? 16 : 8;
+        t.fbase = fbase ? (*fbase)[g] : 0;
         t.eoff = (int32_t)eoff[g];
         t.foff = (int32_t)foff[g];
         t.nchunk = nchunk;
@@ -1456,13 +1588,19 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
 // split product on the context's stream, with every work list, exponent
 // array and the digit arena already on the device.
 static void launch_split(Ctx *ctx, const SplitWork &w, bool cplx, const SplitDev &d, const double *A,
-                         const double *B, double *C, int *err, bool may_fork = true) {
+                         const double *B, double *C, int *err, bool may_fork = true, bool marks = true) {
+  if (w.hp) {
+    launch_split_s<HP_DIGITS, true>(ctx, cplx, d.pairs, nullptr, nullptr, d.sa, (int)w.sa.size(), d.sb,
+                                    (int)w.sb.size(), d.tiles, (int)w.tiles.size(), A, B, C, d.E, d.F, d.arena, w.b,
+                                    w.kchunk, err, may_fork, d.flags, marks);
+    return;
+  }
   switch (w.S) {
 #define QS_CASE(SS)                                                                                      \
   case SS:                                                                                               \
-    launch_split_s<SS>(ctx, cplx, d.pairs, d.va, d.vb, d.sa, (int)w.sa.size(), d.sb, (int)w.sb.size(),    \
-                       d.tiles, (int)w.tiles.size(), A, B, C, d.E, d.F, d.arena, w.b, w.kchunk, err,     \
-                       may_fork);                                                                        \
+    launch_split_s<SS, false>(ctx, cplx, d.pairs, d.va, d.vb, d.sa, (int)w.sa.size(), d.sb,               \
+                              (int)w.sb.size(), d.tiles, (int)w.tiles.size(), A, B, C, d.E, d.F, d.arena, \
+                              w.b, w.kchunk, err, may_fork, nullptr, marks);                             \
     break;
     QS_CASE(2)
     QS_CASE(3)
@@ -1684,15 +1822,171 @@ std::vector<int> split_candidate_bits(double tol, int forced_slices) {
   return out;
 }
 
+// ------------------------------------------- FP64-grade tensor-core products
+// Blocks the tensor-core launch takes: a summed real depth of at least
+// F64T_DEPTH (below it a sum of normally distributed terms often misses the
+// certificate) and at least F64T_WORK real multiply-adds.  GB300's FP64 pipe
+// does about 2 multiply-adds per clock and SM: a 64 x 64 tile of depth 64
+// holds an SM for 70 us, while its digits take two strip launches and one
+// tile of the tensor-core launch.  Measured, FP64 tiles against this path: 300
+// complex products of 8..1024 per side 23.1 -> 1.71 ms (15.6 TFLOP/s of FP64
+// work; error against a 64-bit product 1.2e-15 -> 6.7e-16), 64 real blocks of
+// 4..96 105 -> 77 us.
+constexpr int64_t F64T_DEPTH = 48, F64T_MAX_DEPTH = 1 << 20;
+constexpr double F64T_WORK = 65536.0;
+// Digit bytes of one launch (blocks above it get a launch of their own), and
+// of a block that still takes this path.
+constexpr int64_t F64T_CHUNK_BYTES = int64_t(2) << 30, F64T_BLOCK_BYTES = int64_t(8) << 30;
+
+F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
+                              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, bool cplx,
+                              const std::vector<char> &skip, std::vector<TileDesc> &tiles) {
+  F64TensorList tl;
+  const int64_t nb = (int64_t)bM.size();
+  const int64_t cm = cplx ? 2 : 1;
+  tl.on.assign(nb, 0);
+  tl.fbase.assign(nb, 0);
+  int64_t chunk0 = 0, chunk_bytes = 0;
+  auto up = [](int64_t x, int64_t t) { return (x + t - 1) / t * t; };
+  for (int64_t g = 0; g < nb; ++g) {
+    if (!skip.empty() && skip[g]) continue;
+    int64_t depth = 0, kpad = 0;
+    bool fits = true;
+    for (int64_t p = grp[g]; p < grp[g + 1]; ++p) {
+      const int64_t K = std::max<int32_t>(pairs[p].K, 0);
+      depth += K * cm;
+      kpad += up(std::max<int64_t>(K * cm, 1), TKS);
+      // a factor of 0 keeps the FP64 kernel's 0 * x (NaN for an infinite x)
+      fits = fits && std::isfinite(pairs[p].afac) && pairs[p].afac != 0.0;
+    }
+    const int64_t M = bM[g], N = bN[g];
+    if (!fits || depth < F64T_DEPTH || depth > F64T_MAX_DEPTH ||
+        double(M) * double(N) * double(depth) * double(cm) < F64T_WORK || M > (1 << 24) || N > (1 << 24))
+      continue;
+    // either operand's real form may be the duplicated one
+    const int64_t bytes = (up(M * cm, TMS) + up(N * cm, TMS)) * kpad * (HP_DIGITS + 1) * 2;
+    if (bytes > F64T_BLOCK_BYTES) continue;
+    const int64_t cells = ((M + 63) / 64) * ((N + 63) / 64);
+    if (tl.nflags + cells > INT32_MAX) continue;
+    tl.on[g] = 1;
+    tl.fbase[g] = (int32_t)tl.nflags;
+    tl.nflags += cells;
+    tl.any = true;
+    if (chunk_bytes && chunk_bytes + bytes > F64T_CHUNK_BYTES) {
+      tl.chunks.push_back({chunk0, g});
+      chunk0 = g;
+      chunk_bytes = 0;
+    }
+    chunk_bytes += bytes;
+  }
+  if (!tl.any) return tl;
+  tl.chunks.push_back({chunk0, nb});
+  for (TileDesc &t : tiles)
+    if (tl.on[t.cblk]) t.flag = tl.fbase[t.cblk] + t.m0 / 64 + (t.n0 / 64) * ((t.M + 63) / 64);
+  return tl;
+}
+
+// Work lists of the launch of one block range of a list.
+static void plan_f64_chunk(const F64TensorList &tl, std::pair<int64_t, int64_t> range,
+                           const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
+                           const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
+                           const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
+                           SplitWork &w) {
+  std::vector<char> sel(bM.size(), 0);
+  std::vector<int32_t> fb;
+  for (int64_t g = range.first; g < range.second; ++g)
+    if (tl.on[g]) {
+      sel[g] = 1;
+      fb.push_back(tl.fbase[g]);
+    }
+  const BlockList L = select_blocks(pairs, grp, bM, bN, coff, bldc, sel);
+  plan_split(L.pairs, L.grp, L.bM, L.bN, L.coff, cplx, 0, 0, &L.bldc, w, 0, nullptr, nullptr, &fb);
+}
+
+bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
+                    const std::vector<int64_t> &grp, const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
+                    const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, const double *A,
+                    const double *B, double *C, bool cplx, int *d_flags) {
+  std::vector<SplitWork> ws(tl.chunks.size());
+  int64_t arena = 256;
+  for (size_t k = 0; k < ws.size(); ++k) {
+    plan_f64_chunk(tl, tl.chunks[k], pairs, grp, bM, bN, coff, bldc, cplx, ws[k]);
+    arena = std::max(arena, ws[k].arena);
+  }
+  uint8_t *digits = nullptr;
+  try {
+    digits = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)arena));
+  } catch (const Error &e) {
+    if (e.code != QS_ERR_OOM) throw;
+    cudaGetLastError();
+    return false;
+  }
+  for (size_t k = 0; k < ws.size(); ++k) {
+    const SplitWork &w = ws[k];
+    if (w.tiles.empty()) continue;
+    DevLists L;
+    const size_t sp = L.add(w.sp), sa = L.add(w.sa), sb = L.add(w.sb), st = L.add(w.tiles);
+    const size_t se = L.space((size_t)w.nE * sizeof(int)), sf = L.space((size_t)w.nF * sizeof(int));
+    L.commit(ctx);
+    SplitDev d;
+    d.arena = digits;
+    d.flags = d_flags;
+    d.pairs = L.at<SplitPair>(sp);
+    d.sa = L.at<int4>(sa);
+    d.sb = L.at<int4>(sb);
+    d.tiles = L.at<SplitTile>(st);
+    d.E = L.at<int>(se);
+    d.F = L.at<int>(sf);
+    launch_split(ctx, w, cplx, d, A, B, C, ctx->d_err, true, k == 0);
+  }
+  return true;
+}
+
 // A planned split product that can be launched many times: its work lists,
 // exponent arrays and digit arena are plain device allocations owned by the
 // handle, so their addresses stay fixed (a CUDA graph can replay the launch).
+// An FP64-grade plan may hold several launches, which share the arena.
 struct SplitPlanHandle {
-  SplitWork w;
-  SplitDev d;
+  std::vector<SplitWork> w;
+  std::vector<SplitDev> d;
   bool cplx = false;
-  SplitResult res;
+  int64_t flag_bytes = 0;  // cleared before the first launch
   std::vector<void *> owned;
+  ~SplitPlanHandle() {
+    for (void *p : owned) cudaFree(p);
+  }
+  void *own(size_t bytes) {
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 256));
+    if (e != cudaSuccess)
+      fail(e == cudaErrorMemoryAllocation ? QS_ERR_OOM : QS_ERR_CUDA, "split plan: cudaMalloc(%zu): %s", bytes,
+           cudaGetErrorString(e));
+    owned.push_back(p);
+    return p;
+  }
+  template <class T>
+  T *put(const std::vector<T> &v) {
+    T *p = static_cast<T *>(own(v.size() * sizeof(T)));
+    if (!v.empty()) QS_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    return p;
+  }
+  // device copies of every launch's lists, the exponent arrays and one arena
+  void allocate() {
+    int64_t arena = 0;
+    for (const SplitWork &x : w) arena = std::max(arena, x.arena);
+    uint8_t *digits = static_cast<uint8_t *>(own((size_t)arena));
+    for (const SplitWork &x : w) {
+      SplitDev v;
+      v.arena = digits;
+      v.pairs = put(x.sp);
+      v.sa = put(x.sa);
+      v.sb = put(x.sb);
+      v.tiles = put(x.tiles);
+      v.E = static_cast<int *>(own((size_t)x.nE * sizeof(int)));
+      v.F = static_cast<int *>(own((size_t)x.nF * sizeof(int)));
+      d.push_back(v);
+    }
+  }
 };
 
 SplitPlanHandle *split_plan_create(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
@@ -1701,49 +1995,47 @@ SplitPlanHandle *split_plan_create(const std::vector<PairDesc> &pairs, const std
                                    bool cplx, int forced_slices, double tol, int bits, SplitResult *res) {
   std::unique_ptr<SplitPlanHandle> h(new SplitPlanHandle);
   h->cplx = cplx;
-  h->res = plan_split(pairs, grp, blk_M, blk_N, c_off, cplx, forced_slices, tol, &blk_ldc, h->w, bits);
-  if (res) *res = h->res;
-  if (h->w.tiles.empty()) return h.release();
+  h->w.resize(1);
+  const SplitResult r =
+      plan_split(pairs, grp, blk_M, blk_N, c_off, cplx, forced_slices, tol, &blk_ldc, h->w[0], bits);
+  if (res) *res = r;
+  if (h->w[0].tiles.empty())
+    h->w.clear();
+  else
+    h->allocate();
+  return h.release();
+}
+
+SplitPlanHandle *f64_tensor_plan_create(const F64TensorList &tl, const std::vector<PairDesc> &pairs,
+                                        const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
+                                        const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
+                                        const std::vector<int32_t> &bldc, bool cplx, const int *&d_flags) {
+  std::unique_ptr<SplitPlanHandle> h(new SplitPlanHandle);
+  h->cplx = cplx;
+  h->w.resize(tl.chunks.size());
+  for (size_t k = 0; k < h->w.size(); ++k)
+    plan_f64_chunk(tl, tl.chunks[k], pairs, grp, bM, bN, coff, &bldc, cplx, h->w[k]);
   try {
-    auto own = [&](size_t bytes) -> void * {
-      void *p = nullptr;
-      cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 256));
-      if (e != cudaSuccess)
-        fail(e == cudaErrorMemoryAllocation ? QS_ERR_OOM : QS_ERR_CUDA, "split plan: cudaMalloc(%zu): %s", bytes,
-             cudaGetErrorString(e));
-      h->owned.push_back(p);
-      return p;
-    };
-    auto put = [&](const auto &v) {
-      using T = typename std::decay_t<decltype(v)>::value_type;
-      T *p = static_cast<T *>(own(v.size() * sizeof(T)));
-      if (!v.empty()) QS_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-      return p;
-    };
-    SplitDev &d = h->d;
-    d.pairs = put(h->w.sp);
-    d.sa = put(h->w.sa);
-    d.sb = put(h->w.sb);
-    d.tiles = put(h->w.tiles);
-    d.E = static_cast<int *>(own((size_t)h->w.nE * sizeof(int)));
-    d.F = static_cast<int *>(own((size_t)h->w.nF * sizeof(int)));
-    d.arena = static_cast<uint8_t *>(own((size_t)h->w.arena));
-  } catch (...) {
-    for (void *p : h->owned) cudaFree(p);
-    throw;
+    h->allocate();
+    h->flag_bytes = tl.nflags * (int64_t)sizeof(int);
+    int *flags = static_cast<int *>(h->own((size_t)h->flag_bytes));
+    for (SplitDev &v : h->d) v.flags = flags;
+    d_flags = flags;
+  } catch (const Error &e) {
+    if (e.code != QS_ERR_OOM) throw;
+    cudaGetLastError();
+    return nullptr;
   }
   return h.release();
 }
 
 void split_plan_launch(Ctx *ctx, SplitPlanHandle *h, const double *A, const double *B, double *C) {
-  if (!h->w.tiles.empty()) launch_split(ctx, h->w, h->cplx, h->d, A, B, C, ctx->d_err);
+  if (h->flag_bytes) QS_CUDA(cudaMemsetAsync(h->d[0].flags, 0, (size_t)h->flag_bytes, ctx->stream));
+  for (size_t k = 0; k < h->w.size(); ++k)
+    if (!h->w[k].tiles.empty()) launch_split(ctx, h->w[k], h->cplx, h->d[k], A, B, C, ctx->d_err, true, k == 0);
 }
 
 // The caller makes sure no launch of the handle is still running.
-void split_plan_destroy(SplitPlanHandle *h) {
-  if (!h) return;
-  for (void *p : h->owned) cudaFree(p);
-  delete h;
-}
+void split_plan_destroy(SplitPlanHandle *h) { delete h; }
 
 }  // namespace qs

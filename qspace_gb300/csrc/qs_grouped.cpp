@@ -116,9 +116,8 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
   const int64_t eb = cplx ? 16 : 8;
   const bool deep = reinterpret_cast<uintptr_t>(C) % eb == 0 && split_deep(pairs, grp, bM, bN, coff, bldc, ds);
   double *T = nullptr;
-  PairDesc *dp = nullptr;
-  TileDesc *dt = nullptr;
   DeepReduce *dr = nullptr;
+  DevLists lists;
   try {
     if (deep) {
       T = dev_alloc<double>(ctx, (size_t)std::max<int64_t>(ds.temp_elems, 1) * (cplx ? 2 : 1));
@@ -132,9 +131,9 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
     // (run_dot); the others through the 64 x 64 tiles
     std::vector<int64_t> small;
     std::vector<TileDesc> tiles;
+    std::vector<char> is_small(mm.size(), 0);
     {
       std::vector<TileDesc> all = make_tiles(gg, mm, nn, cc, gemm_f64_tile_m(), gemm_f64_tile_n(), ll, &pp);
-      std::vector<char> is_small(mm.size(), 0);
       for (size_t b = 0; b < mm.size(); ++b)
         if (deep && ds.part[b] && (int64_t)mm[b] * nn[b] <= DOT_OUTPUTS) {
           is_small[b] = 1;
@@ -144,20 +143,32 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
         if (!is_small[t.cblk]) tiles.push_back(t);
     }
     run_dot(ctx, pp, gg, mm, nn, cc, ll, small, A, B, C, cplx);
-    dp = dev_upload(ctx, pp);
-    dt = dev_upload(ctx, tiles);
-    if (!tiles.empty()) launch_gemm_f64(ctx, dp, dt, (int64_t)tiles.size(), A, B, C, cplx ? 1 : 0);
+    // larger blocks on the tensor cores, with the FP64 tiles as their net;
+    // the tile lists go first, as the tensor-core launch raises their flags
+    const F64TensorList tl = plan_f64_tensor(pp, gg, mm, nn, cplx, is_small, tiles);
+    if (!tiles.empty()) {
+      const size_t sp = lists.add(pp), st = lists.add(tiles), sf = lists.zeros((size_t)tl.nflags * sizeof(int));
+      lists.commit(ctx);
+      int *flags = tl.any ? lists.at<int>(sf) : nullptr;
+      if (tl.any && !run_f64_tensor(ctx, tl, pp, gg, mm, nn, cc, ll, A, B, C, cplx, flags)) {
+        // no room for the digits: every tile in FP64
+        for (TileDesc &t : tiles) t.flag = -1;
+        ctx->stage_upload(lists.at<TileDesc>(st), tiles.data(), tiles.size() * sizeof(TileDesc));
+      }
+      launch_gemm_f64(ctx, lists.at<PairDesc>(sp), lists.at<TileDesc>(st), (int64_t)tiles.size(), A, B, C,
+                      cplx ? 1 : 0, flags);
+    }
     if (deep) {
       dr = dev_upload(ctx, ds.red);
       launch_reduce_parts(ctx, dr, (int64_t)ds.red.size(), T, C, cplx);
     }
   } catch (...) {
     cudaStreamSynchronize(ctx->stream);
-    for (void *p : {(void *)T, (void *)dp, (void *)dt, (void *)dr})
+    for (void *p : {(void *)T, (void *)dr})
       if (p) dev_free(ctx, p);
     throw;
   }
-  for (void *p : {(void *)T, (void *)dp, (void *)dt, (void *)dr})
+  for (void *p : {(void *)T, (void *)dr})
     if (p) dev_free(ctx, p);
 }
 

@@ -71,6 +71,10 @@ struct Ctx {
   std::deque<StageMark> stage_q;    // copies in flight, oldest first
   std::vector<cudaEvent_t> stage_ev;  // recycled events
   void stage_upload(void *dst, const void *src, size_t bytes);
+  // room for `bytes` in the ring (host address); published to `dst` by
+  // stage_commit, before the next reservation
+  char *stage_reserve(size_t bytes);
+  void stage_commit(void *dst, size_t bytes);
   void destroy_staging();
   // copy streams of the pipelined host-buffer path (created on first use)
   cudaStream_t h2d = nullptr, d2h = nullptr;
@@ -211,8 +215,10 @@ struct TileDesc {
   int32_t M, N;
   int32_t ldc;
   int32_t cblk;
+  int32_t flag;   // computed only when this flag is raised (-1: always)
+  int32_t pad_;
 };
-static_assert(sizeof(TileDesc) == 40, "TileDesc layout");
+static_assert(sizeof(TileDesc) == 48, "TileDesc layout");
 
 // Generalised transpose of one block: out(j0..jr) = in(P-permuted index).
 struct PermDesc {
@@ -259,10 +265,11 @@ void launch_permute(Ctx *ctx, const PermDesc *d_desc, const int64_t *d_chunk_blk
                     const double *in, double *out, int is_complex, int chunk_elems);
 
 // qs_gemm_f64.cu -- plain FP64 grouped GEMM (deterministic: one CTA owns an
-// output tile, pairs summed in order)
+// output tile, pairs summed in order); tiles with a flag index run only when
+// d_flags holds a nonzero there
 void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles,
                      int64_t ntiles, const double *A, const double *B, double *C,
-                     int is_complex);
+                     int is_complex, const int *d_flags = nullptr);
 int gemm_f64_tile_m();
 int gemm_f64_tile_n();
 
@@ -307,6 +314,56 @@ T *dev_upload(Ctx *ctx, const std::vector<T> &v) {
   if (!v.empty()) ctx->stage_upload(p, v.data(), v.size() * sizeof(T));
   return p;
 }
+
+// Several work lists and scratch arrays of one launch in one device
+// allocation, its host part sent by one staging copy: a small launch costs
+// about as much host time as two of the copies it would otherwise queue.
+// add() / space() give offsets; at() the addresses after commit().
+class DevLists {
+ public:
+  template <class T>
+  size_t add(const std::vector<T> &v) {
+    return put(v.data(), v.size() * sizeof(T));
+  }
+  size_t zeros(size_t bytes) { return put(nullptr, bytes); }  // sent as zeros
+  size_t space(size_t bytes) {                                // not initialised
+    const size_t o = scratch_;
+    scratch_ += round(bytes);
+    return o | SPACE;
+  }
+  void commit(Ctx *ctx);
+  template <class T>
+  T *at(size_t o) const {
+    return reinterpret_cast<T *>(base_ + ((o & SPACE) ? sent_ + (o & ~SPACE) : o));
+  }
+  // stream-ordered release (also by the destructor)
+  void release() {
+    if (base_) dev_free(ctx_, base_);
+    base_ = nullptr;
+  }
+  DevLists() = default;
+  DevLists(const DevLists &) = delete;
+  DevLists &operator=(const DevLists &) = delete;
+  ~DevLists() { release(); }
+
+ private:
+  static constexpr size_t SPACE = size_t(1) << 63;
+  static size_t round(size_t b) { return (b + 255) & ~size_t(255); }
+  size_t put(const void *p, size_t bytes) {
+    const size_t o = sent_;
+    if (bytes) spans_.push_back({p, bytes, o});
+    sent_ += round(bytes);
+    return o;
+  }
+  struct Span {
+    const void *src;
+    size_t bytes, off;
+  };
+  std::vector<Span> spans_;
+  size_t sent_ = 0, scratch_ = 0;
+  char *base_ = nullptr;
+  Ctx *ctx_ = nullptr;
+};
 
 }  // namespace qs
 

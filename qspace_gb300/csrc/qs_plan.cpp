@@ -464,6 +464,7 @@ std::vector<TileDesc> make_tiles(const std::vector<int64_t> &grp,
         t.N = N;
         t.ldc = blk_ldc ? (*blk_ldc)[b] : std::max(M, 1);
         t.cblk = (int32_t)b;
+        t.flag = -1;
         tiles.push_back(t);
       }
   }

@@ -58,6 +58,7 @@ struct qs_grouped_plan {
   PairDesc *d_pairs = nullptr;  // FP64 path
   TileDesc *d_tiles = nullptr;
   int64_t ntiles = 0;
+  const int *d_flags = nullptr;  // tile flags of `split` (FP64 path)
   // shallow output blocks run directly (as in the one-shot calls); `main`
   // holds the other blocks (all of them when none is shallow)
   ShallowPlan shallow;
@@ -75,8 +76,10 @@ void launch_direct(qs_grouped_plan *p, const double *A, const double *B, double 
   if (p->main.pairs.empty()) return;
   if (p->o.prec == QS_PREC_SPLIT)
     split_plan_launch(p->ctx, p->split, A, B, C);
-  else
-    launch_gemm_f64(p->ctx, p->d_pairs, p->d_tiles, p->ntiles, A, B, C, p->g.cplx ? 1 : 0);
+  else {
+    if (p->split) split_plan_launch(p->ctx, p->split, A, B, C);
+    launch_gemm_f64(p->ctx, p->d_pairs, p->d_tiles, p->ntiles, A, B, C, p->g.cplx ? 1 : 0, p->d_flags);
+  }
 }
 
 SplitPlanHandle *make_split(qs_grouped_plan *p, int bits, SplitResult *r) {
@@ -257,6 +260,13 @@ qs_status qs_grouped_plan_create(qs_ctx *ctx, const qs_pair_list *pairs, const q
       std::vector<TileDesc> tiles =
           make_tiles(m.grp, m.bM, m.bN, m.coff, gemm_f64_tile_m(), gemm_f64_tile_n(), &m.bldc, &m.pairs);
       p->ntiles = (int64_t)tiles.size();
+      const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.cplx, {}, tiles);
+      if (tl.any) {
+        c->ensure_aux();
+        p->split = f64_tensor_plan_create(tl, m.pairs, m.grp, m.bM, m.bN, m.coff, m.bldc, m.cplx, p->d_flags);
+        if (!p->split)
+          for (TileDesc &t : tiles) t.flag = -1;
+      }
       QS_CUDA(cudaMalloc(&p->d_pairs, m.pairs.size() * sizeof(PairDesc)));
       QS_CUDA(cudaMemcpy(p->d_pairs, m.pairs.data(), m.pairs.size() * sizeof(PairDesc),
                          cudaMemcpyHostToDevice));

@@ -54,6 +54,31 @@ SplitResult run_split_static(Ctx *ctx, const std::vector<PairDesc> &pairs,
                              int forced_slices, double tol, const std::vector<int32_t> *blk_ldc,
                              uint8_t *scratch, size_t cap, int *err);
 
+// FP64-grade products on the tensor cores, for the plain FP64 path: digits of
+// 56 bits per operand, summed without rounding, with a certificate per output
+// that the truncation stays at the level of an FP64 sum.  Where it does not
+// (and where a line holds an infinity or NaN) the launch raises the flag of
+// the output's 64 x 64 FP64 tile, and the FP64 kernel recomputes it.
+struct F64TensorList {
+  std::vector<char> on;         // per block: computed by the tensor-core launch
+  std::vector<int32_t> fbase;   // per block: first tile flag
+  std::vector<std::pair<int64_t, int64_t>> chunks;  // block ranges of one launch each
+  int64_t nflags = 0;
+  bool any = false;
+};
+// The blocks of a list that the tensor-core launch takes (a property of the
+// block alone), except those marked in `skip`, and the flags of their tiles
+// (entered in `tiles`).
+F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
+                              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, bool cplx,
+                              const std::vector<char> &skip, std::vector<TileDesc> &tiles);
+// Runs them (strips and products); false when the device has no room for
+// their digits (nothing ran: the caller computes every tile in FP64).
+bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
+                    const std::vector<int64_t> &grp, const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
+                    const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, const double *A,
+                    const double *B, double *C, bool cplx, int *d_flags);
+
 // Reusable split plans (stable device addresses, for CUDA graph replay).
 struct SplitPlanHandle;
 std::vector<int> split_candidate_bits(double tol, int forced_slices);
@@ -62,6 +87,11 @@ SplitPlanHandle *split_plan_create(const std::vector<PairDesc> &pairs, const std
                                    const std::vector<int32_t> &blk_M, const std::vector<int32_t> &blk_N,
                                    const std::vector<int64_t> &c_off, const std::vector<int32_t> &blk_ldc,
                                    bool cplx, int forced_slices, double tol, int bits, SplitResult *res);
+// The FP64-grade form; nullptr when the device has no room for the digits.
+SplitPlanHandle *f64_tensor_plan_create(const F64TensorList &tl, const std::vector<PairDesc> &pairs,
+                                        const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
+                                        const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
+                                        const std::vector<int32_t> &bldc, bool cplx, const int *&d_flags);
 void split_plan_launch(Ctx *ctx, SplitPlanHandle *h, const double *A, const double *B, double *C);
 void split_plan_destroy(SplitPlanHandle *h);
 

@@ -1,0 +1,185 @@
+"""The plain FP64 path's tensor-core launch: outputs stay at the level of an
+FP64 sum entry by entry, whatever the operands hold.
+
+The bound is the one of an FP64 dot product of real depth n in any order,
+n u sum_k |a_ik b_kj| (u = 2^-53), times 4.3 for the digits' truncation (the
+certificate of the launch) plus one rounding of the result; operands that miss
+the certificate are recomputed by the FP64 kernel and meet the same bound."""
+import numpy as np
+import pytest
+
+from qspace_gb300.grouped import DeviceBatch, Packed
+
+U = 2.0 ** -53
+
+
+def _ops(rng, M, N, K, cplx):
+    a, b = rng.standard_normal((M, K)), rng.standard_normal((K, N))
+    if cplx:
+        a = a + 1j * rng.standard_normal((M, K))
+        b = b + 1j * rng.standard_normal((K, N))
+    return a, b
+
+
+def _stored(x, trans, conj):
+    """The array to store so that op(stored) = x."""
+    x = x.conj() if conj else x
+    return x.T if trans else x
+
+
+def _batch(ops, afac, blk, trans):
+    """DeviceBatch whose pair p computes afac ops[p][0] @ ops[p][1]."""
+    cplx = np.iscomplexobj(ops[0][0])
+    pk = Packed([a for a, _ in ops], [b for _, b in ops], afac, blk=blk, cplx=cplx)
+    pk.trans = np.asarray(trans, np.int32)
+    flat = lambda xs: np.concatenate([np.asarray(x, pk.abuf.dtype).reshape(-1, order="F") for x in xs])  # noqa: E731
+    pk.abuf = flat([_stored(a, t & 1, t & 4) for (a, _), t in zip(ops, trans)])
+    pk.bbuf = flat([_stored(b, t & 2, t & 8) for (_, b), t in zip(ops, trans)])
+    pk.lda = np.where(pk.trans & 1, pk.K, pk.M).astype(np.int32)
+    pk.ldb = np.where(pk.trans & 2, pk.N, pk.K).astype(np.int32)
+    return DeviceBatch(pk)
+
+
+def _reference(ops, afac, blk):
+    """Per block: the product in extended precision, sum |a||b| and depth."""
+    out = {}
+    for (a, b), f, g in zip(ops, afac, blk):
+        wide = np.clongdouble if np.iscomplexobj(a) else np.longdouble
+        fa = (a * f).astype(wide)       # the factor enters as the FP64 kernel applies it
+        c = fa @ b.astype(wide)
+        s = np.abs(a.real * f) @ np.abs(b.real) + np.abs(a.imag * f) @ np.abs(b.imag) + \
+            np.abs(a.real * f) @ np.abs(b.imag) + np.abs(a.imag * f) @ np.abs(b.real)
+        n = a.shape[1] * (2 if np.iscomplexobj(a) else 1)
+        if g in out:
+            c0, s0, n0 = out[g]
+            out[g] = (c0 + c, s0 + s, n0 + n)
+        else:
+            out[g] = (c, s, n)
+    return [out[g] for g in sorted(out)]
+
+
+def _check(got, ref):
+    for c, (r, s, n) in zip(got, ref):
+        d = c - r
+        err = np.maximum(np.abs(d.real), np.abs(d.imag)).astype(float)
+        # n + 1: the factor's rounding in FP64 (exact in the digits)
+        bound = 4.3 * (n + 1) * U * s + 2 * U * np.abs(r).astype(float)
+        assert np.all(err <= bound), float(np.max(err / np.maximum(bound, 1e-300)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("shape", [(64, 64, 48), (40, 70, 24), (65, 33, 96), (129, 31, 97), (1, 700, 130), (700, 1, 130),
+                                   (128, 32, 193), (63, 127, 512)])
+def test_f64_tensor_sizes(shape, cplx):
+    rng = np.random.default_rng(5)
+    M, N, K = shape
+    ks = [K, max(K // 3, 1), 1]
+    ops = [_ops(rng, M, N, k, cplx) for k in ks]
+    afac, blk = [0.75, -0.3137, 1.0], [0, 0, 0]
+    ref = _reference(ops, afac, blk)
+    norm = float(np.linalg.norm(ref[0][0].astype(complex)))
+    for trans in ([0, 0, 0], [1, 2, 3], [15, 7, 8]):
+        trans = [t if cplx else t & 3 for t in trans]
+        db = _batch(ops, afac, blk, trans)
+        db.run("fp64")
+        got = db.result()
+        _check(got, ref)
+        d = (got[0] - ref[0][0]).astype(complex)
+        assert np.linalg.norm(d) <= 4e-16 * np.sqrt(ref[0][2]) * norm
+        # the plan runs the same launches: same bits
+        plan = db.plan("fp64")
+        for _ in range(3):
+            db.dC.zero_()
+            db.torch.cuda.synchronize()
+            db.run_plan(plan)
+            assert np.array_equal(db.result()[0], got[0])
+        plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["graded", "sparse", "tiny_overlap", "zero_line", "huge", "subnormal", "factors"])
+def test_f64_tensor_hard_operands(kind):
+    """Entries of very different sizes, disjoint supports, extreme
+    exponents: every output keeps the FP64 bound."""
+    rng = np.random.default_rng(11)
+    M, N, K = 90, 75, 200
+    a, b = _ops(rng, M, N, K, False)
+    afac = [1.0, 0.5]
+    if kind == "graded":
+        a *= 10.0 ** -np.linspace(0, 30, K)[None, :]
+        b *= 10.0 ** -np.linspace(30, 0, K)[:, None]
+    elif kind == "sparse":
+        a *= rng.random((M, K)) < 0.02
+        b *= rng.random((K, N)) < 0.02
+    elif kind == "tiny_overlap":
+        a[:, K // 2:] *= 1e-14
+        b[:K // 2, :] = 0.0
+    elif kind == "zero_line":
+        a[7, :] = 0.0
+        b[:, 11] = 0.0
+        a[:, 5] = 0.0
+    elif kind == "huge":
+        a *= 1e200
+        b *= 1e-190
+        a[3, 3] = 1e307
+    elif kind == "subnormal":
+        a *= 1e-160
+        b *= 1e-150
+    else:
+        afac = [1e-290, 3.0]
+    ops = [(a, b), _ops(rng, M, N, 64, False)]
+    if kind in ("huge", "subnormal"):
+        ops = ops[:1]
+    afac, blk = afac[:len(ops)], [0] * len(ops)
+    db = _batch(ops, afac, blk, [0] * len(ops))
+    db.run("fp64")
+    if kind == "subnormal":  # results below the normal range: absolute spacing 2^-1074
+        r, s, n = _reference(ops, afac, blk)[0]
+        err = np.abs(db.result()[0] - r).astype(float)
+        assert np.all(err <= 4.3 * (n + 1) * U * s + 2 * U * np.abs(r).astype(float) + n * 2.0 ** -1074)
+    else:
+        _check(db.result(), _reference(ops, afac, blk))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cplx", [False, True])
+def test_f64_tensor_nonfinite(cplx):
+    """Infinities and NaN in the operands reach the outputs that FP64
+    arithmetic gives them, and no others."""
+    rng = np.random.default_rng(3)
+    M, N, K = 150, 140, 80
+    a, b = _ops(rng, M, N, K, cplx)
+    a[17, 5] = np.nan
+    a[70, 9] = np.inf
+    b[3, 100] = -np.inf
+    ok = np.ones((M, N), bool)
+    ok[17, :] = ok[70, :] = False
+    ok[:, 100] = False
+    db = _batch([(a, b)], [1.0], [0], [0])
+    db.run("fp64")
+    c = db.result()[0]
+    assert np.all(np.isfinite(c[ok])) and not np.any(np.isfinite(c[~ok]))
+    a2, b2 = np.where(np.isfinite(a), a, 0), np.where(np.isfinite(b), b, 0)
+    r, s, n = _reference([(a2, b2)], [1.0], [0])[0]
+    err = np.abs(c[ok] - r[ok]).astype(float)
+    assert np.all(err <= 4.3 * 2 * (n + 1) * U * s[ok])
+    if not cplx:
+        with np.errstate(invalid="ignore"):
+            w = a @ b
+        assert np.array_equal(np.isnan(c), np.isnan(w)) and np.array_equal(c[np.isinf(w)], w[np.isinf(w)])
+
+
+@pytest.mark.gpu
+def test_f64_tensor_alone_and_in_a_list():
+    """A block gives the same bits alone and in a list of others."""
+    rng = np.random.default_rng(8)
+    sizes = [(100, 90, 60), (8, 8, 8), (300, 20, 333), (64, 64, 47), (33, 257, 129)]
+    ops = [_ops(rng, *s, True) for s in sizes]
+    afac = list(rng.uniform(-1, 1, len(ops)))
+    db = _batch(ops, afac, list(range(len(ops))), [0] * len(ops))
+    db.run("fp64")
+    for p, c in enumerate(db.result()):
+        one = _batch([ops[p]], [afac[p]], [0], [0])
+        one.run("fp64")
+        assert np.array_equal(one.result()[0], c)
