@@ -2,20 +2,28 @@
 //
 // Replaces the per-pair dgemm/zgemm of contractDATA_group (Source/
 // QSpace_aux.cc:27-355 -> wbarray::contract Source/wbarray.cc:3389-3500 ->
-// DZGEMM Source/wbarray_blas.cc:121-213).  One CTA owns one 64x64 tile of one
-// output block and sums all block pairs of that block in plan order, so the
-// result is deterministic and needs no atomics.  The K loop stages 64xKC
-// panels of op(A) and KCx64 panels of op(B) in shared memory (coalesced
-// loads in either storage order); each thread accumulates a 4x4 sub-tile in
-// registers with FP64 FMAs (GB300's FP64 rate, not memory, bounds this path).
-#include <type_traits>
+// DZGEMM Source/wbarray_blas.cc:121-213) for the output blocks that the
+// tensor-core launch leaves (small or shallow sums) and for the tiles whose
+// flag that launch raised.  One CTA owns one 32x32 tile of one output block
+// and sums all block pairs of that block in plan order, so the result is
+// deterministic and needs no atomics.  The K loop stages 32xKC panels of
+// op(A) and KCx32 panels of op(B) in shared memory (coalesced loads in either
+// storage order), the next panel's loads in flight behind the current one's
+// arithmetic; each thread accumulates a 2x2 sub-tile with FP64 FMAs.
+//
+// GB300's FP64 pipe (about 2 multiply-adds per clock and SM) bounds this
+// kernel: a panel step of a full tile keeps it busy for 540 clocks, against
+// 512 or 1024 bytes loaded, so a small tile costs no bandwidth.  32x32 tiles
+// spread a list of small blocks over four times the SMs of 64x64 ones.
+#include <algorithm>
 
 #include "qs_internal.h"
 
 namespace qs {
 
 namespace {
-constexpr int TM = 64, TN = 64;
+constexpr int TM = F64_TILE, TN = F64_TILE;
+constexpr int THREADS = 256;  // 16 x 16, two rows and two columns each
 
 template <bool CPLX>
 struct Elem;
@@ -47,9 +55,10 @@ struct Elem<true> {
 };
 
 // One staged K panel into the accumulators, for the NI x NJ leading 16 x 16
-// groups of the tile and the first kn of its KC steps (CTA-uniform bounds).
+// groups of the tile and the first kn of its KC steps (CTA-uniform bounds):
+// padding would cost the FP64 pipe as much as real work.
 template <class E, int NI, int NJ, int KC>
-__device__ __forceinline__ void panel_fma(typename E::T (&acc)[4][4], const typename E::T (*As)[TM + 1],
+__device__ __forceinline__ void panel_fma(typename E::T (&acc)[2][2], const typename E::T (*As)[TM + 1],
                                           const typename E::T (*Bs)[TN + 1], int tx, int ty, int kn) {
   using T = typename E::T;
 #pragma unroll
@@ -68,116 +77,158 @@ __device__ __forceinline__ void panel_fma(typename E::T (&acc)[4][4], const type
   }
 }
 
+template <class E>
+struct Panels {
+  typename E::T a[E::KC][TM + 1], b[E::KC][TN + 1];
+};
+
 template <bool CPLX>
-__global__ void __launch_bounds__(256)
-gemm_f64_kernel(const PairDesc *__restrict__ pairs, const TileDesc *__restrict__ tiles,
-                const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C,
-                const int *__restrict__ flags) {
+__device__ __forceinline__ void tile_product(const TileDesc &t, const PairDesc *__restrict__ pairs,
+                                             const double *__restrict__ A, const double *__restrict__ B,
+                                             double *__restrict__ C, Panels<Elem<CPLX>> &sm) {
   using E = Elem<CPLX>;
   using T = typename E::T;
   constexpr int KC = E::KC;
-  __shared__ T As[KC][TM + 1];
-  __shared__ T Bs[KC][TN + 1];
-
-  const TileDesc t = tiles[blockIdx.x];
-  if (t.flag >= 0 && !flags[t.flag]) return;  // the tensor-core launch has computed this tile
+  constexpr int NL = TM * KC / THREADS;  // elements of each panel per thread
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
-  const int shape = (min(4, (t.M - t.m0 + 15) / 16) - 1) * 4 + (min(4, (t.N - t.n0 + 15) / 16) - 1);
+  const bool two_rows = t.M - t.m0 > 16, two_cols = t.N - t.n0 > 16;
 
-  T acc[4][4];
+  T acc[2][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = E::zero();
+    for (int j = 0; j < 2; ++j) acc[i][j] = E::zero();
 
-  for (int p = t.p0; p < t.p1; ++p) {
+  // panel (p, k0) into registers; (mm, kk) / (nn, kk) of element e follow the
+  // operand's fast index
+  T va[NL], vb[NL];
+  bool ta = false, tb = false;
+  auto fetch = [&](int p, int k0) {
     const PairDesc pd = pairs[p];
-    const bool ta = pd.trans & 1, tb = pd.trans & 2;
-    const bool ca = pd.trans & 4, cb = pd.trans & 8;
-    for (int k0 = 0; k0 < pd.K; k0 += KC) {
+    ta = pd.trans & 1;
+    tb = pd.trans & 2;
+#pragma unroll
+    for (int u = 0; u < NL; ++u) {
+      const int e = tid + u * THREADS;
       // op(A)(m,k): stored M x K (m fastest) or K x M (k fastest)
-#pragma unroll
-      for (int e = tid; e < TM * KC; e += 256) {
-        int mm, kk;
-        if (ta) { kk = e % KC; mm = e / KC; }
-        else    { mm = e % TM; kk = e / TM; }
-        const int m = t.m0 + mm, k = k0 + kk;
-        T v = E::zero();
-        if (m < pd.M && k < pd.K)
-          v = E::load(A, pd.a_off + (ta ? (int64_t)k + (int64_t)m * pd.lda
-                                        : (int64_t)m + (int64_t)k * pd.lda), ca, pd.afac);
-        As[kk][mm] = v;
-      }
+      const int ka = k0 + (ta ? e % KC : e / TM), m = t.m0 + (ta ? e / KC : e % TM);
+      va[u] = E::zero();
+      if (m < pd.M && ka < pd.K)
+        va[u] = E::load(A, pd.a_off + (ta ? (int64_t)ka + (int64_t)m * pd.lda : (int64_t)m + (int64_t)ka * pd.lda),
+                        pd.trans & 4, pd.afac);
       // op(B)(k,n): stored K x N (k fastest) or N x K (n fastest)
-#pragma unroll
-      for (int e = tid; e < TN * KC; e += 256) {
-        int nn, kk;
-        if (tb) { nn = e % TN; kk = e / TN; }
-        else    { kk = e % KC; nn = e / KC; }
-        const int n = t.n0 + nn, k = k0 + kk;
-        T v = E::zero();
-        if (n < pd.N && k < pd.K)
-          v = E::load(B, pd.b_off + (tb ? (int64_t)n + (int64_t)k * pd.ldb
-                                        : (int64_t)k + (int64_t)n * pd.ldb), cb, 1.0);
-        Bs[kk][nn] = v;
-      }
-      __syncthreads();
-      // only the 16-row / 16-column groups of the tile that hold outputs
-      // of the block, and only the pair's own K steps: the FP64 pipe bounds
-      // this kernel, so the padding a 64 x 64 tile carries on small blocks
-      // would cost as much as real work
-      const int kn = min(KC, pd.K - k0);
-      switch (shape) {
-        case 0: panel_fma<E, 1, 1, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 1: panel_fma<E, 1, 2, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 2: panel_fma<E, 1, 3, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 3: panel_fma<E, 1, 4, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 4: panel_fma<E, 2, 1, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 5: panel_fma<E, 2, 2, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 6: panel_fma<E, 2, 3, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 7: panel_fma<E, 2, 4, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 8: panel_fma<E, 3, 1, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 9: panel_fma<E, 3, 2, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 10: panel_fma<E, 3, 3, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 11: panel_fma<E, 3, 4, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 12: panel_fma<E, 4, 1, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 13: panel_fma<E, 4, 2, KC>(acc, As, Bs, tx, ty, kn); break;
-        case 14: panel_fma<E, 4, 3, KC>(acc, As, Bs, tx, ty, kn); break;
-        default: panel_fma<E, 4, 4, KC>(acc, As, Bs, tx, ty, kn); break;
-      }
-      __syncthreads();
+      const int kb = k0 + (tb ? e / TN : e % KC), n = t.n0 + (tb ? e % TN : e / KC);
+      vb[u] = E::zero();
+      if (n < pd.N && kb < pd.K)
+        vb[u] = E::load(B, pd.b_off + (tb ? (int64_t)n + (int64_t)kb * pd.ldb : (int64_t)kb + (int64_t)n * pd.ldb),
+                        pd.trans & 8, 1.0);
     }
+    return pd.K;
+  };
+
+  int p = t.p0, k0 = 0, K = 0;
+  while (p < t.p1 && (K = pairs[p].K) <= 0) ++p;
+  if (p < t.p1) fetch(p, 0);
+  while (p < t.p1) {
+#pragma unroll
+    for (int u = 0; u < NL; ++u) {
+      const int e = tid + u * THREADS;
+      sm.a[ta ? e % KC : e / TM][ta ? e / KC : e % TM] = va[u];
+      sm.b[tb ? e / TN : e % KC][tb ? e % TN : e / KC] = vb[u];
+    }
+    const int kn = min(KC, K - k0);
+    // the next panel: of this pair, or of the next one that has depth
+    k0 += KC;
+    if (k0 >= K) {
+      k0 = 0;
+      do ++p;
+      while (p < t.p1 && (K = pairs[p].K) <= 0);
+    }
+    __syncthreads();
+    if (p < t.p1) fetch(p, k0);
+    if (two_rows) {
+      if (two_cols) panel_fma<E, 2, 2, KC>(acc, sm.a, sm.b, tx, ty, kn);
+      else panel_fma<E, 2, 1, KC>(acc, sm.a, sm.b, tx, ty, kn);
+    } else {
+      if (two_cols) panel_fma<E, 1, 2, KC>(acc, sm.a, sm.b, tx, ty, kn);
+      else panel_fma<E, 1, 1, KC>(acc, sm.a, sm.b, tx, ty, kn);
+    }
+    __syncthreads();
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 2; ++j) {
     const int n = t.n0 + ty + 16 * j;
     if (n >= t.N) continue;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 2; ++i) {
       const int m = t.m0 + tx + 16 * i;
       if (m < t.M) E::store(C, t.c_off + (int64_t)m + (int64_t)n * t.ldc, acc[i][j]);
     }
   }
 }
+
+// CTAs 0 .. ntiles-1 compute the listed tiles.  The others walk the flags of
+// the tensor-core launch (ncells of them, one per tile of the checked blocks,
+// column of tiles by column) and recompute the tiles whose flag is raised;
+// usually none is, and the walk takes about 2 us.
+template <bool CPLX>
+__global__ void __launch_bounds__(THREADS)
+gemm_f64_kernel(const PairDesc *__restrict__ pairs, const TileDesc *__restrict__ tiles, int ntiles,
+                const TileDesc *__restrict__ checked, int nchecked, int ncells, const int *__restrict__ flags,
+                const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C) {
+  __shared__ Panels<Elem<CPLX>> sm;
+  __shared__ unsigned raised[THREADS / 32];
+  const int tid = threadIdx.x;
+  if ((int)blockIdx.x < ntiles) {
+    tile_product<CPLX>(tiles[blockIdx.x], pairs, A, B, C, sm);
+    return;
+  }
+  const int w = (int)blockIdx.x - ntiles, G = (int)gridDim.x - ntiles;
+  for (int64_t c0 = w; c0 < ncells; c0 += (int64_t)THREADS * G) {
+    const int64_t c = c0 + (int64_t)tid * G;  // cells c0, c0 + G, ...: thread t looks at the t-th
+    const bool f = c < ncells && flags[c] != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, f);
+    if ((tid & 31) == 0) raised[tid >> 5] = m;
+    if (__syncthreads_or(f)) {
+      for (int u = 0; u < THREADS; ++u) {
+        if (!((raised[u >> 5] >> (u & 31)) & 1u)) continue;
+        const int cell = (int)(c0 + (int64_t)u * G);
+        int lo = 0, hi = nchecked - 1;  // the block: last one whose first flag is <= cell
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (checked[mid].flag <= cell) lo = mid;
+          else hi = mid - 1;
+        }
+        TileDesc t = checked[lo];
+        const int rows = (t.M + TM - 1) / TM, i = cell - t.flag;
+        t.m0 = (i % rows) * TM;
+        t.n0 = (i / rows) * TN;
+        tile_product<CPLX>(t, pairs, A, B, C, sm);
+      }
+    }
+    __syncthreads();  // `raised` is rewritten by the next round
+  }
+}
 }  // namespace
 
-int gemm_f64_tile_m() { return TM; }
-int gemm_f64_tile_n() { return TN; }
-
-void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles,
-                     int64_t ntiles, const double *A, const double *B, double *C,
-                     int is_complex, const int *d_flags) {
-  if (ntiles <= 0) return;
-  if (ntiles > 0x7fffffff) fail(QS_ERR_SHAPE, "gemm_f64: too many tiles");
-  if (!d_flags) {  // else the marks of the tensor-core launch before it stand
+void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles, int64_t ntiles,
+                     const TileDesc *d_checked, int64_t nchecked, int64_t ncells, const int *d_flags,
+                     const double *A, const double *B, double *C, int is_complex) {
+  const int64_t walkers = nchecked > 0 ? std::min<int64_t>(ncells, (int64_t)std::max(ctx->num_sms, 1) * 4) : 0;
+  if (ntiles + walkers <= 0) return;
+  if (ntiles + walkers > 0x7fffffff || ncells > 0x7fffffff) fail(QS_ERR_SHAPE, "gemm_f64: too many tiles");
+  if (!walkers) {  // else the marks of the tensor-core launch before it stand
     ctx->mark(0);
     ctx->mark(1);
   }
+  const unsigned grid = (unsigned)(ntiles + walkers);
   if (is_complex)
-    gemm_f64_kernel<true><<<(unsigned)ntiles, 256, 0, ctx->stream>>>(d_pairs, d_tiles, A, B, C, d_flags);
+    gemm_f64_kernel<true><<<grid, THREADS, 0, ctx->stream>>>(d_pairs, d_tiles, (int)ntiles, d_checked, (int)nchecked,
+                                                             (int)ncells, d_flags, A, B, C);
   else
-    gemm_f64_kernel<false><<<(unsigned)ntiles, 256, 0, ctx->stream>>>(d_pairs, d_tiles, A, B, C, d_flags);
+    gemm_f64_kernel<false><<<grid, THREADS, 0, ctx->stream>>>(d_pairs, d_tiles, (int)ntiles, d_checked,
+                                                              (int)nchecked, (int)ncells, d_flags, A, B, C);
   QS_LAUNCHED(ctx);
   ctx->mark(2);
 }

@@ -1120,7 +1120,8 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
                 const int lr = i_glob >> rdup, lc = j >> cdup;
                 const bool sw = T.splits & 4;
                 const int rows = sw ? T.N >> cdup : T.Mr >> rdup;  // of C
-                flags[T.fbase + ((sw ? lc : lr) >> 6) + ((sw ? lr : lc) >> 6) * ((rows + 63) >> 6)] = 1;
+                flags[T.fbase + (sw ? lc : lr) / F64_TILE +
+                      (sw ? lr : lc) / F64_TILE * ((rows + F64_TILE - 1) / F64_TILE)] = 1;
               }
             } else {
               const long long V = (long long)(((unsigned long long)Vh[jj] << 32) + Vl[jj]);
@@ -1839,8 +1840,9 @@ constexpr double F64T_WORK = 65536.0;
 constexpr int64_t F64T_CHUNK_BYTES = int64_t(2) << 30, F64T_BLOCK_BYTES = int64_t(8) << 30;
 
 F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
-                              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, bool cplx,
-                              const std::vector<char> &skip, std::vector<TileDesc> &tiles) {
+                              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
+                              const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
+                              const std::vector<char> &skip) {
   F64TensorList tl;
   const int64_t nb = (int64_t)bM.size();
   const int64_t cm = cplx ? 2 : 1;
@@ -1866,12 +1868,21 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
     // either operand's real form may be the duplicated one
     const int64_t bytes = (up(M * cm, TMS) + up(N * cm, TMS)) * kpad * (HP_DIGITS + 1) * 2;
     if (bytes > F64T_BLOCK_BYTES) continue;
-    const int64_t cells = ((M + 63) / 64) * ((N + 63) / 64);
+    const int64_t cells = ((M + F64_TILE - 1) / F64_TILE) * ((N + F64_TILE - 1) / F64_TILE);
     if (tl.nflags + cells > INT32_MAX) continue;
     tl.on[g] = 1;
     tl.fbase[g] = (int32_t)tl.nflags;
+    TileDesc t{};
+    t.c_off = coff[g];
+    t.p0 = (int32_t)grp[g];
+    t.p1 = (int32_t)grp[g + 1];
+    t.M = bM[g];
+    t.N = bN[g];
+    t.ldc = bldc ? (*bldc)[g] : std::max(bM[g], 1);
+    t.cblk = (int32_t)g;
+    t.flag = tl.fbase[g];
+    tl.checked.push_back(t);
     tl.nflags += cells;
-    tl.any = true;
     if (chunk_bytes && chunk_bytes + bytes > F64T_CHUNK_BYTES) {
       tl.chunks.push_back({chunk0, g});
       chunk0 = g;
@@ -1879,10 +1890,7 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
     }
     chunk_bytes += bytes;
   }
-  if (!tl.any) return tl;
-  tl.chunks.push_back({chunk0, nb});
-  for (TileDesc &t : tiles)
-    if (tl.on[t.cblk]) t.flag = tl.fbase[t.cblk] + t.m0 / 64 + (t.n0 / 64) * ((t.M + 63) / 64);
+  if (!tl.checked.empty()) tl.chunks.push_back({chunk0, nb});
   return tl;
 }
 

@@ -117,7 +117,7 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
   const bool deep = reinterpret_cast<uintptr_t>(C) % eb == 0 && split_deep(pairs, grp, bM, bN, coff, bldc, ds);
   double *T = nullptr;
   DeepReduce *dr = nullptr;
-  DevLists lists;
+  DevLists lists, more;
   try {
     if (deep) {
       T = dev_alloc<double>(ctx, (size_t)std::max<int64_t>(ds.temp_elems, 1) * (cplx ? 2 : 1));
@@ -128,35 +128,38 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
     const std::vector<int32_t> &mm = deep ? ds.bM : bM, &nn = deep ? ds.bN : bN;
     const std::vector<int32_t> *ll = deep ? &ds.bldc : bldc;
     // parts of deep blocks with a few outputs: one CTA per output element
-    // (run_dot); the others through the 64 x 64 tiles
+    // (run_dot); larger blocks on the tensor cores, with the FP64 tiles as
+    // their net; the others through the FP64 tiles
     std::vector<int64_t> small;
-    std::vector<TileDesc> tiles;
-    std::vector<char> is_small(mm.size(), 0);
-    {
-      std::vector<TileDesc> all = make_tiles(gg, mm, nn, cc, gemm_f64_tile_m(), gemm_f64_tile_n(), ll, &pp);
-      for (size_t b = 0; b < mm.size(); ++b)
-        if (deep && ds.part[b] && (int64_t)mm[b] * nn[b] <= DOT_OUTPUTS) {
-          is_small[b] = 1;
-          small.push_back((int64_t)b);
-        }
-      for (const TileDesc &t : all)
-        if (!is_small[t.cblk]) tiles.push_back(t);
-    }
-    run_dot(ctx, pp, gg, mm, nn, cc, ll, small, A, B, C, cplx);
-    // larger blocks on the tensor cores, with the FP64 tiles as their net;
-    // the tile lists go first, as the tensor-core launch raises their flags
-    const F64TensorList tl = plan_f64_tensor(pp, gg, mm, nn, cplx, is_small, tiles);
-    if (!tiles.empty()) {
-      const size_t sp = lists.add(pp), st = lists.add(tiles), sf = lists.zeros((size_t)tl.nflags * sizeof(int));
-      lists.commit(ctx);
-      int *flags = tl.any ? lists.at<int>(sf) : nullptr;
-      if (tl.any && !run_f64_tensor(ctx, tl, pp, gg, mm, nn, cc, ll, A, B, C, cplx, flags)) {
-        // no room for the digits: every tile in FP64
-        for (TileDesc &t : tiles) t.flag = -1;
-        ctx->stage_upload(lists.at<TileDesc>(st), tiles.data(), tiles.size() * sizeof(TileDesc));
+    std::vector<char> skip(mm.size(), 0);
+    for (size_t b = 0; b < mm.size(); ++b)
+      if (deep && ds.part[b] && (int64_t)mm[b] * nn[b] <= DOT_OUTPUTS) {
+        skip[b] = 1;
+        small.push_back((int64_t)b);
       }
-      launch_gemm_f64(ctx, lists.at<PairDesc>(sp), lists.at<TileDesc>(st), (int64_t)tiles.size(), A, B, C,
-                      cplx ? 1 : 0, flags);
+    run_dot(ctx, pp, gg, mm, nn, cc, ll, small, A, B, C, cplx);
+    const F64TensorList tl = plan_f64_tensor(pp, gg, mm, nn, cc, ll, cplx, skip);
+    const std::vector<char> dots = skip;
+    for (size_t b = 0; b < mm.size(); ++b) skip[b] |= tl.on[b];
+    std::vector<TileDesc> tiles = make_tiles(gg, mm, nn, cc, F64_TILE, F64_TILE, ll, &pp, &skip);
+    if (!tiles.empty() || !tl.checked.empty()) {
+      // the flags are cleared with the lists, before the launch that raises them
+      const size_t sp = lists.add(pp), st = lists.add(tiles), sc = lists.add(tl.checked),
+                   sf = lists.zeros((size_t)tl.nflags * sizeof(int));
+      lists.commit(ctx);
+      int64_t nchecked = (int64_t)tl.checked.size();
+      if (nchecked && !run_f64_tensor(ctx, tl, pp, gg, mm, nn, cc, ll, A, B, C, cplx, lists.at<int>(sf))) {
+        // no room for the digits: every tile in FP64
+        tiles = make_tiles(gg, mm, nn, cc, F64_TILE, F64_TILE, ll, &pp, &dots);
+        nchecked = 0;
+        const size_t all = more.add(tiles);
+        more.commit(ctx);
+        launch_gemm_f64(ctx, lists.at<PairDesc>(sp), more.at<TileDesc>(all), (int64_t)tiles.size(), nullptr, 0, 0,
+                        nullptr, A, B, C, cplx ? 1 : 0);
+      } else {
+        launch_gemm_f64(ctx, lists.at<PairDesc>(sp), lists.at<TileDesc>(st), (int64_t)tiles.size(),
+                        lists.at<TileDesc>(sc), nchecked, tl.nflags, lists.at<int>(sf), A, B, C, cplx ? 1 : 0);
+      }
     }
     if (deep) {
       dr = dev_upload(ctx, ds.red);

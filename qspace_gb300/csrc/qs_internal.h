@@ -215,7 +215,7 @@ struct TileDesc {
   int32_t M, N;
   int32_t ldc;
   int32_t cblk;
-  int32_t flag;   // computed only when this flag is raised (-1: always)
+  int32_t flag;   // first tile flag of a checked block (launch_gemm_f64)
   int32_t pad_;
 };
 static_assert(sizeof(TileDesc) == 48, "TileDesc layout");
@@ -265,13 +265,13 @@ void launch_permute(Ctx *ctx, const PermDesc *d_desc, const int64_t *d_chunk_blk
                     const double *in, double *out, int is_complex, int chunk_elems);
 
 // qs_gemm_f64.cu -- plain FP64 grouped GEMM (deterministic: one CTA owns an
-// output tile, pairs summed in order); tiles with a flag index run only when
-// d_flags holds a nonzero there
-void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles,
-                     int64_t ntiles, const double *A, const double *B, double *C,
-                     int is_complex, const int *d_flags = nullptr);
-int gemm_f64_tile_m();
-int gemm_f64_tile_n();
+// output tile, pairs summed in order) of the listed tiles, and of the tiles of
+// the blocks in d_checked whose flag is raised (each entry describes a block:
+// m0 = n0 = 0, `flag` the index of its first tile's flag; ascending)
+constexpr int F64_TILE = 32;
+void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles, int64_t ntiles,
+                     const TileDesc *d_checked, int64_t nchecked, int64_t ncells, const int *d_flags,
+                     const double *A, const double *B, double *C, int is_complex);
 
 // qs_permute.cu -- per-block "all zero" test for SkipZeroData, and the
 // real -> complex widening of an operand arena

@@ -447,10 +447,12 @@ std::vector<TileDesc> make_tiles(const std::vector<int64_t> &grp,
                                  const std::vector<int32_t> &blk_M,
                                  const std::vector<int32_t> &blk_N,
                                  const std::vector<int64_t> &c_off, int tm, int tn,
-                                 const std::vector<int32_t> *blk_ldc, const std::vector<PairDesc> *pairs) {
+                                 const std::vector<int32_t> *blk_ldc, const std::vector<PairDesc> *pairs,
+                                 const std::vector<char> *skip) {
   std::vector<TileDesc> tiles;
   const int64_t nb = (int64_t)blk_M.size();
   for (int64_t b = 0; b < nb; ++b) {
+    if (skip && (*skip)[b]) continue;
     const int32_t M = blk_M[b], N = blk_N[b];
     for (int32_t n0 = 0; n0 < N; n0 += tn)
       for (int32_t m0 = 0; m0 < M; m0 += tm) {
@@ -464,7 +466,6 @@ std::vector<TileDesc> make_tiles(const std::vector<int64_t> &grp,
         t.N = N;
         t.ldc = blk_ldc ? (*blk_ldc)[b] : std::max(M, 1);
         t.cblk = (int32_t)b;
-        t.flag = -1;
         tiles.push_back(t);
       }
   }

@@ -80,13 +80,14 @@ ContractPlan plan_contract(const QMeta &A, const char *ia, const QMeta &B,
 // Tiles of the grouped GEMM over the plan's output blocks; with `pairs`,
 // ordered by estimated work, largest first (the summed depth of the block
 // times the tile's 16 x 16 groups that hold outputs), so that the tail of
-// the launch is made of short tiles.
+// the launch is made of short tiles.  Blocks marked in `skip` get none.
 std::vector<TileDesc> make_tiles(const std::vector<int64_t> &grp,
                                  const std::vector<int32_t> &blk_M,
                                  const std::vector<int32_t> &blk_N,
                                  const std::vector<int64_t> &c_off, int tm, int tn,
                                  const std::vector<int32_t> *blk_ldc = nullptr,
-                                 const std::vector<PairDesc> *pairs = nullptr);
+                                 const std::vector<PairDesc> *pairs = nullptr,
+                                 const std::vector<char> *skip = nullptr);
 
 // Permutation descriptors: out block = permute(in block, perm) [+conj].
 std::vector<PermDesc> make_perm_descs(const QMeta &in, const std::vector<int> &perm,

@@ -58,7 +58,10 @@ struct qs_grouped_plan {
   PairDesc *d_pairs = nullptr;  // FP64 path
   TileDesc *d_tiles = nullptr;
   int64_t ntiles = 0;
-  const int *d_flags = nullptr;  // tile flags of `split` (FP64 path)
+  // FP64 path: blocks of `split` whose tiles are recomputed when flagged
+  TileDesc *d_checked = nullptr;
+  int64_t nchecked = 0, ncells = 0;
+  const int *d_flags = nullptr;
   // shallow output blocks run directly (as in the one-shot calls); `main`
   // holds the other blocks (all of them when none is shallow)
   ShallowPlan shallow;
@@ -78,7 +81,8 @@ void launch_direct(qs_grouped_plan *p, const double *A, const double *B, double 
     split_plan_launch(p->ctx, p->split, A, B, C);
   else {
     if (p->split) split_plan_launch(p->ctx, p->split, A, B, C);
-    launch_gemm_f64(p->ctx, p->d_pairs, p->d_tiles, p->ntiles, A, B, C, p->g.cplx ? 1 : 0, p->d_flags);
+    launch_gemm_f64(p->ctx, p->d_pairs, p->d_tiles, p->ntiles, p->d_checked, p->nchecked, p->ncells, p->d_flags, A, B,
+                    C, p->g.cplx ? 1 : 0);
   }
 }
 
@@ -257,22 +261,27 @@ qs_status qs_grouped_plan_create(qs_ctx *ctx, const qs_pair_list *pairs, const q
   } else if (p->o.prec == QS_PREC_FP64) {
     if (!p->main.pairs.empty()) {
       const GroupedPlan &m = p->main;
-      std::vector<TileDesc> tiles =
-          make_tiles(m.grp, m.bM, m.bN, m.coff, gemm_f64_tile_m(), gemm_f64_tile_n(), &m.bldc, &m.pairs);
-      p->ntiles = (int64_t)tiles.size();
-      const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.cplx, {}, tiles);
-      if (tl.any) {
+      const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.coff, &m.bldc, m.cplx, {});
+      if (!tl.checked.empty()) {
         c->ensure_aux();
         p->split = f64_tensor_plan_create(tl, m.pairs, m.grp, m.bM, m.bN, m.coff, m.bldc, m.cplx, p->d_flags);
-        if (!p->split)
-          for (TileDesc &t : tiles) t.flag = -1;
       }
-      QS_CUDA(cudaMalloc(&p->d_pairs, m.pairs.size() * sizeof(PairDesc)));
-      QS_CUDA(cudaMemcpy(p->d_pairs, m.pairs.data(), m.pairs.size() * sizeof(PairDesc),
-                         cudaMemcpyHostToDevice));
-      QS_CUDA(cudaMalloc(&p->d_tiles, std::max<size_t>(tiles.size(), 1) * sizeof(TileDesc)));
-      if (!tiles.empty())
-        QS_CUDA(cudaMemcpy(p->d_tiles, tiles.data(), tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice));
+      // every tile in FP64 when there is no room for the digits
+      const std::vector<TileDesc> tiles =
+          make_tiles(m.grp, m.bM, m.bN, m.coff, F64_TILE, F64_TILE, &m.bldc, &m.pairs, p->split ? &tl.on : nullptr);
+      auto put = [](auto *&d, const auto &v) {
+        if (v.empty()) return;
+        QS_CUDA(cudaMalloc(&d, v.size() * sizeof(v[0])));
+        QS_CUDA(cudaMemcpy(d, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
+      };
+      p->ntiles = (int64_t)tiles.size();
+      put(p->d_pairs, m.pairs);
+      put(p->d_tiles, tiles);
+      if (p->split) {
+        p->nchecked = (int64_t)tl.checked.size();
+        p->ncells = tl.nflags;
+        put(p->d_checked, tl.checked);
+      }
     }
   } else {
     fail(QS_ERR_ARG, "unknown precision mode %d", p->o.prec);
@@ -328,6 +337,7 @@ void qs_grouped_plan_destroy(qs_grouped_plan *p) {
   shallow_release(p->shallow);
   if (p->d_pairs) cudaFree(p->d_pairs);
   if (p->d_tiles) cudaFree(p->d_tiles);
+  if (p->d_checked) cudaFree(p->d_checked);
   delete p;
 }
 

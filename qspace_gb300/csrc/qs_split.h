@@ -58,20 +58,20 @@ SplitResult run_split_static(Ctx *ctx, const std::vector<PairDesc> &pairs,
 // 56 bits per operand, summed without rounding, with a certificate per output
 // that the truncation stays at the level of an FP64 sum.  Where it does not
 // (and where a line holds an infinity or NaN) the launch raises the flag of
-// the output's 64 x 64 FP64 tile, and the FP64 kernel recomputes it.
+// the output's FP64 tile (F64_TILE), and the FP64 kernel recomputes it.
 struct F64TensorList {
   std::vector<char> on;         // per block: computed by the tensor-core launch
   std::vector<int32_t> fbase;   // per block: first tile flag
   std::vector<std::pair<int64_t, int64_t>> chunks;  // block ranges of one launch each
+  std::vector<TileDesc> checked;  // the blocks as launch_gemm_f64 takes them
   int64_t nflags = 0;
-  bool any = false;
 };
 // The blocks of a list that the tensor-core launch takes (a property of the
-// block alone), except those marked in `skip`, and the flags of their tiles
-// (entered in `tiles`).
+// block alone), except those marked in `skip`.
 F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
-                              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, bool cplx,
-                              const std::vector<char> &skip, std::vector<TileDesc> &tiles);
+                              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
+                              const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
+                              const std::vector<char> &skip);
 // Runs them (strips and products); false when the device has no room for
 // their digits (nothing ran: the caller computes every tile in FP64).
 bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
