@@ -787,7 +787,8 @@ __device__ __forceinline__ void fold_groups(uint32_t set_base, int cbase, int b,
 // the digit products left out -- are below K 2^(E_i+F_j) 2^-54.9, so a sum of
 // at least full scale / 16 keeps them within 4.3 K u sum_k |a_ik b_kj|
 // (u = 2^-53; an FP64 dot product is bounded by K u of the same sum).
-// Normally distributed entries pass for sums of about 48 terms on.
+// Normally distributed entries pass from nine terms on: 4e-6 of the outputs
+// miss it at nine terms, none of 10^7 at sixteen.
 constexpr float CERT_MIN = 65536.0f / 16.0f;
 
 // FP64-grade fold (S digits, two 64-bit words): the groups 0..HG-1 into Vh
@@ -1826,18 +1827,43 @@ std::vector<int> split_candidate_bits(double tol, int forced_slices) {
 // ------------------------------------------- FP64-grade tensor-core products
 // Blocks the tensor-core launch takes: a summed real depth of at least
 // F64T_DEPTH (below it a sum of normally distributed terms often misses the
-// certificate) and at least F64T_WORK real multiply-adds.  GB300's FP64 pipe
-// does about 2 multiply-adds per clock and SM: a 64 x 64 tile of depth 64
-// holds an SM for 70 us, while its digits take two strip launches and one
-// tile of the tensor-core launch.  Measured, FP64 tiles against this path: 300
+// certificate) and at least F64T_WORK real multiply-adds, which take the
+// narrow FP64 pipe (about 2 multiply-adds per clock and SM) 9 us in one tile;
+// the three launches take about 25 us in sum whatever the block.  Measured, FP64 tiles against this path: 300
 // complex products of 8..1024 per side 23.1 -> 1.71 ms (15.6 TFLOP/s of FP64
 // work; error against a 64-bit product 1.2e-15 -> 6.7e-16), 64 real blocks of
 // 4..96 105 -> 77 us.
-constexpr int64_t F64T_DEPTH = 48, F64T_MAX_DEPTH = 1 << 20;
-constexpr double F64T_WORK = 65536.0;
+constexpr int64_t F64T_DEPTH = 9, F64T_MAX_DEPTH = 1 << 20;
+constexpr double F64T_WORK = 32768.0;
 // Digit bytes of one launch (blocks above it get a launch of their own), and
 // of a block that still takes this path.
 constexpr int64_t F64T_CHUNK_BYTES = int64_t(2) << 30, F64T_BLOCK_BYTES = int64_t(8) << 30;
+
+// Whether the tensor-core launch takes a block; `bytes` its digits (at most).
+static bool f64_tensor_takes(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int64_t M, int64_t N,
+                             bool cplx, int64_t &bytes) {
+  const int64_t cm = cplx ? 2 : 1;
+  auto up = [](int64_t x, int64_t t) { return (x + t - 1) / t * t; };
+  int64_t depth = 0, kpad = 0;
+  for (int64_t p = p0; p < p1; ++p) {
+    const int64_t K = std::max<int32_t>(pairs[p].K, 0);
+    depth += K * cm;
+    kpad += up(std::max<int64_t>(K * cm, 1), TKS);
+    // a factor of 0 keeps the FP64 kernel's 0 * x (NaN for an infinite x)
+    if (!std::isfinite(pairs[p].afac) || pairs[p].afac == 0.0) return false;
+  }
+  if (depth < F64T_DEPTH || depth > F64T_MAX_DEPTH || M > (1 << 24) || N > (1 << 24) ||
+      double(M) * double(N) * double(depth) * double(cm) < F64T_WORK)
+    return false;
+  // either operand's real form may be the duplicated one
+  bytes = (up(M * cm, TMS) + up(N * cm, TMS)) * kpad * (HP_DIGITS + 1) * 2;
+  return bytes <= F64T_BLOCK_BYTES;
+}
+
+bool f64_direct(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int32_t M, int32_t N, bool cplx) {
+  int64_t bytes = 0;
+  return !f64_tensor_takes(pairs, p0, p1, M, N, cplx, bytes) || shallow_direct_wins(pairs, p0, p1, M, N, cplx);
+}
 
 F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                               const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
@@ -1845,29 +1871,13 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
                               const std::vector<char> &skip) {
   F64TensorList tl;
   const int64_t nb = (int64_t)bM.size();
-  const int64_t cm = cplx ? 2 : 1;
   tl.on.assign(nb, 0);
   tl.fbase.assign(nb, 0);
   int64_t chunk0 = 0, chunk_bytes = 0;
-  auto up = [](int64_t x, int64_t t) { return (x + t - 1) / t * t; };
   for (int64_t g = 0; g < nb; ++g) {
-    if (!skip.empty() && skip[g]) continue;
-    int64_t depth = 0, kpad = 0;
-    bool fits = true;
-    for (int64_t p = grp[g]; p < grp[g + 1]; ++p) {
-      const int64_t K = std::max<int32_t>(pairs[p].K, 0);
-      depth += K * cm;
-      kpad += up(std::max<int64_t>(K * cm, 1), TKS);
-      // a factor of 0 keeps the FP64 kernel's 0 * x (NaN for an infinite x)
-      fits = fits && std::isfinite(pairs[p].afac) && pairs[p].afac != 0.0;
-    }
     const int64_t M = bM[g], N = bN[g];
-    if (!fits || depth < F64T_DEPTH || depth > F64T_MAX_DEPTH ||
-        double(M) * double(N) * double(depth) * double(cm) < F64T_WORK || M > (1 << 24) || N > (1 << 24))
-      continue;
-    // either operand's real form may be the duplicated one
-    const int64_t bytes = (up(M * cm, TMS) + up(N * cm, TMS)) * kpad * (HP_DIGITS + 1) * 2;
-    if (bytes > F64T_BLOCK_BYTES) continue;
+    int64_t bytes = 0;
+    if ((!skip.empty() && skip[g]) || !f64_tensor_takes(pairs, grp[g], grp[g + 1], M, N, cplx, bytes)) continue;
     const int64_t cells = ((M + F64_TILE - 1) / F64_TILE) * ((N + F64_TILE - 1) / F64_TILE);
     if (tl.nflags + cells > INT32_MAX) continue;
     tl.on[g] = 1;

@@ -101,7 +101,8 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
   std::vector<char> rest(bM.size(), 1);
   std::vector<int64_t> ids;
   for (size_t b = 0; b < bM.size(); ++b)
-    if (is_shallow(pairs, grp[b], grp[b + 1])) {
+    if (is_shallow(pairs, grp[b], grp[b + 1]) &&
+        f64_direct(pairs, grp[b], grp[b + 1], bM[b], bN[b], cplx)) {
       rest[b] = 0;
       ids.push_back((int64_t)b);
     }

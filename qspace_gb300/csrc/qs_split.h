@@ -72,6 +72,9 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
                               const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                               const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
                               const std::vector<char> &skip);
+// Whether the FP64 path computes a shallow block directly (run_shallow): it
+// does unless the tensor-core launch takes the block and is estimated faster.
+bool f64_direct(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int32_t M, int32_t N, bool cplx);
 // Runs them (strips and products); false when the device has no room for
 // their digits (nothing ran: the caller computes every tile in FP64).
 bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,

@@ -71,7 +71,7 @@ def _check(got, ref):
 @pytest.mark.parametrize("cplx", [False, True])
 @pytest.mark.parametrize("shape", [(64, 64, 48), (40, 70, 24), (65, 33, 96), (129, 31, 97), (1, 700, 130), (700, 1, 130),
                                    (128, 32, 193), (63, 127, 512), (31, 33, 9), (17, 48, 20), (64, 16, 16),
-                                   (1, 33, 17)])
+                                   (1, 33, 17), (300, 200, 5), (260, 515, 9)])
 def test_f64_tensor_sizes(shape, cplx):
     rng = np.random.default_rng(5)
     M, N, K = shape
