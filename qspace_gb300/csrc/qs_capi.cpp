@@ -352,20 +352,40 @@ static bool make_view(const QMeta &m, int64_t blk, const std::vector<int> &line_
     stride[k] = sacc;
     sacc *= m.drow(blk)[k];
   }
-  v.nl = (int32_t)ll.size();
-  v.nk = (int32_t)kl.size();
-  for (int i = 0; i < v.nl; ++i) {
-    v.ldim[i] = (int32_t)m.drow(blk)[ll[i]];
-    v.lstr[i] = stride[ll[i]];
-  }
-  for (int i = 0; i < v.nk; ++i) {
-    v.kdim[i] = (int32_t)m.drow(blk)[kl[i]];
-    v.kstr[i] = stride[kl[i]];
-  }
+  // a leg that continues the one before it in storage joins it
+  auto legs = [&](const std::vector<int> &from, int32_t &n, int32_t *dim, int64_t *str) {
+    n = 0;
+    for (int k : from) {
+      if (n > 0 && str[n - 1] * dim[n - 1] == stride[k]) {
+        dim[n - 1] *= (int32_t)m.drow(blk)[k];
+        continue;
+      }
+      dim[n] = (int32_t)m.drow(blk)[k];
+      str[n++] = stride[k];
+    }
+  };
+  legs(ll, v.nl, v.ldim, v.lstr);
+  legs(kl, v.nk, v.kdim, v.kstr);
   if (v.nl == 0) {  // a single line: one leg of size 1 keeps the view active
     v.nl = 1;
     v.ldim[0] = 1;
     v.lstr[0] = 0;
+  }
+  return true;
+}
+
+// Whether the permuted copy of every block would have the block's own memory
+// order: the legs that move have size 1 (site legs of abelian tensors mostly
+// do), so the operand is read where it lies.
+static bool keeps_order(const QMeta &m, const std::vector<int> &perm) {
+  for (int64_t b = 0; b < m.nblk; ++b) {
+    const int64_t *d = m.drow(b);
+    int last = -1;
+    for (int k : perm) {
+      if (d[k] == 1) continue;
+      if (k < last) return false;
+      last = k;
+    }
   }
   return true;
 }
@@ -392,7 +412,7 @@ static void append_offsets(int n, const int32_t *dim, const int64_t *str, std::v
 // allocate the output (kernels on ctx->stream).
 static void prepare(Ctx *ctx, Prepared &w, const QMeta &Am, const double *dA, const QMeta &Bm,
                     const double *dB, const char *ia, const char *ib, const int32_t *perm, int32_t nperm,
-                    bool views = false) {
+                    bool split = false) {
   w.pl = plan_contract(Am, ia, Bm, ib, perm, nperm);
   ContractPlan &pl = w.pl;
   const bool cplx = w.cplx = pl.C.cplx;
@@ -404,29 +424,40 @@ static void prepare(Ctx *ctx, Prepared &w, const QMeta &Am, const double *dA, co
     return;
   }
   const int es = cplx ? 2 : 1;
-  // The split path reads a permuted operand in place through per-pair
-  // strided views (lines over the kept legs, depth over the contracted legs
-  // in pairing order, the order of permute_to's copy) when every block's legs
-  // fit a view; the FP64 path reads the permuted copy.
+  // An operand whose permuted copy would have its own memory order is read
+  // where it lies.  Otherwise the split path, and contractions whose blocks
+  // are all computed directly (run_shallow), read a permuted operand in place
+  // through per-pair strided views (lines over the kept legs, depth over the
+  // contracted legs in pairing order, the order of permute_to's copy) when
+  // every block's legs fit a view; the FP64 tiles read the permuted copy.
   // Deep output blocks are cut along their depth (split_deep), which needs
   // plain operands: such contractions read permuted copies.
-  bool deep = views && has_deep_blocks(pl.pairs, pl.grp, pl.blk_M, pl.blk_N);
-  // likewise contractions whose blocks are all shallow (computed directly
-  // from plain operands)
-  if (views && !deep) {
-    bool all_shallow = true;
-    for (size_t b = 0; b + 1 < pl.grp.size() && all_shallow; ++b)
-      all_shallow = is_shallow(pl.pairs, pl.grp[b], pl.grp[b + 1]) &&
-                    shallow_direct_wins(pl.pairs, pl.grp[b], pl.grp[b + 1], pl.blk_M[b], pl.blk_N[b], w.cplx);
-    deep = all_shallow;
-  }
+  bool all_direct = true;
+  for (size_t b = 0; b + 1 < pl.grp.size() && all_direct; ++b)
+    all_direct = is_shallow(pl.pairs, pl.grp[b], pl.grp[b + 1]) &&
+                 (split ? shallow_direct_wins(pl.pairs, pl.grp[b], pl.grp[b + 1], pl.blk_M[b], pl.blk_N[b], cplx)
+                        : f64_direct(pl.pairs, pl.grp[b], pl.grp[b + 1], pl.blk_M[b], pl.blk_N[b], cplx));
+  const bool views = (split || all_direct) && !has_deep_blocks(pl.pairs, pl.grp, pl.blk_M, pl.blk_N);
   // the views' offset tables, one pair of tables per operand block (every
   // pair reading the block shares them): all in one upload
   std::vector<int64_t> vtab;
   std::vector<std::pair<int64_t, int64_t>> toff_a, toff_b;  // per pair: (line, depth) table starts
+  // the permuted copy would have been conjugated: conjugate on the fly.
+  // XOR, not OR: the conjugation flag may be set as well (the auto-conj
+  // rule of contract_getIdxSet, after permute_to flipped the copy's itags),
+  // and the two conjugations then cancel, as they do for the copy
+  auto conj_in_place = [&](bool is_a) {
+    if ((is_a ? pl.la : pl.lb).conj)
+      for (PairDesc &d : pl.pairs) d.trans ^= is_a ? 4 : 8;
+  };
   auto fused = [&](const QMeta &m, bool is_a, std::vector<OperandView> &out) -> bool {
     const OperandLayout &lay = is_a ? pl.la : pl.lb;
-    if (!views || deep || !lay.permute) return false;
+    if (!lay.permute) return false;
+    if (keeps_order(m, lay.perm)) {
+      conj_in_place(is_a);
+      return true;
+    }
+    if (!views) return false;
     const std::vector<int> &lines = is_a ? pl.ika : pl.ikb;
     const std::vector<int> &ks = is_a ? pl.ica.idx : pl.icb.idx;
     std::vector<OperandView> v(pl.pairs.size());
@@ -445,6 +476,10 @@ static void prepare(Ctx *ctx, Prepared &w, const QMeta &Am, const double *dA, co
         vtab.resize(tab0);
         return false;
       }
+      if (all_direct) {  // the direct kernel takes the legs themselves
+        first.emplace(blk, p);
+        continue;
+      }
       toff[p] = {(int64_t)vtab.size(), 0};
       append_offsets(v[p].nl, v[p].ldim, v[p].lstr, vtab);
       toff[p].second = (int64_t)vtab.size();
@@ -453,12 +488,7 @@ static void prepare(Ctx *ctx, Prepared &w, const QMeta &Am, const double *dA, co
     }
     out.swap(v);
     (is_a ? toff_a : toff_b).swap(toff);
-    // the permuted copy would have been conjugated: conjugate on the fly.
-    // XOR, not OR: the conjugation flag may be set as well (the auto-conj
-    // rule of contract_getIdxSet, after permute_to flipped the copy's itags),
-    // and the two conjugations then cancel, as they do for the copy
-    if (lay.conj)
-      for (PairDesc &d : pl.pairs) d.trans ^= is_a ? 4 : 8;
+    conj_in_place(is_a);
     return true;
   };
   const bool fa = fused(Am, true, w.va), fb = fused(Bm, false, w.vb);
@@ -558,8 +588,8 @@ static void run_products(Ctx *ctx, const std::vector<Prepared *> &batch, const q
       stats->err_bound = sr.err_bound;
     }
   } else if (prec == QS_PREC_FP64) {
-    if (any_view) fail(QS_ERR_INTERNAL, "FP64 products of operands read through views");
-    run_f64(ctx, pairs, grp, bM, bN, c_off, nullptr, baseA, baseB, baseC, cplx);
+    run_f64(ctx, pairs, grp, bM, bN, c_off, nullptr, baseA, baseB, baseC, cplx, any_view ? &va : nullptr,
+            any_view ? &vb : nullptr);
   } else {
     fail(QS_ERR_ARG, "unknown precision mode %d", prec);
   }

@@ -53,47 +53,187 @@ __global__ void reduce_parts_kernel(const DeepReduce *__restrict__ red, const do
   }
 }
 
-// One thread per output element of a shallow block: C(i, j) = sum over the
-// block's pairs, in order, of afac sum_k op(A)(i, k) op(B)(k, j).
+// Shallow blocks: C(i, j) = sum over the block's pairs, in order, of
+// afac sum_k op(A)(i, k) op(B)(k, j), with at most SHALLOW_K terms in all.  A
+// thread owns lines of one side (rows of op(A) with their unit-stride stores;
+// columns of op(B) when there are few rows and more columns) and keeps the
+// sums of up to NC lines of the other side in registers, so that it loads
+// each element of its line once; the other side's terms sit in shared memory.
+// The FP64 multiply-adds bound it (2 per clock and SM): pairs with factor 1
+// add their products to the running sum directly.  Applying an MPO tensor
+// over a leg of dimension 3 (12 million outputs, up to 3 terms of 3): 190 us
+// with one thread per output and a permuted copy, 140 us here, 73 us of it the
+// FP64 pipe's.
 struct ShallowTask {
   int64_t c_off;
-  int32_t p0, p1, M, N, ldc, pad_;
-  int64_t e0, e1;   // elements of this task (column-major over M x N)
+  int32_t p0, p1, M, N, ldc;
+  int32_t swapped;          // lines are columns of C
+  int32_t l0, l1;           // lines of this task
+  int32_t o0;               // first line of the other side
+  int32_t pad_;
 };
-
+constexpr int SHALLOW_THREADS = 128;
+constexpr int SHALLOW_NC = 4;  // lines of the other side per CTA
+// lines per thread: their loads are in flight together (one line at a time
+// leaves the kernel at 2.3 TB/s)
 template <bool CPLX>
-__global__ void shallow_kernel(const ShallowTask *__restrict__ tasks, const PairDesc *__restrict__ pairs,
-                               const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C) {
-  const ShallowTask t = tasks[blockIdx.x];
-  for (int64_t e = t.e0 + threadIdx.x; e < t.e1; e += blockDim.x) {
-    const int64_t i = e % t.M, j = e / t.M;
-    double re = 0.0, im = 0.0;
-    for (int p = t.p0; p < t.p1; ++p) {
-      const PairDesc P = pairs[p];
-      const bool ta = P.trans & 1, tb = P.trans & 2, ca = P.trans & 4, cb = P.trans & 8;
-      double sr = 0.0, si = 0.0;
-      for (int k = 0; k < P.K; ++k) {
-        const int64_t ia = P.a_off + (ta ? k + i * (int64_t)P.lda : i + k * (int64_t)P.lda);
-        const int64_t ib = P.b_off + (tb ? j + k * (int64_t)P.ldb : k + j * (int64_t)P.ldb);
+constexpr int shallow_u() { return CPLX ? 2 : 4; }
+
+// Offset of index l in a view's legs (first leg fastest).
+__device__ __forceinline__ int64_t legs_offset(int n, const int32_t *dim, const int64_t *str, int32_t l) {
+  int64_t off = 0;
+  for (int i = 0; i + 1 < n; ++i) {
+    const int32_t q = (int32_t)((uint32_t)l / (uint32_t)dim[i]);
+    off += (l - q * dim[i]) * str[i];
+    l = q;
+  }
+  return n > 0 ? off + l * str[n - 1] : off;
+}
+
+// Addresses of one operand in the role it plays: line l, depth k.
+struct ShallowAddr {
+  int64_t off, ls, ks;
+  const OperandView *v;
+  __device__ __forceinline__ int64_t line(int32_t l) const {
+    return off + (v ? legs_offset(v->nl, v->ldim, v->lstr, l) : l * ls);
+  }
+  __device__ __forceinline__ int64_t depth(int32_t k) const {
+    return v ? legs_offset(v->nk, v->kdim, v->kstr, k) : k * ks;
+  }
+};
+__device__ __forceinline__ ShallowAddr shallow_addr(const PairDesc &P, bool b, const OperandView *views, int p) {
+  const bool t = P.trans & (b ? 2 : 1);
+  const int64_t ld = b ? P.ldb : P.lda;
+  // A: line = row, depth = column; B: line = column, depth = row
+  const bool unit_line = b == t;
+  ShallowAddr a{b ? P.b_off : P.a_off, unit_line ? 1 : ld, unit_line ? ld : 1, nullptr};
+  if (views && views[p].nl > 0) a.v = views + p;
+  return a;
+}
+
+// The lines of this thread against NC lines of the other side (a count known
+// at compile time: predicated multiply-adds would take the FP64 pipe as real
+// ones do).
+template <bool CPLX, int NC>
+__device__ __forceinline__ void shallow_lines(const ShallowTask &t, const PairDesc *__restrict__ pairs,
+                                              const OperandView *vx, const double *__restrict__ X, bool wide_x,
+                                              const double2 (*yc)[SHALLOW_NC], double *__restrict__ C, bool wide_c) {
+  constexpr int U = shallow_u<CPLX>();
+  const int lb = t.l0 + threadIdx.x;
+  if (lb >= t.l1) return;
+  double re[U][NC], im[U][NC];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) re[u][c] = im[u][c] = 0.0;
+  int term = 0;
+  for (int p = t.p0; p < t.p1; ++p) {
+    const PairDesc &P = pairs[p];
+    const int K = P.K;
+    if (K <= 0) continue;
+    const ShallowAddr ax = shallow_addr(P, t.swapped, vx, p);
+    const bool cx = P.trans & (t.swapped ? 8 : 4);
+    const double f = P.afac;
+    int64_t lo[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) lo[u] = ax.line(min(lb + u * SHALLOW_THREADS, t.l1 - 1));
+    for (int k = 0; k < K; ++k) {
+      const int64_t kd = ax.depth(k);
+      double xr[U], xi[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = lo[u] + kd;
+        xi[u] = 0.0;
         if (CPLX) {
-          const double ar = A[2 * ia], ai = ca ? -A[2 * ia + 1] : A[2 * ia + 1];
-          const double br = B[2 * ib], bi = cb ? -B[2 * ib + 1] : B[2 * ib + 1];
-          sr += ar * br - ai * bi;
-          si += ar * bi + ai * br;
+          const double2 x = wide_x ? reinterpret_cast<const double2 *>(X)[i] : make_double2(X[2 * i], X[2 * i + 1]);
+          xr[u] = x.x;
+          xi[u] = cx ? -x.y : x.y;
         } else {
-          sr += A[ia] * B[ib];
+          xr[u] = X[i];
         }
       }
-      re += P.afac * sr;
-      im += P.afac * si;
+      if (f != 1.0) {  // uniform: the factor scales the line's element, as in the tiled kernel
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          xr[u] *= f;
+          xi[u] *= f;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double2 y = yc[term + k][c];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          re[u][c] = fma(xr[u], y.x, re[u][c]);
+          if (CPLX) {
+            re[u][c] = fma(-xi[u], y.y, re[u][c]);
+            im[u][c] = fma(xr[u], y.y, im[u][c]);
+            im[u][c] = fma(xi[u], y.x, im[u][c]);
+          }
+        }
+      }
     }
-    const int64_t o = t.c_off + i + j * (int64_t)t.ldc;
-    if (CPLX) {
-      C[2 * o] = re;
-      C[2 * o + 1] = im;
-    } else {
-      C[o] = re;
+    term += K;
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t l = lb + u * SHALLOW_THREADS;
+    if (l >= t.l1) break;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int64_t i = t.swapped ? t.o0 + c : l, j = t.swapped ? l : t.o0 + c;
+      const int64_t o = t.c_off + i + j * (int64_t)t.ldc;
+      if (!CPLX) {
+        C[o] = re[u][c];
+      } else if (wide_c) {
+        reinterpret_cast<double2 *>(C)[o] = make_double2(re[u][c], im[u][c]);
+      } else {
+        C[2 * o] = re[u][c];
+        C[2 * o + 1] = im[u][c];
+      }
     }
+  }
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(SHALLOW_THREADS)
+shallow_kernel(const ShallowTask *__restrict__ tasks, const PairDesc *__restrict__ pairs,
+               const OperandView *__restrict__ va, const OperandView *__restrict__ vb, const double *__restrict__ A,
+               const double *__restrict__ B, double *__restrict__ C) {
+  constexpr int NC = SHALLOW_NC;
+  __shared__ double2 yc[SHALLOW_K][NC];  // the other side: term (in pair, k order) x line
+  const ShallowTask t = tasks[blockIdx.x];
+  const int other = t.swapped ? t.M : t.N;
+  const int nc = min(NC, other - t.o0);
+  const OperandView *vx = t.swapped ? vb : va, *vy = t.swapped ? va : vb;
+  const double *__restrict__ X = t.swapped ? B : A;
+  const double *__restrict__ Y = t.swapped ? A : B;
+  // complex buffers may be aligned to 8 bytes only
+  const bool wide_x = (reinterpret_cast<uintptr_t>(X) & 15) == 0, wide_c = (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+  int term = 0;
+  for (int p = t.p0; p < t.p1; ++p) {
+    const PairDesc P = pairs[p];
+    const int K = max(P.K, 0);
+    const ShallowAddr ay = shallow_addr(P, !t.swapped, vy, p);
+    const bool cy = P.trans & (t.swapped ? 4 : 8);
+    for (int e = threadIdx.x; e < K * NC; e += SHALLOW_THREADS) {
+      const int k = e / NC, c = e % NC;
+      double2 v = make_double2(0.0, 0.0);
+      if (c < nc) {
+        const int64_t i = ay.line(t.o0 + c) + ay.depth(k);
+        if (CPLX) v = make_double2(Y[2 * i], cy ? -Y[2 * i + 1] : Y[2 * i + 1]);
+        else v.x = Y[i];
+      }
+      yc[term + k][c] = v;
+    }
+    term += K;
+  }
+  __syncthreads();
+  switch (nc) {
+    case 1: shallow_lines<CPLX, 1>(t, pairs, vx, X, wide_x, yc, C, wide_c); break;
+    case 2: shallow_lines<CPLX, 2>(t, pairs, vx, X, wide_x, yc, C, wide_c); break;
+    case 3: shallow_lines<CPLX, 3>(t, pairs, vx, X, wide_x, yc, C, wide_c); break;
+    default: shallow_lines<CPLX, 4>(t, pairs, vx, X, wide_x, yc, C, wide_c); break;
   }
 }
 
@@ -196,51 +336,81 @@ bool shallow_direct_wins(const std::vector<PairDesc> &pairs, int64_t p0, int64_t
   return direct < tiled;
 }
 
+// Tasks over the listed blocks, whose pairs are numbered consecutively in
+// list order (the compact pair list that goes with them).
 static std::vector<ShallowTask> shallow_tasks(const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
                                               const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
-                                              const std::vector<int32_t> *bldc, const std::vector<int64_t> &blocks) {
-  constexpr int64_t CHUNK = 8192;  // elements per CTA
+                                              const std::vector<int32_t> *bldc, const std::vector<int64_t> &blocks,
+                                              bool cplx) {
+  const int NC = SHALLOW_NC, LINES = SHALLOW_THREADS * (cplx ? shallow_u<true>() : shallow_u<false>());
   std::vector<ShallowTask> tasks;
+  int64_t p = 0;
   for (int64_t b : blocks) {
-    const int64_t n = (int64_t)bM[b] * bN[b];
-    for (int64_t e0 = 0; e0 < n; e0 += CHUNK) {
-      ShallowTask t{};
-      t.c_off = coff[b];
-      t.p0 = (int32_t)grp[b];
-      t.p1 = (int32_t)grp[b + 1];
-      t.M = bM[b];
-      t.N = bN[b];
-      t.ldc = bldc ? (*bldc)[b] : std::max(bM[b], 1);
-      t.e0 = e0;
-      t.e1 = std::min(n, e0 + CHUNK);
-      tasks.push_back(t);
-    }
+    ShallowTask t{};
+    t.c_off = coff[b];
+    t.p0 = (int32_t)p;
+    p += grp[b + 1] - grp[b];
+    t.p1 = (int32_t)p;
+    t.M = bM[b];
+    t.N = bN[b];
+    t.ldc = bldc ? (*bldc)[b] : std::max(bM[b], 1);
+    // rows as lines keep the stores coalesced; a block of fewer rows than a
+    // warp has more parallelism along its columns
+    t.swapped = t.M < 32 && t.N > t.M;
+    const int32_t lines = t.swapped ? t.N : t.M, other = t.swapped ? t.M : t.N;
+    for (int32_t o = 0; o < other; o += NC)
+      for (int64_t l = 0; l < lines; l += LINES) {
+        t.o0 = o;
+        t.l0 = (int32_t)l;
+        t.l1 = (int32_t)std::min<int64_t>(lines, l + LINES);
+        tasks.push_back(t);
+      }
   }
   if (tasks.size() > 0x7fffffff) fail(QS_ERR_SHAPE, "shallow products: too many tasks");
   return tasks;
 }
 
+template <class T>
+static std::vector<T> pairs_of(const std::vector<T> &all, const std::vector<int64_t> &grp,
+                               const std::vector<int64_t> &blocks) {
+  std::vector<T> out;
+  for (int64_t b : blocks) out.insert(out.end(), all.begin() + grp[b], all.begin() + grp[b + 1]);
+  return out;
+}
+
+static void launch_shallow(Ctx *ctx, const ShallowTask *tasks, int64_t n, const PairDesc *pairs,
+                           const OperandView *va, const OperandView *vb, const double *A, const double *B, double *C,
+                           bool cplx) {
+  if (cplx) shallow_kernel<true><<<(unsigned)n, SHALLOW_THREADS, 0, ctx->stream>>>(tasks, pairs, va, vb, A, B, C);
+  else shallow_kernel<false><<<(unsigned)n, SHALLOW_THREADS, 0, ctx->stream>>>(tasks, pairs, va, vb, A, B, C);
+  QS_LAUNCHED(ctx);
+}
+
 void run_shallow(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                  const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
                  const std::vector<int32_t> *bldc, const std::vector<int64_t> &blocks, const double *A,
-                 const double *B, double *C, bool cplx) {
-  const std::vector<ShallowTask> tasks = shallow_tasks(grp, bM, bN, coff, bldc, blocks);
+                 const double *B, double *C, bool cplx, const std::vector<OperandView> *va,
+                 const std::vector<OperandView> *vb) {
+  const std::vector<ShallowTask> tasks = shallow_tasks(grp, bM, bN, coff, bldc, blocks, cplx);
   if (tasks.empty()) return;
-  ShallowTask *dt = dev_upload(ctx, tasks);
-  PairDesc *dp = dev_upload(ctx, pairs);
-  if (cplx) shallow_kernel<true><<<(unsigned)tasks.size(), 256, 0, ctx->stream>>>(dt, dp, A, B, C);
-  else shallow_kernel<false><<<(unsigned)tasks.size(), 256, 0, ctx->stream>>>(dt, dp, A, B, C);
-  // the work lists are released in stream order, also when the launch failed
-  dev_free(ctx, dt);
-  dev_free(ctx, dp);
-  QS_LAUNCHED(ctx);
+  const std::vector<PairDesc> pp = pairs_of(pairs, grp, blocks);
+  const std::vector<OperandView> none;
+  const std::vector<OperandView> wa = va ? pairs_of(*va, grp, blocks) : none;
+  const std::vector<OperandView> wb = vb ? pairs_of(*vb, grp, blocks) : none;
+  DevLists L;
+  const size_t st = L.add(tasks), sp = L.add(pp), sa = L.add(wa), sb = L.add(wb);
+  L.commit(ctx);
+  launch_shallow(ctx, L.at<ShallowTask>(st), (int64_t)tasks.size(), L.at<PairDesc>(sp),
+                 wa.empty() ? nullptr : L.at<OperandView>(sa), wb.empty() ? nullptr : L.at<OperandView>(sb), A, B, C,
+                 cplx);
 }
 
 ShallowPlan shallow_prepare(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                             const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                             const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc,
                             const std::vector<int64_t> &blocks, bool cplx) {
-  const std::vector<ShallowTask> tasks = shallow_tasks(grp, bM, bN, coff, bldc, blocks);
+  const std::vector<ShallowTask> tasks = shallow_tasks(grp, bM, bN, coff, bldc, blocks, cplx);
+  const std::vector<PairDesc> pp = pairs_of(pairs, grp, blocks);
   ShallowPlan sp;
   sp.cplx = cplx;
   sp.ntasks = (int64_t)tasks.size();
@@ -248,9 +418,8 @@ ShallowPlan shallow_prepare(const std::vector<PairDesc> &pairs, const std::vecto
   try {
     QS_CUDA(cudaMalloc(&sp.tasks, tasks.size() * sizeof(ShallowTask)));
     QS_CUDA(cudaMemcpy(sp.tasks, tasks.data(), tasks.size() * sizeof(ShallowTask), cudaMemcpyHostToDevice));
-    QS_CUDA(cudaMalloc(&sp.pairs, std::max<size_t>(pairs.size(), 1) * sizeof(PairDesc)));
-    if (!pairs.empty())
-      QS_CUDA(cudaMemcpy(sp.pairs, pairs.data(), pairs.size() * sizeof(PairDesc), cudaMemcpyHostToDevice));
+    QS_CUDA(cudaMalloc(&sp.pairs, std::max<size_t>(pp.size(), 1) * sizeof(PairDesc)));
+    if (!pp.empty()) QS_CUDA(cudaMemcpy(sp.pairs, pp.data(), pp.size() * sizeof(PairDesc), cudaMemcpyHostToDevice));
   } catch (...) {
     shallow_release(sp);
     throw;
@@ -260,11 +429,8 @@ ShallowPlan shallow_prepare(const std::vector<PairDesc> &pairs, const std::vecto
 
 void shallow_launch(Ctx *ctx, const ShallowPlan &sp, const double *A, const double *B, double *C) {
   if (!sp.ntasks) return;
-  const ShallowTask *dt = static_cast<const ShallowTask *>(sp.tasks);
-  const PairDesc *dp = static_cast<const PairDesc *>(sp.pairs);
-  if (sp.cplx) shallow_kernel<true><<<(unsigned)sp.ntasks, 256, 0, ctx->stream>>>(dt, dp, A, B, C);
-  else shallow_kernel<false><<<(unsigned)sp.ntasks, 256, 0, ctx->stream>>>(dt, dp, A, B, C);
-  QS_LAUNCHED(ctx);
+  launch_shallow(ctx, static_cast<const ShallowTask *>(sp.tasks), sp.ntasks, static_cast<const PairDesc *>(sp.pairs),
+                 nullptr, nullptr, A, B, C, sp.cplx);
 }
 
 void shallow_release(ShallowPlan &sp) {

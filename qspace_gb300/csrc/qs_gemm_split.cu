@@ -1418,6 +1418,12 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
           w.vb[p] = y;
         }
       }
+    // a role without views runs the strips with the view code compiled out
+    auto none_in = [](const std::vector<OperandView> &v) {
+      return std::none_of(v.begin(), v.end(), [](const OperandView &x) { return x.nl > 0; });
+    };
+    if (none_in(w.va)) w.va.clear();
+    if (none_in(w.vb)) w.vb.clear();
   }
   w.hp = fbase != nullptr;
   DigitPlan dp = w.hp ? DigitPlan{HP_BITS, HP_DIGITS, (HP_DIGITS + 2) * std::ldexp(1.0, -HP_BITS * HP_DIGITS)}
@@ -1629,8 +1635,8 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
 // their depth into parts computed as blocks of their own in a temporary
 // buffer and summed in part order (split_deep).  Both decisions depend on the
 // block alone, and the digit plan is the one of the list as given, so a
-// block gives the same bits whatever else is in the launch.  Blocks with a
-// pair read through a view run as they are.
+// block gives the same bits whatever else is in the launch.  Deeper blocks
+// with a pair read through a view run as they are.
 SplitResult run_split(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                       const std::vector<int32_t> &blk_M, const std::vector<int32_t> &blk_N,
                       const std::vector<int64_t> &c_off, const double *A, const double *B, double *C,
@@ -1639,7 +1645,7 @@ SplitResult run_split(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::v
                       const std::vector<OperandView> *vb) {
   const size_t nb = blk_M.size();
   const int64_t eb = cplx ? 16 : 8;
-  // blocks with a pair read through a view stay as they are
+  // blocks with a pair read through a view are not cut along their depth
   std::vector<char> keep;
   if (va || vb) {
     keep.assign(nb, 0);
@@ -1650,7 +1656,7 @@ SplitResult run_split(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::v
   std::vector<char> shallow(nb, 0), rest(nb, 1);
   std::vector<int64_t> shallow_ids;
   for (size_t g = 0; g < nb; ++g)
-    if (!(keep.size() && keep[g]) && is_shallow(pairs, grp[g], grp[g + 1]) &&
+    if (is_shallow(pairs, grp[g], grp[g + 1]) &&
         shallow_direct_wins(pairs, grp[g], grp[g + 1], blk_M[g], blk_N[g], cplx)) {
       shallow[g] = 1;
       rest[g] = 0;
@@ -1658,7 +1664,7 @@ SplitResult run_split(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::v
     }
   if (!shallow_ids.empty()) {
     const DigitPlan dp = choose_digits_for(pairs, grp, blk_M, blk_N, cplx ? 2 : 1, tol, forced_slices, forced_bits);
-    run_shallow(ctx, pairs, grp, blk_M, blk_N, c_off, blk_ldc, shallow_ids, A, B, C, cplx);
+    run_shallow(ctx, pairs, grp, blk_M, blk_N, c_off, blk_ldc, shallow_ids, A, B, C, cplx, va, vb);
     SplitResult res;
     res.nslices = dp.nslices;
     res.bits = dp.bits;
@@ -1746,10 +1752,8 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
   d.sa = dev_upload(ctx, w.sa);
   d.sb = dev_upload(ctx, w.sb);
   d.tiles = dev_upload(ctx, w.tiles);
-  if (!w.va.empty()) {
-    d.va = dev_upload(ctx, w.va);
-    d.vb = dev_upload(ctx, w.vb);
-  }
+  if (!w.va.empty()) d.va = dev_upload(ctx, w.va);
+  if (!w.vb.empty()) d.vb = dev_upload(ctx, w.vb);
   d.E = dev_alloc<int>(ctx, (size_t)w.nE);
   d.F = dev_alloc<int>(ctx, (size_t)w.nF);
   launch_split(ctx, w, cplx, d, A, B, C, ctx->d_err);

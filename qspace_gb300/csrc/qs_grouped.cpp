@@ -96,7 +96,8 @@ GroupedPlan grouped_plan(const qs_pair_list *pl, int64_t a_elems, int64_t b_elem
 
 void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
-             const std::vector<int32_t> *bldc, const double *A, const double *B, double *C, bool cplx) {
+             const std::vector<int32_t> *bldc, const double *A, const double *B, double *C, bool cplx,
+             const std::vector<OperandView> *va, const std::vector<OperandView> *vb) {
   // shallow blocks directly (run_shallow), the rest through the tiles
   std::vector<char> rest(bM.size(), 1);
   std::vector<int64_t> ids;
@@ -107,9 +108,12 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
       ids.push_back((int64_t)b);
     }
   if (!ids.empty()) {
-    run_shallow(ctx, pairs, grp, bM, bN, coff, bldc, ids, A, B, C, cplx);
+    run_shallow(ctx, pairs, grp, bM, bN, coff, bldc, ids, A, B, C, cplx, va, vb);
     if (ids.size() == bM.size()) return;
     const BlockList R = select_blocks(pairs, grp, bM, bN, coff, bldc, rest);
+    for (int32_t q : R.src)
+      if ((va && (*va)[q].nl > 0) || (vb && (*vb)[q].nl > 0))
+        fail(QS_ERR_INTERNAL, "FP64 tiles of an operand read through a view");
     run_f64(ctx, R.pairs, R.grp, R.bM, R.bN, R.coff, &R.bldc, A, B, C, cplx);
     return;
   }

@@ -27,10 +27,12 @@ GroupedPlan grouped_plan(const qs_pair_list *pl, int64_t a_elems, int64_t b_elem
 
 // The plain FP64 grouped product of a list (tensor cores with an FP64 net, FP64 tiles): shallow output
 // blocks computed directly (run_shallow), deep ones cut along their depth and
-// summed in part order (split_deep).
+// summed in part order (split_deep).  Pairs of blocks computed directly may
+// read their operands through views (va / vb, one per pair).
 void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
-             const std::vector<int32_t> *bldc, const double *A, const double *B, double *C, bool cplx);
+             const std::vector<int32_t> *bldc, const double *A, const double *B, double *C, bool cplx,
+             const std::vector<OperandView> *va = nullptr, const std::vector<OperandView> *vb = nullptr);
 
 // Validates the pair list, then launches the FP64 or the split path on all of
 // it.

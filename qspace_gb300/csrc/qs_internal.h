@@ -113,6 +113,24 @@ struct PairDesc {
 };
 static_assert(sizeof(PairDesc) == 48, "PairDesc layout");
 
+// A strided view of one operand block in place of the permuted copy that
+// permute_to makes (Source/QSpace.hh:2824-2866) when the contracted legs of
+// an operand are not contiguous: element (line, k) of the operand as the
+// GEMM reads it -- line = row of op(A) / column of op(B), k = depth -- sits at
+// block offset  sum_i l_i lstr[i] + sum_t k_t kstr[t],  line = sum_i l_i
+// prod_{i'<i} ldim[i'] (first leg fastest), likewise k.  nl = 0: no view.
+// The strip kernels read the offsets from tables built on the host once per
+// operand block: ltab[line] = sum_i l_i lstr[i], ktab[k] likewise (device
+// pointers; the host fills them in after the tables are uploaded); the
+// direct kernel takes the legs.
+constexpr int VIEW_LEGS = 4;
+struct OperandView {
+  int32_t nl, nk;
+  int32_t ldim[VIEW_LEGS], kdim[VIEW_LEGS];
+  int64_t lstr[VIEW_LEGS], kstr[VIEW_LEGS];
+  const int64_t *ltab, *ktab;
+};
+
 // Deep output blocks.  The grouped kernels give each output tile to one CTA
 // for the block's whole summed depth, so a block with few tiles and a very
 // deep sum (a reduced density matrix or an overlap over large bonds) would
@@ -167,11 +185,13 @@ bool is_shallow(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1);
 // shallow block directly.
 bool shallow_direct_wins(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int32_t M, int32_t N,
                          bool cplx);
-// Runs the listed blocks (indices into grp / bM / ...) directly.
+// Runs the listed blocks (indices into grp / bM / ...) directly;
+// va / vb (one per pair; nl = 0: none) read op(A) / op(B) through strided views.
 void run_shallow(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                  const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
                  const std::vector<int32_t> *bldc, const std::vector<int64_t> &blocks, const double *A,
-                 const double *B, double *C, bool cplx);
+                 const double *B, double *C, bool cplx, const std::vector<OperandView> *va = nullptr,
+                 const std::vector<OperandView> *vb = nullptr);
 // Parts of deep output blocks with at most DOT_OUTPUTS elements on the FP64
 // path: one CTA per output element reduces over the part's pairs and depth
 // (a fixed partition and tree order); 64 x 64 tiles would compute 4096
@@ -230,23 +250,6 @@ struct PermDesc {
   int64_t in_stride[8]; // stride in the input of output leg k
   int32_t fast_in_leg;  // output leg with input stride 1 (tiled blocks)
   int32_t pad_;
-};
-
-// A strided view of one operand block in place of the permuted copy that
-// permute_to makes (Source/QSpace.hh:2824-2866) when the contracted legs of
-// an operand are not contiguous: element (line, k) of the operand as the
-// GEMM reads it -- line = row of op(A) / column of op(B), k = depth -- sits at
-// block offset  sum_i l_i lstr[i] + sum_t k_t kstr[t],  line = sum_i l_i
-// prod_{i'<i} ldim[i'] (first leg fastest), likewise k.  nl = 0: no view.
-// The kernels read the offsets from tables built on the host once per
-// operand block: ltab[line] = sum_i l_i lstr[i], ktab[k] likewise (device
-// pointers; the host fills them in after the tables are uploaded).
-constexpr int VIEW_LEGS = 4;
-struct OperandView {
-  int32_t nl, nk;
-  int32_t ldim[VIEW_LEGS], kdim[VIEW_LEGS];
-  int64_t lstr[VIEW_LEGS], kstr[VIEW_LEGS];
-  const int64_t *ltab, *ktab;
 };
 
 // One 32 x 32 tile of a tiled block: tile (ti, tj) of (output leg 0,

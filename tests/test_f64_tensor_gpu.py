@@ -35,8 +35,8 @@ def _batch(ops, afac, blk, trans):
     flat = lambda xs: np.concatenate([np.asarray(x, pk.abuf.dtype).reshape(-1, order="F") for x in xs])  # noqa: E731
     pk.abuf = flat([_stored(a, t & 1, t & 4) for (a, _), t in zip(ops, trans)])
     pk.bbuf = flat([_stored(b, t & 2, t & 8) for (_, b), t in zip(ops, trans)])
-    pk.lda = np.where(pk.trans & 1, pk.K, pk.M).astype(np.int32)
-    pk.ldb = np.where(pk.trans & 2, pk.N, pk.K).astype(np.int32)
+    pk.lda = np.maximum(np.where(pk.trans & 1, pk.K, pk.M), 1).astype(np.int32)
+    pk.ldb = np.maximum(np.where(pk.trans & 2, pk.N, pk.K), 1).astype(np.int32)
     return DeviceBatch(pk)
 
 
@@ -184,3 +184,49 @@ def test_f64_tensor_alone_and_in_a_list():
         one = _batch([ops[p]], [afac[p]], [0], [0])
         one.run("fp64")
         assert np.array_equal(one.result()[0], c)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("prec", ["fp64", "split"])
+def test_shallow_blocks(prec, cplx):
+    """Blocks with at most eight summed terms: either side long, remainders of
+    the register and line blocking, several pairs, factors, every flag."""
+    rng = np.random.default_rng(21)
+    ops, afac, blk, trans = [], [], [], []
+    for g, (M, N) in enumerate([(1, 1), (1, 700), (700, 1), (31, 40), (32, 31), (513, 9), (5, 1025), (2, 513), (70, 17)]):
+        for K, f in ((3, 1.0), (1, -0.31), (0, 1.0), (4, 0.77)):
+            ops.append(_ops(rng, M, N, K, cplx))
+            afac.append(f)
+            blk.append(g)
+            trans.append(int(rng.integers(0, 16 if cplx else 4)))
+    db = _batch(ops, afac, blk, trans)
+    db.run(prec)
+    got = db.result()
+    ref = _reference(ops, afac, blk)
+    if prec == "fp64":
+        _check(got, ref)
+    else:  # blocks that the digits take instead: the path's own tolerance
+        for c, (r, s, n) in zip(got, ref):
+            assert np.linalg.norm((c - r).astype(complex)) <= 1e-12 * np.linalg.norm(s)
+    plan = db.plan(prec)
+    db.run_plan(plan)
+    for c, d in zip(db.result(), got):
+        assert np.array_equal(c, d)
+    plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift", [0, 1])
+def test_shallow_complex_alignment(shift):
+    """Complex buffers at an odd multiple of eight bytes, direct blocks."""
+    rng = np.random.default_rng(2)
+    ops = [_ops(rng, 50, 3, 2, True), _ops(rng, 4, 90, 5, True)]
+    db = _batch(ops, [1.0, 0.5], [0, 1], [0, 0])
+    t = db.torch
+    pad = lambda x: t.cat([t.zeros(shift, dtype=t.float64, device=x.device), x])[shift:]  # noqa: E731
+    want = _reference(ops, [1.0, 0.5], [0, 1])
+    db.dA, db.dB, db.dC = pad(db.dA), pad(db.dB), pad(db.dC)
+    t.cuda.synchronize()
+    db.run("fp64")
+    _check(db.result(), want)
