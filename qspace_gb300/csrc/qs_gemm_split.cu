@@ -46,7 +46,7 @@
 // warps = epilogue (EPI_WARPS / 4 per TMEM lane quarter).  Every mbarrier wait is bounded; on
 // timeout the kernel records an error code, stops issuing work, waits a
 // bounded time for what is in flight, frees its TMEM and returns.
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
@@ -90,6 +90,7 @@ struct SplitPair {
   int32_t e_afac;          // exponent added by the CG factor (|afac| < 2^e)
   int32_t fe, fneg;        // CG factor folded into A's digits: fm 2^fe, sign
   uint64_t fm;             // (fm = 0: factor 1)
+  double fac;              // the factor
   int32_t swap;            // block computed as C^T = op(B)^T op(A)^T: the A role reads the B arena
   // Real form of a complex block.  dupb = 0: A~ (2M x 2K) rows 2m, 2m+1 =
   // (Re, -Im), (Im, Re) of row m of op(A), B~ (2K x N) rows 2k, 2k+1 = (Re, Im)
@@ -124,11 +125,18 @@ constexpr int TILE_WORDS = (int)(sizeof(SplitTile) / 4);
 static_assert(sizeof(SplitTile) % 8 == 0 && TILE_WORDS <= 16, "tile descriptor fits one 64-byte slot");
 
 // ------------------------------------------------------------ bit helpers
-__device__ __forceinline__ int exp_key(double x) {
-  const long long b = __double_as_longlong(x);
-  const int be = (int)((b >> 52) & 0x7ff);
-  return ((b << 1) != 0) ? max(be, 1) : 0;
-}
+// Largest magnitude of a line, as far as its exponent goes: the high words'
+// maximum without the signs, and the low words' bits (a line of subnormals
+// below 2^-1042 has zero high words).
+struct LineMax {
+  unsigned hi = 0, lo = 0;
+  __device__ __forceinline__ void add(double x) {
+    hi = max(hi, (unsigned)__double2hiint(x) & 0x7fffffffu);
+    lo |= (unsigned)__double2loint(x);
+  }
+  // biased exponent of the maximum (at least 1), 0 for a line of zeros
+  __device__ __forceinline__ int key() const { return (hi | lo) ? max((int)(hi >> 20), 1) : 0; }
+};
 
 // A factor f (CG coefficient) as an exact integer mantissa and exponent,
 // f = fm * 2^fe; fm = 0 means "no factor" (f = 1); fe = -100000 means f = 0.
@@ -136,10 +144,11 @@ struct Factor {
   unsigned long long fm;
   int fe;
   bool neg;
+  double f;  // the factor itself
 };
 
 __host__ __device__ inline Factor make_factor(double f) {
-  Factor r{0ull, 0, false};
+  Factor r{0ull, 0, false, f};
   if (f == 1.0) return r;
   unsigned long long bits;
   memcpy(&bits, &f, 8);
@@ -210,10 +219,81 @@ __device__ __forceinline__ void digits_f(long long N, float (&d)[S]) {
   d[0] = __int_as_float(0x4B400000 + d0) - 12582912.0f;
 }
 
-// Two BF16 values packed as (lo, hi) halves of a 32-bit word.
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t *>(&v);
+// ---- digits of two values as packed FP16 planes
+// The digits are integers of at most 9 bits, exact in FP16.  For 8-bit digits
+// a value is first brought into the fixed-point word
+//   W = N + sum_{t>=1} 2^7 2^(8(S-1-t)) + 2^9 2^(8(S-1)),
+// whose bytes are d_t + 128 and whose ten bits from 8(S-1) on are d_0 + 512
+// (bits above are not looked at).  One byte permute takes the same digit of
+// two values, one logic operation puts it behind the exponent of 1024 (an
+// FP16 whose last place is one) and one packed subtraction removes the
+// offset: 1.5 instructions per digit, against 3.5 with a shift, a mask, an
+// FP32 subtraction and a conversion (the strips' ALU pipe was 60-70 % busy).
+template <int S>
+__host__ __device__ constexpr unsigned long long word_offset() {
+  unsigned long long h = 0;
+  for (int t = 1; t < S; ++t) h = (h << 8) + 128;
+  return h + (512ull << (8 * (S - 1)));
+}
+
+// Words of at most six digits come from the FP64 pipe, idle otherwise: the low
+// mantissa bits of x f + C are N = round(x f 2^(8S-E)) plus C's own, for C =
+// 2^(E-8S) (2^52 + 2^51 + word_offset).  C is not a normal number for extreme
+// E: those lines take the integer form.
+template <int S>
+struct LineScale {
+  double c = 0.0;
+  bool fast = false;
+  __device__ __forceinline__ LineScale(int E) {
+    const int be = E - 8 * S + 52 + 1023;
+    fast = S <= 6 && be > 0 && be < 2046;
+    if (fast) c = __longlong_as_double(((long long)be << 52) + (1ll << 51) + (long long)word_offset<S>());
+  }
+};
+
+template <int S, int B>
+__device__ __forceinline__ unsigned long long fixed_word(double x, int E, const LineScale<S> &ls, const Factor &F) {
+  if constexpr (B == 8) {
+    if (S <= 6 && ls.fast) return (unsigned long long)__double_as_longlong(fma(x, F.f, ls.c));
+    return (unsigned long long)scaled_int(x, E, B * S, F) + word_offset<S>();
+  } else {
+    return (unsigned long long)scaled_int(x, E, B * S, F);
+  }
+}
+
+// Plane t of the digits of two values: (first, second) as the halves of w[t].
+template <int S, int B>
+__device__ __forceinline__ void digit_planes(unsigned long long w0, unsigned long long w1, uint32_t (&w)[S]) {
+  if constexpr (B == 8) {
+    const uint32_t l0 = (uint32_t)w0, h0 = (uint32_t)(w0 >> 32), l1 = (uint32_t)w1, h1 = (uint32_t)(w1 >> 32);
+    const __half2 off = __float2half2_rn(1152.0f), off0 = __float2half2_rn(1536.0f);
+    auto sub = [](uint32_t v, __half2 o) {
+      const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&v), o);
+      return *reinterpret_cast<const uint32_t *>(&d);
+    };
+#pragma unroll
+    for (int t = 1; t < S; ++t) {
+      const int by = S - 1 - t;
+      const uint32_t k = by & 3, sel = k | ((4 + k) << 8);
+      const uint32_t u = by < 4 ? __byte_perm(l0, l1, sel) : __byte_perm(h0, h1, sel);
+      w[t] = sub((u & 0x00FF00FFu) | 0x64006400u, off);
+    }
+    constexpr int top = S - 1;  // first byte of the leading field
+    uint32_t u;
+    if constexpr (top == 3) u = __byte_perm(__funnelshift_r(l0, h0, 24), __funnelshift_r(l1, h1, 24), 0x5410);
+    else if constexpr (top < 3) u = __byte_perm(l0, l1, top == 1 ? 0x6521 : 0x7632);
+    else u = __byte_perm(h0, h1, top == 4 ? 0x5410 : top == 5 ? 0x6521 : 0x7632);
+    w[0] = sub((u & 0x03FF03FFu) | 0x64006400u, off0);
+  } else {
+    float d0[S], d1[S];
+    digits_f<S, B>((long long)w0, d0);
+    digits_f<S, B>((long long)w1, d1);
+#pragma unroll
+    for (int t = 0; t < S; ++t) {
+      const __half2 v = __floats2half2_rn(d0[t], d1[t]);
+      w[t] = *reinterpret_cast<const uint32_t *>(&v);
+    }
+  }
 }
 
 // L2 eviction priorities of the strip kernels (createpolicy, PTX ISA 7.4+):
@@ -317,7 +397,7 @@ __device__ __forceinline__ void strip_maxima(const SplitPair *__restrict__ pairs
     constexpr int NPH = STRIP_THREADS / STRIP;
     const int line = contig ? threadIdx.x / NPH : threadIdx.x % STRIP;
     const int ph = contig ? threadIdx.x % NPH : threadIdx.x / STRIP;
-    int key = 0;
+    LineMax lm;
     if (line < nl) {
       const uint64_t keep = l2_policy_keep();
       const int64_t base = off + ad.line(l0 + line);
@@ -327,25 +407,30 @@ __device__ __forceinline__ void strip_maxima(const SplitPair *__restrict__ pairs
                       o3 = base + ad.depth(k + 3 * NPH);
         if (CPLX) {
           const double2 *x = reinterpret_cast<const double2 *>(X);
-          const double2 v0 = ld_pol(x + o0, keep), v1 = ld_pol(x + o1, keep), v2 = ld_pol(x + o2, keep),
-                        v3 = ld_pol(x + o3, keep);
-          key = max(key, max(max(max(exp_key(v0.x), exp_key(v0.y)), max(exp_key(v1.x), exp_key(v1.y))),
-                             max(max(exp_key(v2.x), exp_key(v2.y)), max(exp_key(v3.x), exp_key(v3.y)))));
+          const double2 v[4] = {ld_pol(x + o0, keep), ld_pol(x + o1, keep), ld_pol(x + o2, keep), ld_pol(x + o3, keep)};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            lm.add(v[u].x);
+            lm.add(v[u].y);
+          }
         } else {
-          key = max(key, max(max(exp_key(ld_pol(X + o0, keep)), exp_key(ld_pol(X + o1, keep))),
-                             max(exp_key(ld_pol(X + o2, keep)), exp_key(ld_pol(X + o3, keep)))));
+          const double v[4] = {ld_pol(X + o0, keep), ld_pol(X + o1, keep), ld_pol(X + o2, keep), ld_pol(X + o3, keep)};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) lm.add(v[u]);
         }
       }
       for (; k < P.K; k += NPH) {
         const int64_t o = base + ad.depth(k);
         if (CPLX) {
           const double2 v = ld_pol(reinterpret_cast<const double2 *>(X) + o, keep);
-          key = max(key, max(exp_key(v.x), exp_key(v.y)));
+          lm.add(v.x);
+          lm.add(v.y);
         } else {
-          key = max(key, exp_key(ld_pol(X + o, keep)));
+          lm.add(ld_pol(X + o, keep));
         }
       }
     }
+    int key = lm.key();
     // an infinity or NaN: no scale; every tile that reads the line goes to the FP64 kernel
     if (HP && key == 0x7ff) key = NONFINITE_EXP + 1022 - (ROLE_B ? 0 : P.e_afac);
     if (key) atomicMax(&smax[line], key - 1022 + (ROLE_B ? 0 : P.e_afac));
@@ -382,7 +467,7 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
     const double *__restrict__ A = P.swap ? Barena : Aarena;
     const bool ca = P.trans & 4;
     const OpAddr ad = addr_a(P, views, p);
-    const Factor Fa{P.fm, P.fe, P.fneg != 0};
+    const Factor Fa{P.fm, P.fe, P.fneg != 0, P.fac};
     uint8_t *tiles = arena + P.as_off + (int64_t)mt * P.KB * NP * A_DIGIT_BYTES;
     if (dup) {
       // item = one row of op(A) (real rows 2m, 2m+1) x 4 complex k
@@ -400,18 +485,19 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
           a[j] = make_double2(0.0, 0.0);
           if (k < P.K) a[j] = ld_pol(reinterpret_cast<const double2 *>(A) + lo + ad.depth(k), last);
         }
-        // row 2m: ( re, -im ); row 2m+1 is formed from it at the store, which
-        // saves half of the digit registers (72 -> 54, two more CTAs per SM;
-        // the strips of the 2000-product batch 1.98 -> 1.89 ms)
+        // ( re, im ) per plane; the rows 2m and 2m+1 are formed from it at the
+        // stores, which saves half of the digit registers (72 -> 54, two more
+        // CTAs per SM; the strips of the 2000-product batch 1.98 -> 1.89 ms)
         uint32_t pw[NP][4];
+        const LineScale<S> ls(Ei);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          float dr[S], di[S];
-          digits_f<S, B>(scaled_int(a[j].x, Ei, B * S, Fa), dr);
-          digits_f<S, B>(scaled_int(ca ? -a[j].y : a[j].y, Ei, B * S, Fa), di);
+          uint32_t w2[S];
+          digit_planes<S, B>(fixed_word<S, B>(a[j].x, Ei, ls, Fa),
+                             fixed_word<S, B>(ca ? -a[j].y : a[j].y, Ei, ls, Fa), w2);
 #pragma unroll
-          for (int t = 0; t < S; ++t) pw[t][j] = pack2(dr[t], -di[t]);
-          if constexpr (HP) pw[S][j] = pw[0][j] & 0x7FFF7FFFu;
+          for (int t = 0; t < S; ++t) pw[t][j] = w2[t];
+          if constexpr (HP) pw[S][j] = w2[0] & 0x7FFF7FFFu;
         }
         const int rr0 = rl + 2 * ml, rr1 = rr0 + 1;
         uint8_t *tile = tiles + (int64_t)kb * NP * A_DIGIT_BYTES;
@@ -419,12 +505,13 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
         uint8_t *d1 = tile + ((rr1 >> 3) * KCM + q) * 128 + (rr1 & 7) * 16;
 #pragma unroll
         for (int t = 0; t < NP; ++t) {
-          st_pol(d0 + t * A_DIGIT_BYTES, make_uint4(pw[t][0], pw[t][1], pw[t][2], pw[t][3]), last);
-          // row 2m+1: ( im, re ) = the halves of row 2m exchanged, the sign of im flipped back
-          const uint32_t flip = t < S ? 0x8000u : 0u;
+          const uint32_t neg = t < S ? 0x80000000u : 0u;  // row 2m: ( re, -im )
+          st_pol(d0 + t * A_DIGIT_BYTES,
+                 make_uint4(pw[t][0] ^ neg, pw[t][1] ^ neg, pw[t][2] ^ neg, pw[t][3] ^ neg), last);
+          // row 2m+1: ( im, re )
           st_pol(d1 + t * A_DIGIT_BYTES,
-                 make_uint4(__byte_perm(pw[t][0], 0, 0x1032) ^ flip, __byte_perm(pw[t][1], 0, 0x1032) ^ flip,
-                            __byte_perm(pw[t][2], 0, 0x1032) ^ flip, __byte_perm(pw[t][3], 0, 0x1032) ^ flip),
+                 make_uint4(__byte_perm(pw[t][0], 0, 0x1032), __byte_perm(pw[t][1], 0, 0x1032),
+                            __byte_perm(pw[t][2], 0, 0x1032), __byte_perm(pw[t][3], 0, 0x1032)),
                  last);
         }
       }
@@ -446,13 +533,14 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
             a[j] = make_double2(0.0, 0.0);
             if (k < P.K) a[j] = ld_pol(reinterpret_cast<const double2 *>(A) + lo + ad.depth(k), last);
           }
+          const LineScale<S> ls(Ei);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            float dr[S], di[S];
-            digits_f<S, B>(scaled_int(a[j].x, Ei, B * S, Fa), dr);
-            digits_f<S, B>(scaled_int(ca ? -a[j].y : a[j].y, Ei, B * S, Fa), di);
+            uint32_t w2[S];
+            digit_planes<S, B>(fixed_word<S, B>(a[j].x, Ei, ls, Fa),
+                               fixed_word<S, B>(ca ? -a[j].y : a[j].y, Ei, ls, Fa), w2);
 #pragma unroll
-            for (int t = 0; t < S; ++t) pk[t][j] = pack2(dr[t], di[t]);
+            for (int t = 0; t < S; ++t) pk[t][j] = w2[t];
           }
         } else {
           double v[8];
@@ -462,13 +550,13 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
             v[e] = 0.0;
             if (kk < P.Kr) v[e] = ld_pol(A + lo + ad.depth(kk), last);
           }
+          const LineScale<S> ls(Ei);
 #pragma unroll
           for (int e = 0; e < 8; e += 2) {
-            float d0[S], d1[S];
-            digits_f<S, B>(scaled_int(v[e], Ei, B * S, Fa), d0);
-            digits_f<S, B>(scaled_int(v[e + 1], Ei, B * S, Fa), d1);
+            uint32_t w2[S];
+            digit_planes<S, B>(fixed_word<S, B>(v[e], Ei, ls, Fa), fixed_word<S, B>(v[e + 1], Ei, ls, Fa), w2);
 #pragma unroll
-            for (int t = 0; t < S; ++t) pk[t][e >> 1] = pack2(d0[t], d1[t]);
+            for (int t = 0; t < S; ++t) pk[t][e >> 1] = w2[t];
           }
         }
         if constexpr (HP) {
@@ -509,7 +597,7 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
   }
   const int nt = c0 / TNS, cl = c0 % TNS;
   const int ncols = dup ? 2 * nl : nl;  // real columns of this strip inside the block
-  const Factor F1{0ull, 0, false};
+  const Factor F1{0ull, 0, false, 1.0};
   const uint64_t last = l2_policy_stream();  // last use of operand lines; digit stores
   for (int p = p0; p < p1; ++p) {
     const SplitPair &P = pairs[p];
@@ -537,15 +625,17 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
           x[j] = make_double2(0.0, 0.0);
           if (k < P.K) x[j] = ld_pol(reinterpret_cast<const double2 *>(Bm) + lo + ad.depth(k), last);
         }
+        // B-duplicated form: even columns ( re; -im ), odd ones ( im; re )
         const bool odd = dup && (cloc & 1);
+        const uint32_t sel = odd ? 0x1032u : 0x3210u, neg = dup && !odd ? 0x80000000u : 0u;
+        const LineScale<S> ls(Fj);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          float dr[S], di[S];
-          digits_f<S, B>(scaled_int(x[j].x, Fj, B * S, F1), dr);
-          digits_f<S, B>(scaled_int(cb ? -x[j].y : x[j].y, Fj, B * S, F1), di);
+          uint32_t w2[S];
+          digit_planes<S, B>(fixed_word<S, B>(x[j].x, Fj, ls, F1),
+                             fixed_word<S, B>(cb ? -x[j].y : x[j].y, Fj, ls, F1), w2);
 #pragma unroll
-          for (int t = 0; t < S; ++t)
-            pk[t][j] = dup ? (odd ? pack2(di[t], dr[t]) : pack2(dr[t], -di[t])) : pack2(dr[t], di[t]);
+          for (int t = 0; t < S; ++t) pk[t][j] = dup ? __byte_perm(w2[t], 0, sel) ^ neg : w2[t];
         }
       } else {
         const int64_t lo = P.b_off + ad.line(l0 + cloc);
@@ -556,13 +646,13 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
           v[e] = 0.0;
           if (kk < P.Kr) v[e] = ld_pol(Bm + lo + ad.depth(kk), last);
         }
+        const LineScale<S> ls(Fj);
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {
-          float d0[S], d1[S];
-          digits_f<S, B>(scaled_int(v[e], Fj, B * S, F1), d0);
-          digits_f<S, B>(scaled_int(v[e + 1], Fj, B * S, F1), d1);
+          uint32_t w2[S];
+          digit_planes<S, B>(fixed_word<S, B>(v[e], Fj, ls, F1), fixed_word<S, B>(v[e + 1], Fj, ls, F1), w2);
 #pragma unroll
-          for (int t = 0; t < S; ++t) pk[t][e >> 1] = pack2(d0[t], d1[t]);
+          for (int t = 0; t < S; ++t) pk[t][e >> 1] = w2[t];
         }
       }
       if constexpr (HP) {
@@ -681,11 +771,11 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint
   d |= (uint64_t)1 << 46;
   return d;
 }
-// kind::f16 instruction descriptor: D=F32, A=B=BF16, both K-major, N, M=128.
+// kind::f16 instruction descriptor: D=F32, A=B=FP16, both K-major, N, M=128.
 __host__ __device__ constexpr uint32_t make_idesc(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TMS >> 4) << 24);
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TMS >> 4) << 24);
 }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -1003,12 +1093,12 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
                 const uint64_t ad = dst0 + (uint64_t)((t * A_DIGIT_BYTES + ks * 256) >> 4);
                 const uint64_t bd = dst0 + (uint64_t)((A_BYTES + ks * 256) >> 4);
                 const uint32_t acc = (fresh && ks == 0 && t == 0) ? 0u : 1u;
-                umma_bf16(dset + (uint32_t)(t * TNS), ad, bd, idesc[S - 1 - t], acc);
+                umma_f16(dset + (uint32_t)(t * TNS), ad, bd, idesc[S - 1 - t], acc);
               }
               if constexpr (HP) {
                 const uint64_t ad = dst0 + (uint64_t)((S * A_DIGIT_BYTES + ks * 256) >> 4);
                 const uint64_t bd = dst0 + (uint64_t)((A_BYTES + S * B_DIGIT_BYTES + ks * 256) >> 4);
-                umma_bf16(dset + (uint32_t)(S * TNS), ad, bd, idesc[0], (fresh && ks == 0) ? 0u : 1u);
+                umma_f16(dset + (uint32_t)(S * TNS), ad, bd, idesc[0], (fresh && ks == 0) ? 0u : 1u);
               }
             }
             fresh = false;
@@ -1487,6 +1577,7 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
       s.fm = f.fm;
       s.fe = f.fe;
       s.fneg = f.neg ? 1 : 0;
+      s.fac = d.afac;
       int e = 0;
       if (d.afac != 1.0 && d.afac != 0.0) std::frexp(d.afac, &e);
       s.e_afac = e;
