@@ -137,6 +137,22 @@ void DevLists::commit(Ctx *ctx) {
   ctx->stage_commit(base_, sent_);
 }
 
+void Ctx::ensure_ret(size_t bytes) {
+  if (bytes <= ret_cap) return;
+  QS_CUDA(cudaStreamSynchronize(stream));  // nothing may still write the old buffer
+  if (ret_buf) cudaFreeHost(ret_buf);
+  ret_buf = ret_dev = nullptr;
+  ret_cap = 0;
+  const size_t cap = std::max<size_t>(bytes * 2, 64 << 10);
+  cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&ret_buf), cap, cudaHostAllocMapped);
+  if (e != cudaSuccess) {
+    ret_buf = nullptr;
+    fail(QS_ERR_OOM, "page-locked result buffer of %zu bytes: %s", cap, cudaGetErrorString(e));
+  }
+  QS_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&ret_dev), ret_buf, 0));
+  ret_cap = cap;
+}
+
 void Ctx::destroy_staging() {
   if (stream) cudaStreamSynchronize(stream);
   for (auto &m : stage_q) cudaEventDestroy(m.ev);
@@ -146,6 +162,9 @@ void Ctx::destroy_staging() {
   if (stage_buf) cudaFreeHost(stage_buf);
   stage_buf = stage_dev = nullptr;
   stage_cap = 0;
+  if (ret_buf) cudaFreeHost(ret_buf);
+  ret_buf = ret_dev = nullptr;
+  ret_cap = 0;
 }
 
 void Ctx::ensure_copy_streams() {
@@ -236,20 +255,16 @@ static void run_permute(Ctx *ctx, const std::vector<PermDesc> &descs_in, const d
     descs.push_back(d);
   }
   if (descs.empty()) return;
-  PermDesc *dd = dev_upload(ctx, descs);
-  int64_t *dcb = cb.empty() ? nullptr : dev_upload(ctx, cb);
-  int64_t *dcs = cs.empty() ? nullptr : dev_upload(ctx, cs);
-  PermTile *dt = tiles.empty() ? nullptr : dev_upload(ctx, tiles);
+  DevLists L;
+  const size_t sd = L.add(descs), sb = L.add(cb), ss = L.add(cs), st = L.add(tiles);
+  L.commit(ctx);
   if (timed) ctx->mark(0);
-  launch_permute(ctx, dd, dcb, dcs, (int64_t)cb.size(), dt, (int64_t)tiles.size(), in, out, cplx ? 1 : 0, CH);
+  launch_permute(ctx, L.at<PermDesc>(sd), L.at<int64_t>(sb), L.at<int64_t>(ss), (int64_t)cb.size(),
+                 L.at<PermTile>(st), (int64_t)tiles.size(), in, out, cplx ? 1 : 0, CH);
   if (timed) {
     ctx->mark(1);
     ctx->mark(2);
   }
-  dev_free(ctx, dd);
-  if (dcb) dev_free(ctx, dcb);
-  if (dcs) dev_free(ctx, dcs);
-  if (dt) dev_free(ctx, dt);
 }
 
 // Rank-2 exemption of SkipZeroData (Source/QSpace.cc:3225-3229): zero blocks
@@ -462,29 +477,25 @@ static void prepare(Ctx *ctx, Prepared &w, const QMeta &Am, const double *dA, co
     const std::vector<int> &ks = is_a ? pl.ica.idx : pl.icb.idx;
     std::vector<OperandView> v(pl.pairs.size());
     std::vector<std::pair<int64_t, int64_t>> toff(pl.pairs.size());
-    std::unordered_map<int64_t, size_t> first;  // block -> first pair that reads it
+    std::vector<int64_t> first(m.nblk, -1);  // block -> first pair that reads it
     const size_t tab0 = vtab.size();
     for (size_t p = 0; p < pl.pairs.size(); ++p) {
       const int64_t blk = is_a ? pl.pair_ia[p] : pl.pair_ib[p];
-      auto it = first.find(blk);
-      if (it != first.end()) {
-        v[p] = v[it->second];
-        toff[p] = toff[it->second];
+      if (first[blk] >= 0) {
+        v[p] = v[first[blk]];
+        toff[p] = toff[first[blk]];
         continue;
       }
       if (!make_view(m, blk, lines, ks, v[p])) {
         vtab.resize(tab0);
         return false;
       }
-      if (all_direct) {  // the direct kernel takes the legs themselves
-        first.emplace(blk, p);
-        continue;
-      }
+      first[blk] = (int64_t)p;
+      if (all_direct) continue;  // the direct kernel takes the legs themselves
       toff[p] = {(int64_t)vtab.size(), 0};
       append_offsets(v[p].nl, v[p].ldim, v[p].lstr, vtab);
       toff[p].second = (int64_t)vtab.size();
       append_offsets(v[p].nk, v[p].kdim, v[p].kstr, vtab);
-      first.emplace(blk, p);
     }
     out.swap(v);
     (is_a ? toff_a : toff_b).swap(toff);
@@ -555,7 +566,20 @@ static void run_products(Ctx *ctx, const std::vector<Prepared *> &batch, const q
   std::vector<int32_t> bM, bN;
   std::vector<OperandView> va, vb;
   bool any_view = false;
-  for (Prepared *w : batch) any_view = any_view || !w->va.empty() || !w->vb.empty();
+  size_t np = 0, nbk = 0;
+  for (Prepared *w : batch) {
+    any_view = any_view || !w->va.empty() || !w->vb.empty();
+    np += w->pl.pairs.size();
+    nbk += w->pl.blk_M.size();
+  }
+  pairs.reserve(np);
+  if (any_view) {
+    va.reserve(np);
+    vb.reserve(np);
+  }
+  for (auto *v : {&bM, &bN}) v->reserve(nbk);
+  c_off.reserve(nbk);
+  grp.reserve(nbk + 1);
   for (Prepared *w : batch) {
     const ContractPlan &pl = w->pl;
     const int64_t da = rel(w->a2, baseA), db = rel(w->b2, baseB), dc = rel(w->dC, baseC);
@@ -618,17 +642,20 @@ static void finish(Ctx *ctx, const std::vector<Prepared *> &batch) {
     first[r + 1] = (int64_t)offs.size();
   }
   const int64_t nb = (int64_t)offs.size();
-  int64_t *doff = dev_upload(ctx, offs), *dsz = dev_upload(ctx, sizes);
-  int *dflag = dev_alloc<int>(ctx, nb);
-  launch_block_nonzero(ctx, doff, dsz, nb, base, batch[0]->cplx ? 1 : 0, dflag);
   std::vector<int> flags(nb);
   int kerr = 0;
-  QS_CUDA(cudaMemcpyAsync(flags.data(), dflag, nb * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  QS_CUDA(cudaMemcpyAsync(&kerr, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  QS_CUDA(cudaStreamSynchronize(ctx->stream));
-  dev_free(ctx, doff);
-  dev_free(ctx, dsz);
-  dev_free(ctx, dflag);
+  {
+    DevLists L;
+    const size_t so = L.add(offs), sz = L.add(sizes);
+    L.commit(ctx);
+    ctx->ensure_ret((size_t)(nb + 1) * sizeof(int));
+    launch_block_nonzero(ctx, L.at<int64_t>(so), L.at<int64_t>(sz), nb, base, batch[0]->cplx ? 1 : 0,
+                         reinterpret_cast<int *>(ctx->ret_dev));
+    QS_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int *ret = reinterpret_cast<const int *>(ctx->ret_buf);
+    std::copy(ret, ret + nb, flags.begin());
+    kerr = ret[nb];
+  }
   if (kerr) {
     QS_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
     fail(QS_ERR_TIMEOUT, "a bounded device wait ran out (code %d)", kerr);
@@ -670,10 +697,16 @@ static void finish(Ctx *ctx, const std::vector<Prepared *> &batch) {
       w.dC = nullptr;
       M.rank = 0;
     } else if (pl.P.empty()) {
-      for (int64_t i : keep) {
-        M.q.insert(M.q.end(), pl.C.qrow(i), pl.C.qrow(i) + rk * qd);
-        M.dims.insert(M.dims.end(), pl.C.drow(i), pl.C.drow(i) + rk);
-        M.offs.push_back(pl.C.offs[i]);
+      if ((int64_t)keep.size() == nbr) {
+        M.q = pl.C.q;
+        M.dims = pl.C.dims;
+        M.offs = pl.C.offs;
+      } else {
+        for (int64_t i : keep) {
+          M.q.insert(M.q.end(), pl.C.qrow(i), pl.C.qrow(i) + rk * qd);
+          M.dims.insert(M.dims.end(), pl.C.drow(i), pl.C.drow(i) + rk);
+          M.offs.push_back(pl.C.offs[i]);
+        }
       }
       M.nelem = pl.C.nelem;
       T->d = w.dC;
@@ -1043,7 +1076,13 @@ qs_status qs_contractQS(qs_ctx *ctx, const qs_qspace_view *A, const char *ia,
   *C = nullptr;
   QS_CUDA(cudaSetDevice(ctx->c.device));
   auto tA = upload(&ctx->c, A);
-  auto tB = upload(&ctx->c, B);
+  // an operand contracted with itself (a density matrix, a norm) is sent once
+  std::unique_ptr<qs_tensor> own;
+  const qs_tensor *tB = tA.get();
+  if (B != A) {
+    own = upload(&ctx->c, B);
+    tB = own.get();
+  }
   auto tC = contract_core(&ctx->c, tA->meta, tA->d, tB->meta, tB->d, ia, ib, perm, nperm, opts, stats);
   *C = download(&ctx->c, tC.get());
   QS_API_END

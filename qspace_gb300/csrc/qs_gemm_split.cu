@@ -1314,20 +1314,37 @@ static int kchunk_of(int b, int S) {
 // Accumulator drains of one output block: a new chunk starts when the next K
 // block would push the chunk's summed depth above kchunk (the MMA issuer
 // applies the same rule).
+// (counted per pair, not per K block: a reduced density matrix over a large
+// bond sums 10^5 blocks, which took 0.6 ms of a call)
 static int chunks_of(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int cm, int kchunk) {
-  int nchunk = 1, depth = 0;
+  const int64_t per = std::max(1, kchunk / TKS);  // whole K blocks of a chunk
+  int64_t nchunk = 1, depth = 0;
   bool fresh = true;
   for (int64_t p = p0; p < p1; ++p) {
-    const int Kr = pairs[p].K * cm;
-    const int KB = std::max(1, (Kr + TKS - 1) / TKS);
-    for (int kb = 0; kb < KB; ++kb) {
-      const int dk = std::max(std::min(TKS, Kr - kb * TKS), 0);
-      if (!fresh && depth + dk > kchunk) { ++nchunk; depth = 0; fresh = true; }
-      depth += dk;
+    const int64_t Kr = std::max<int64_t>((int64_t)pairs[p].K * cm, 0);
+    int64_t whole = Kr / TKS;
+    const int64_t tail = Kr % TKS;
+    if (whole > 0) {
+      const int64_t room = fresh ? per : std::max<int64_t>(0, (kchunk - depth) / TKS);
+      if (whole <= room) {
+        depth += whole * TKS;
+      } else {
+        whole -= room;
+        nchunk += (whole + per - 1) / per;
+        depth = ((whole - 1) % per + 1) * TKS;
+      }
+      fresh = false;
+    }
+    if (tail > 0 || Kr == 0) {
+      if (!fresh && depth + tail > kchunk) {
+        ++nchunk;
+        depth = 0;
+      }
+      depth += tail;
       fresh = false;
     }
   }
-  return nchunk;
+  return (int)nchunk;
 }
 
 // Digit plan: the (bits, digits) pair that reaches the wanted precision at
@@ -1721,6 +1738,25 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
                                    int forced_bits, const std::vector<OperandView> *va,
                                    const std::vector<OperandView> *vb);
 
+// Sends a planned product's work lists (one staging copy; L keeps them until
+// the launches are queued) and launches it; the arena and the flags are set.
+static void run_split_work(Ctx *ctx, const SplitWork &w, bool cplx, SplitDev d, DevLists &L, const double *A,
+                           const double *B, double *C, bool marks) {
+  const size_t sp = L.add(w.sp), sa = L.add(w.sa), sb = L.add(w.sb), st = L.add(w.tiles);
+  const size_t va = L.add(w.va), vb = L.add(w.vb);
+  const size_t se = L.space((size_t)w.nE * sizeof(int)), sf = L.space((size_t)w.nF * sizeof(int));
+  L.commit(ctx);
+  d.pairs = L.at<SplitPair>(sp);
+  d.sa = L.at<int4>(sa);
+  d.sb = L.at<int4>(sb);
+  d.tiles = L.at<SplitTile>(st);
+  if (!w.va.empty()) d.va = L.at<OperandView>(va);
+  if (!w.vb.empty()) d.vb = L.at<OperandView>(vb);
+  d.E = L.at<int>(se);
+  d.F = L.at<int>(sf);
+  launch_split(ctx, w, cplx, d, A, B, C, ctx->d_err, true, marks);
+}
+
 // Shallow output blocks (summed depth <= SHALLOW_K) are computed directly in
 // FP64 (run_shallow); deep ones (few tiles, a very deep sum) are cut along
 // their depth into parts computed as blocks of their own in a temporary
@@ -1836,26 +1872,11 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
   SplitResult res = plan_split(pairs, grp, blk_M, blk_N, c_off, cplx, forced_slices, tol, blk_ldc, w, forced_bits,
                                va, vb);
   if (w.tiles.empty()) return res;
-  // device buffers: one allocation for the digit arena (pooled scratch)
+  // the digit arena is pooled scratch
   SplitDev d;
   d.arena = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)std::max<int64_t>(w.arena, 256)));
-  d.pairs = dev_upload(ctx, w.sp);
-  d.sa = dev_upload(ctx, w.sa);
-  d.sb = dev_upload(ctx, w.sb);
-  d.tiles = dev_upload(ctx, w.tiles);
-  if (!w.va.empty()) d.va = dev_upload(ctx, w.va);
-  if (!w.vb.empty()) d.vb = dev_upload(ctx, w.vb);
-  d.E = dev_alloc<int>(ctx, (size_t)w.nE);
-  d.F = dev_alloc<int>(ctx, (size_t)w.nF);
-  launch_split(ctx, w, cplx, d, A, B, C, ctx->d_err);
-  dev_free(ctx, d.pairs);
-  dev_free(ctx, d.sa);
-  dev_free(ctx, d.sb);
-  if (d.va) dev_free(ctx, d.va);
-  if (d.vb) dev_free(ctx, d.vb);
-  dev_free(ctx, d.tiles);
-  dev_free(ctx, d.E);
-  dev_free(ctx, d.F);
+  DevLists L;
+  run_split_work(ctx, w, cplx, d, L, A, B, C, true);
   return res;
 }
 
@@ -2037,20 +2058,11 @@ bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDes
   for (size_t k = 0; k < ws.size(); ++k) {
     const SplitWork &w = ws[k];
     if (w.tiles.empty()) continue;
-    DevLists L;
-    const size_t sp = L.add(w.sp), sa = L.add(w.sa), sb = L.add(w.sb), st = L.add(w.tiles);
-    const size_t se = L.space((size_t)w.nE * sizeof(int)), sf = L.space((size_t)w.nF * sizeof(int));
-    L.commit(ctx);
     SplitDev d;
     d.arena = digits;
     d.flags = d_flags;
-    d.pairs = L.at<SplitPair>(sp);
-    d.sa = L.at<int4>(sa);
-    d.sb = L.at<int4>(sb);
-    d.tiles = L.at<SplitTile>(st);
-    d.E = L.at<int>(se);
-    d.F = L.at<int>(sf);
-    launch_split(ctx, w, cplx, d, A, B, C, ctx->d_err, true, k == 0);
+    DevLists L;
+    run_split_work(ctx, w, cplx, d, L, A, B, C, k == 0);
   }
   return true;
 }

@@ -76,6 +76,11 @@ struct Ctx {
   char *stage_reserve(size_t bytes);
   void stage_commit(void *dst, size_t bytes);
   void destroy_staging();
+  // mapped page-locked memory that a kernel writes small results to (read by
+  // the host after a stream synchronisation): no copy back
+  char *ret_buf = nullptr, *ret_dev = nullptr;
+  size_t ret_cap = 0;
+  void ensure_ret(size_t bytes);
   // copy streams of the pipelined host-buffer path (created on first use)
   cudaStream_t h2d = nullptr, d2h = nullptr;
   void ensure_copy_streams();
@@ -278,9 +283,10 @@ void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles,
 
 // qs_permute.cu -- per-block "all zero" test for SkipZeroData, and the
 // real -> complex widening of an operand arena
+// (flags[nblk] receives the context's error word)
 void launch_block_nonzero(Ctx *ctx, const int64_t *d_offs, const int64_t *d_sizes,
                           int64_t nblk, const double *data, int is_complex,
-                          int *d_flags);
+                          int *flags);
 void launch_widen(Ctx *ctx, const double *in, double *out, int64_t n);
 // dst block b += f * src block b (element offsets / sizes; es = 1 real, 2
 // complex; a real source into a complex destination adds to the real parts)

@@ -240,11 +240,18 @@ void launch_block_axpy(Ctx *ctx, const int64_t *d_soff, const int64_t *d_doff, c
 }
 
 // Per-block nonzero test (SkipZeroData with eps = 0, Source/QSpace.cc:
-// 3201-3269): flags[b] = 1 when any element of block b differs from zero.
+// 3201-3269): flags[b] = 1 when any element of block b differs from zero;
+// flags[nblk] = the error word of the launches before.  The flags go to mapped
+// host memory, so the host reads them after one synchronisation (two copies
+// back to pageable memory took 25 us of every contraction).
 __global__ void block_nonzero_kernel(const int64_t *__restrict__ offs,
                                      const int64_t *__restrict__ sizes, const double *__restrict__ data,
-                                     int cplx, int *__restrict__ flags) {
+                                     int cplx, int *__restrict__ flags, const int *__restrict__ err) {
   const int64_t b = blockIdx.x;
+  if (b + 1 == gridDim.x) {
+    if (threadIdx.x == 0) flags[b] = *err;
+    return;
+  }
   const int64_t n = sizes[b] * (cplx ? 2 : 1);
   const double *p = data + offs[b] * (cplx ? 2 : 1);
   int nz = 0;
@@ -254,10 +261,10 @@ __global__ void block_nonzero_kernel(const int64_t *__restrict__ offs,
 }
 
 void launch_block_nonzero(Ctx *ctx, const int64_t *d_offs, const int64_t *d_sizes,
-                          int64_t nblk, const double *data, int is_complex, int *d_flags) {
+                          int64_t nblk, const double *data, int is_complex, int *flags) {
   if (nblk <= 0) return;
-  block_nonzero_kernel<<<(unsigned)nblk, 128, 0, ctx->stream>>>(d_offs, d_sizes, data,
-                                                                 is_complex, d_flags);
+  block_nonzero_kernel<<<(unsigned)(nblk + 1), 128, 0, ctx->stream>>>(d_offs, d_sizes, data, is_complex, flags,
+                                                                      ctx->d_err);
   QS_LAUNCHED(ctx);
 }
 

@@ -81,17 +81,18 @@ class QSpace:
             q = np.ascontiguousarray(q.reshape(n, r * qd), dtype=np.int32)
         else:
             q = np.zeros((0,), np.int32)
-        dims = np.array([self.block_dims(i) for i in range(n)], dtype=np.int64).reshape(n, r)
+        if all(type(d) is np.ndarray and d.ndim == r for d in self.data):
+            dims = np.array([d.shape for d in self.data], dtype=np.int64).reshape(n, r)
+        else:
+            dims = np.array([self.block_dims(i) for i in range(n)], dtype=np.int64).reshape(n, r)
         sizes = np.prod(dims, axis=1) if r else np.ones(n, np.int64)
         offs = np.zeros(n, np.int64)
         if n > 1:
             offs[1:] = np.cumsum(sizes)[:-1]
         total = int(sizes.sum()) if n else 0
         buf = np.empty(total, dtype=np.complex128 if cplx else np.float64)
-        for i, d in enumerate(self.data):
-            a = np.asarray(d, dtype=buf.dtype)
-            buf[offs[i]:offs[i] + sizes[i]] = a.reshape(-1, order="F") if a.ndim > 1 else a.reshape(-1)
-        dims = np.ascontiguousarray(dims)
+        if n:
+            np.concatenate([np.ravel(d, order="F") for d in self.data], out=buf, casting="unsafe")
         v = QSpaceView()
         v.rank, v.qdim, v.nblk = r, qd, n
         v.q = q.ctypes.data_as(_capi.c_int32_p)
@@ -114,11 +115,8 @@ class QSpace:
         arr = np.asarray(data)
         if cplx:
             arr = arr.view(np.complex128)
-        blocks = []
-        for i in range(n):
-            s = int(np.prod(dims[i])) if rank else 1
-            blk = arr[offs[i]:offs[i] + s]
-            blocks.append(blk.reshape(tuple(dims[i]), order="F") if rank else blk.reshape(()))
+        sizes = np.prod(dims, axis=1).tolist() if rank else [1] * n
+        blocks = [arr[o:o + s].reshape(d, order="F") for o, s, d in zip(offs.tolist(), sizes, dims.tolist())]
         Q = [np.ascontiguousarray(q[:, k, :]) for k in range(rank)]
         return cls(Q, blocks, dict(info or {}))
 
@@ -264,7 +262,7 @@ def contractQS(A, ia=None, B: QSpace | None = None, ib=None, perm=None, *, prec:
         return contract_itags(A, ia, prec=prec, nslices=nslices, tol=tol, ctx=ctx)
     ctx = ctx or default_context()
     va, ka = A.pack()
-    vb, kb = B.pack()
+    vb, kb = (va, ka) if B is A else B.pack()
     p, n = _perm_arg(perm)
     o = make_opts(prec, nslices, tol)
     st = Stats()
