@@ -713,6 +713,19 @@ strip_b_kernel(const SplitPair *__restrict__ pairs, const OperandView *__restric
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
+// One lane of a converged warp.  A branch on elect.sync tells the compiler that
+// a single thread runs it: operands of tcgen05.mma, commits and bulk copies then
+// reach the uniform registers directly (12 clocks an instruction; 46 behind a
+// branch on the lane number, where they go through a loop over active lanes).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(e));
+  return e != 0;
+}
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -993,7 +1006,7 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------------------------ TMA producer
       int it = 0, st = 0;  // stage it % nstages, its phase bit ph
       uint32_t ph = 0;
@@ -1031,7 +1044,7 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------------------------ MMA issuer
       // one instruction per A digit t: N = (S - t) * 32 columns of B digits
       uint32_t idesc[S];
@@ -1086,21 +1099,29 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
             tc_fence_after();
             const uint64_t dst0 = desc0 + (uint64_t)((st * STAGE_BYTES) >> 4);
             const uint32_t dset = tmem + (uint32_t)((u & 1) * SET_COLS);
+            // digit t of K step ks: N = (S - t) * 32 columns
+            auto digit = [&](int t, int ks) {
+              const uint64_t ad = dst0 + (uint64_t)((t * A_DIGIT_BYTES + ks * 256) >> 4);
+              const uint64_t bd = dst0 + (uint64_t)((A_BYTES + ks * 256) >> 4);
+              umma_f16(dset + (uint32_t)(t * TNS), ad, bd, idesc[S - 1 - t], (fresh && ks == 0 && t == 0) ? 0u : 1u);
+            };
+            auto magnitude = [&](int ks) {
+              const uint64_t ad = dst0 + (uint64_t)((S * A_DIGIT_BYTES + ks * 256) >> 4);
+              const uint64_t bd = dst0 + (uint64_t)((A_BYTES + S * B_DIGIT_BYTES + ks * 256) >> 4);
+              umma_f16(dset + (uint32_t)(S * TNS), ad, bd, idesc[0], (fresh && ks == 0) ? 0u : 1u);
+            };
+            // The tensor core takes four instructions ahead: with the long
+            // products last they outlast the commit and the wait for the next
+            // stage (a stage's products run in 0.91 of the time of t = 0..S-1
+            // twice, at S = 6 with nothing else on the SM).
 #pragma unroll
-            for (int ks = 0; ks < TKS / 16; ++ks) {
-#pragma unroll
-              for (int t = 0; t < S; ++t) {
-                const uint64_t ad = dst0 + (uint64_t)((t * A_DIGIT_BYTES + ks * 256) >> 4);
-                const uint64_t bd = dst0 + (uint64_t)((A_BYTES + ks * 256) >> 4);
-                const uint32_t acc = (fresh && ks == 0 && t == 0) ? 0u : 1u;
-                umma_f16(dset + (uint32_t)(t * TNS), ad, bd, idesc[S - 1 - t], acc);
-              }
-              if constexpr (HP) {
-                const uint64_t ad = dst0 + (uint64_t)((S * A_DIGIT_BYTES + ks * 256) >> 4);
-                const uint64_t bd = dst0 + (uint64_t)((A_BYTES + S * B_DIGIT_BYTES + ks * 256) >> 4);
-                umma_f16(dset + (uint32_t)(S * TNS), ad, bd, idesc[0], (fresh && ks == 0) ? 0u : 1u);
-              }
+            for (int t = 0; t < S; ++t) digit(t, 0);
+            if constexpr (HP) {
+              magnitude(0);
+              magnitude(1);
             }
+#pragma unroll
+            for (int t = S - 1; t >= 0; --t) digit(t, 1);
             fresh = false;
             umma_commit(&empty[st]);
             if (++st == nstages) {
