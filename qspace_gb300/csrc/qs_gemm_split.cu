@@ -1,7 +1,7 @@
 // Split-precision grouped block GEMM on the sm_103a tensor cores.
 //
 // Method (error-free digit slicing in the spirit of Ozaki, Ogita, Oishi and
-// Rump, Numer. Algorithms 59 (2012), adapted to BF16 operands with exact FP32
+// Rump, Numer. Algorithms 59 (2012), adapted to FP16 operands with exact FP32
 // accumulation):
 //
 //  * Every output block gets one power-of-two scale per row of op(A) and per
@@ -11,7 +11,7 @@
 //  * Each scaled FP64 entry is rounded to the integer N = round(x 2^(bS-E))
 //    and cut into S balanced signed digits of b bits,
 //    N = sum_t d_t 2^(b(S-1-t)), |d_0| <= 2^b, |d_t| <= 2^(b-1).
-//    The digits are small integers, exact in BF16.  The cut uses integer
+//    The digits are small integers, exact in FP16.  The cut uses integer
 //    operations on the FP64 bit pattern only (GB300's FP64 pipe is narrow).
 //  * The product of the two digit expansions is
 //      sum_k x_ik y_kj = 2^(E_i+F_j-2b) sum_g 2^(-bg) acc_g,
@@ -199,7 +199,7 @@ __device__ __forceinline__ long long scaled_int(double x, int E, int bS, const F
 // With H = sum_{t>=1} 2^(B-1) 2^(B(S-1-t)), the low B(S-1) bits of M = N + H
 // are the base-2^B digits d_t + 2^(B-1), and d_0 = floor(M / 2^(B(S-1))).
 // Each digit is a funnel shift, one logic op (mask | 2^23 exponent) and one
-// FP32 subtraction; all values are exact in BF16 (at most 8 significant bits).
+// FP32 subtraction; all values are exact in FP16 (at most 9 significant bits).
 template <int S, int B>
 __device__ __forceinline__ void digits_f(long long N, float (&d)[S]) {
   constexpr long long HALF = 1LL << (B - 1);
@@ -839,19 +839,18 @@ __device__ __forceinline__ unsigned long long mad_wide(int a, int m, unsigned lo
 // acc / 2^-sh rounded.  All words wrap; V itself fits in int64, so
 // V = hi * 2^32 + lo (mod 2^64) is exact.
 
-// V * 2^scale: one int64 -> FP64 conversion (round to nearest even) and an
-// exponent add.  Integer-only assemblies (64-bit or 32-bit words, exactly
-// rounded, measured on GB300) made the launch slower: on short tiles the
-// epilogue is the bottleneck and its cost follows its instruction count.
-__device__ __forceinline__ double fixed_to_double(long long V, int scale) {
-  if (V == 0) return 0.0;
+// V * 2^scale by one int64 -> FP64 conversion (round to nearest even) and an
+// exponent add; `rare` is raised where that does not hold (the result is no
+// normal number) and fixed_to_double_rare has to be taken.  No branch: a
+// thread's eight outputs overlap (one after the other, each with its own
+// branches and its own reads of the tile's descriptor, took 4400 clocks a tile).
+__device__ __forceinline__ double fixed_to_double(long long V, int scale, bool &rare) {
   const double d = __ll2double_rn(V);
-  const long long bits = __double_as_longlong(d);
-  const int e = (int)((bits >> 52) & 0x7ff) + scale;
-  if (e <= 0 || e >= 2047) return ldexp(d, scale);
-  return __longlong_as_double(bits + ((long long)scale << 52));
+  const int hi = __double2hiint(d), e = (hi >> 20 & 0x7ff) + scale;
+  rare |= V != 0 && (unsigned)(e - 1) >= 2046u;
+  return __hiloint2double(V != 0 ? hi + (int)((unsigned)scale << 20) : 0, __double2loint(d));
 }
-
+__device__ __noinline__ double fixed_to_double_rare(long long V, int scale) { return ldexp(__ll2double_rn(V), scale); }
 // Folds accumulator groups G0..G0+NG-1 of one set (this thread's TMEM lane,
 // 8 columns from cbase) into the fixed-point words: group g enters with shift
 // sh = b(S-1-g) - rsh, >= 32 into the high word Vh, 0..30 into the low word
@@ -935,7 +934,9 @@ __device__ __forceinline__ double wide_to_double(long long Vh, long long Vl, int
   const int k = min(max(room, 0), lb);
   long long V = (long long)((unsigned long long)T << k) | (long long)(rem >> (lb - k));
   if (rem & ((1ull << (lb - k)) - 1)) V |= 1;                // sticky
-  return fixed_to_double(V, scale + lb - k);
+  bool rare = false;
+  const double d = fixed_to_double(V, scale + lb - k, rare);
+  return rare ? fixed_to_double_rare(V, scale + lb - k) : d;
 }
 
 // Chunking rule shared by the host and the MMA issuer: a new chunk starts
@@ -1175,12 +1176,12 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
       tw = (ti < ntiles && lane < TILE_WORDS) ? reinterpret_cast<const uint32_t *>(tiles + ti)[lane] : 0u;
       const int i_glob = T.mt * TMS + q * 32 + lane;
       const bool rv = i_glob < T.Mr;
-      // the row exponent is fetched now so that its load latency hides behind
-      // the accumulation; the column exponents (broadcast loads) are read at
-      // the stores, which keeps the drain's registers below the 96 a thread
-      // of this launch has
+      // the row's exponent and, one per lane, those of the warp's columns are
+      // fetched now, so that their latency hides behind the accumulation
       const int j0 = T.nt * TNS + cbase;
       const int Ei = rv ? E[T.eoff + i_glob] : 0;
+      int Fl = 0;
+      if constexpr (!HP) Fl = lane < CW && j0 + lane < T.N ? F[T.foff + j0 + lane] : 0;
       const int rsh = T.rshift;
       unsigned long long Vl[CW];
       std::conditional_t<HP, unsigned long long, unsigned int> Vh[CW];
@@ -1215,31 +1216,52 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
         if (lane == 0) mbar_arrive(&acc_empty[u & 1]);
       }
       if (!ok) break;
-      if (rv) {
-        const int rsplit = T.splits & 1, csplit = (T.splits >> 1) & 1;
+      if constexpr (HP) {
+        if (rv) {
+          const int rsplit = T.splits & 1, csplit = (T.splits >> 1) & 1;
+          double *crow = C + T.c_off + (int64_t)(i_glob >> rsplit) * T.rs + (i_glob & rsplit);
+#pragma unroll
+          for (int jj = 0; jj < CW; ++jj) {
+            const int j = j0 + jj;
+            if (j >= T.N) continue;
+            const int Fj = F[T.foff + j];
+            crow[(int64_t)(j >> csplit) * T.ldc + (j & csplit)] =
+                wide_to_double((long long)Vh[jj], (long long)Vl[jj], b * (S - HG), Ei + Fj + scale_b);
+            // a row or column of zeros (EMPTY_EXP) is exact
+            if (max(Ei, Fj) >= NONFINITE_EXP || (min(Ei, Fj) > EMPTY_EXP && cert[jj] < CERT_MIN)) {
+              const int rdup = (T.splits >> 3) & 1, cdup = (T.splits >> 4) & 1;
+              const int lr = i_glob >> rdup, lc = j >> cdup;
+              const bool sw = T.splits & 4;
+              const int rows = sw ? T.N >> cdup : T.Mr >> rdup;  // of C
+              flags[T.fbase + (sw ? lc : lr) / F64_TILE +
+                    (sw ? lr : lc) / F64_TILE * ((rows + F64_TILE - 1) / F64_TILE)] = 1;
+            }
+          }
+        }
+      } else {
+        // the eight outputs side by side, then their stores (1024 x 1024 blocks
+        // of depth 128: 508 -> 422 us)
+        double v[CW];
+        bool rare = false;
+        const int sc0 = Ei + scale_b + rsh;
+#pragma unroll
+        for (int jj = 0; jj < CW; ++jj) {
+          const int Fj = __shfl_sync(0xffffffffu, Fl, jj);
+          v[jj] = fixed_to_double((long long)(((unsigned long long)Vh[jj] << 32) + Vl[jj]), sc0 + Fj, rare);
+        }
+        const int splits = T.splits, rsplit = splits & 1, csplit = (splits >> 1) & 1, N = T.N;
+        const int64_t ldc = T.ldc;
         double *crow = C + T.c_off + (int64_t)(i_glob >> rsplit) * T.rs + (i_glob & rsplit);
+        if (rare) {
+#pragma unroll
+          for (int jj = 0; jj < CW; ++jj)
+            v[jj] = fixed_to_double_rare((long long)(((unsigned long long)Vh[jj] << 32) + Vl[jj]),
+                                         sc0 + F[T.foff + min(j0 + jj, N - 1)]);
+        }
 #pragma unroll
         for (int jj = 0; jj < CW; ++jj) {
           const int j = j0 + jj;
-          if (j < T.N) {
-            double *out = crow + (int64_t)(j >> csplit) * T.ldc + (j & csplit);
-            if constexpr (HP) {
-              const int Fj = F[T.foff + j];
-              *out = wide_to_double((long long)Vh[jj], (long long)Vl[jj], b * (S - HG), Ei + Fj + scale_b);
-              // a row or column of zeros (EMPTY_EXP) is exact
-              if (max(Ei, Fj) >= NONFINITE_EXP || (min(Ei, Fj) > EMPTY_EXP && cert[jj] < CERT_MIN)) {
-                const int rdup = (T.splits >> 3) & 1, cdup = (T.splits >> 4) & 1;
-                const int lr = i_glob >> rdup, lc = j >> cdup;
-                const bool sw = T.splits & 4;
-                const int rows = sw ? T.N >> cdup : T.Mr >> rdup;  // of C
-                flags[T.fbase + (sw ? lc : lr) / F64_TILE +
-                      (sw ? lr : lc) / F64_TILE * ((rows + F64_TILE - 1) / F64_TILE)] = 1;
-              }
-            } else {
-              const long long V = (long long)(((unsigned long long)Vh[jj] << 32) + Vl[jj]);
-              *out = fixed_to_double(V, Ei + F[T.foff + j] + rsh + scale_b);
-            }
-          }
+          if (rv && j < N) crow[(j >> csplit) * ldc + (j & csplit)] = v[jj];
         }
       }
     }
