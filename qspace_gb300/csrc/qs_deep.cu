@@ -256,9 +256,10 @@ struct DotTask {
 };
 constexpr int DOT_THREADS = 256;
 constexpr int DOT_U = 4;
+constexpr int DOT_SELF_U = 8;
 
 template <bool CPLX>
-__global__ void __launch_bounds__(DOT_THREADS)
+__global__ void __launch_bounds__(DOT_THREADS, 4)
 dot_kernel(const DotTask *__restrict__ tasks, const PairDesc *__restrict__ pairs, const double *__restrict__ A,
            const double *__restrict__ B, double *__restrict__ C) {
   __shared__ double red[2][DOT_THREADS];
@@ -271,6 +272,35 @@ dot_kernel(const DotTask *__restrict__ tasks, const PairDesc *__restrict__ pairs
     const bool ta = P.trans & 1, tb = P.trans & 2, ca = P.trans & 4, cb = P.trans & 8;
     const int64_t a0 = P.a_off + (ta ? t.i * (int64_t)P.lda : t.i), as = ta ? 1 : P.lda;
     const int64_t b0 = P.b_off + (tb ? t.j : t.j * (int64_t)P.ldb), bs = tb ? P.ldb : 1;
+    // An operand against its own conjugate (a norm, a diagonal entry of a
+    // density matrix): two multiply-adds per term and one load instead of four
+    // and two; the imaginary part is zero.  The four bound the kernel (GB300's
+    // FP64 pipe does two per clock and SM; a site density matrix of bond 8192,
+    // 5 10^6 terms: 209 -> 171 us for the call).  Sums that leave the finite
+    // numbers take the general form below.
+    if (CPLX && A + 2 * a0 == B + 2 * b0 && as == bs && ca != cb) {
+      double s[DOT_SELF_U];
+#pragma unroll
+      for (int u = 0; u < DOT_SELF_U; ++u) s[u] = 0.0;
+      for (int64_t k = threadIdx.x; k < P.K; k += DOT_SELF_U * DOT_THREADS) {
+        double2 a[DOT_SELF_U];
+#pragma unroll
+        for (int u = 0; u < DOT_SELF_U; ++u) {
+          const int64_t kk = k + u * DOT_THREADS, ia = a0 + kk * as;
+          a[u] = make_double2(0.0, 0.0);
+          if (kk < P.K)
+            a[u] = wide ? reinterpret_cast<const double2 *>(A)[ia] : make_double2(A[2 * ia], A[2 * ia + 1]);
+        }
+#pragma unroll
+        for (int u = 0; u < DOT_SELF_U; ++u) s[u] = fma(a[u].x, a[u].x, fma(a[u].y, a[u].y, s[u]));
+      }
+#pragma unroll
+      for (int u = 1; u < DOT_SELF_U; ++u) s[0] += s[u];
+      if (isfinite(s[0])) {
+        re += P.afac * s[0];
+        continue;
+      }
+    }
     // DOT_U terms in flight per thread, each with its own running sum
     double sr[DOT_U], si[DOT_U];
 #pragma unroll
