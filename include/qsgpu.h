@@ -59,7 +59,7 @@ typedef enum {
 
 typedef enum {
   QS_PREC_FP64 = 0,   /* plain FP64 (DFMA) path: the drop-in                   */
-  QS_PREC_SPLIT = 1   /* FP64 sliced into BF16 digits, tcgen05 products with
+  QS_PREC_SPLIT = 1   /* FP64 sliced into FP16 digits, tcgen05 products with
                          exact FP32 accumulation, compensated recombination   */
 } qs_prec;
 
@@ -86,7 +86,7 @@ typedef struct {
 
 typedef struct {
   int32_t prec;       /* qs_prec                                               */
-  int32_t nslices;    /* split path: BF16 digits per operand; 0 = automatic     */
+  int32_t nslices;    /* split path: FP16 digits per operand; 0 = automatic     */
   double tol;         /* split path: target relative error (default 1e-12)     */
   int32_t flags;      /* QS_FLAG_*                                              */
 } qs_opts;
@@ -309,7 +309,7 @@ QS_EXPORT void qs_grouped_plan_destroy(qs_grouped_plan *plan);
  * device.  It allocates no device memory: no cudaMalloc/cudaMallocAsync/
  * cudaFree, no memory pool, no library workspace (its host-side planning uses
  * ordinary host memory).  Its device scratch (work lists,
- * exponents, BF16 digits) is one file-scope array of
+ * exponents, FP16 digits) is one file-scope array of
  * QS_STATIC_SCRATCH_BYTES per device and process; a pair list that needs
  * more is refused with QS_ERR_OOM before anything is launched.
  *  - The first call on each device looks the array up (cudaGetSymbolAddress)

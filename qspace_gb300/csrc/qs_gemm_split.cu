@@ -374,7 +374,11 @@ __device__ __forceinline__ OpAddr addr_b(const SplitPair &P, const OperandView *
 // in the B-duplicated form row m of op(A) is one row of A' ((Re, Im) along
 // k) and column n of op(B) the columns 2n, 2n+1 of B' ((Re; -Im), (Im; Re)).
 constexpr int STRIP = 16;          // real lines per strip (two core-matrix groups)
-constexpr int STRIP_THREADS = 128;
+// 256 threads, five CTAs an SM: the last wave of deep strips is shorter than with
+// 128 threads and ten CTAs (480 real products 176 -> 169 us, 300 complex FP64
+// products 1150 -> 1138 us, the 2000-product batch the same); 512 threads leave
+// too few strips in flight (4.54 -> 4.98 ms)
+constexpr int STRIP_THREADS = 256;
 
 // Phase 1 for the lines l0 .. l0+nl-1 of op(X) (X = A role: rows, line m at
 // m + k*ld (contig: k + m*ld); X = B role: columns, line n at k + n*ld
@@ -670,7 +674,7 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
 // VIEWS = false: no pair of the launch reads its operand through a view, and
 // the view addressing is compiled out
 template <bool CPLX, int S, bool VIEWS, bool HP>
-__global__ void __launch_bounds__(STRIP_THREADS)
+__global__ void __launch_bounds__(STRIP_THREADS, 5)
 strip_a_kernel(const SplitPair *__restrict__ pairs, const OperandView *__restrict__ views_in,
                const int4 *__restrict__ tasks, const double *__restrict__ A, const double *__restrict__ B,
                int *__restrict__ E, uint8_t *__restrict__ arena, int b) {
@@ -691,7 +695,7 @@ strip_a_kernel(const SplitPair *__restrict__ pairs, const OperandView *__restric
 // VIEWS = false: no pair of the launch reads its operand through a view, and
 // the view addressing is compiled out
 template <bool CPLX, int S, bool VIEWS, bool HP>
-__global__ void __launch_bounds__(STRIP_THREADS)
+__global__ void __launch_bounds__(STRIP_THREADS, 5)
 strip_b_kernel(const SplitPair *__restrict__ pairs, const OperandView *__restrict__ views_in,
                const int4 *__restrict__ tasks, const double *__restrict__ A, const double *__restrict__ B,
                int *__restrict__ F, uint8_t *__restrict__ arena, int b) {
@@ -1944,7 +1948,7 @@ SplitResult run_split_static(Ctx *ctx, const std::vector<PairDesc> &pairs, const
   const size_t o_arena = take((size_t)w.arena);
   if (used > cap)
     fail(QS_ERR_OOM, "split (static scratch): this pair list needs %zu bytes of scratch (%lld of them "
-         "BF16 digits), more than the %zu available", used, (long long)w.arena, cap);
+         "FP16 digits), more than the %zu available", used, (long long)w.arena, cap);
   SplitDev d;
   d.pairs = reinterpret_cast<SplitPair *>(scratch + o_pairs);
   d.sa = reinterpret_cast<int4 *>(scratch + o_sa);

@@ -1,4 +1,4 @@
-// Split-precision grouped block GEMM (FP64 emulated with BF16 digits on the
+// Split-precision grouped block GEMM (FP64 emulated with FP16 digits on the
 // 5th-generation tensor cores).  See qs_gemm_split.cu for the method.
 #pragma once
 

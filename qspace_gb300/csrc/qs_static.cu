@@ -1,6 +1,6 @@
 // qs_grouped_gemm_split_static: the split-precision grouped GEMM for callers
 // that must not allocate device memory while they run.  Every device buffer
-// of the call -- work lists, exponent arrays, BF16 digit arena, error word --
+// of the call -- work lists, exponent arrays, FP16 digit arena, error word --
 // lives in one file-scope array per device and process; nothing is allocated.
 #include <mutex>
 
