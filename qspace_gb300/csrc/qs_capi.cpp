@@ -450,8 +450,7 @@ static void prepare(Ctx *ctx, Prepared &w, const QMeta &Am, const double *dA, co
   bool all_direct = true;
   for (size_t b = 0; b + 1 < pl.grp.size() && all_direct; ++b)
     all_direct = is_shallow(pl.pairs, pl.grp[b], pl.grp[b + 1]) &&
-                 (split ? shallow_direct_wins(pl.pairs, pl.grp[b], pl.grp[b + 1], pl.blk_M[b], pl.blk_N[b], cplx)
-                        : f64_direct(pl.pairs, pl.grp[b], pl.grp[b + 1], pl.blk_M[b], pl.blk_N[b], cplx));
+                 (!split || shallow_direct_wins(pl.pairs, pl.grp[b], pl.grp[b + 1], pl.blk_M[b], pl.blk_N[b], cplx));
   const bool views = (split || all_direct) && !has_deep_blocks(pl.pairs, pl.grp, pl.blk_M, pl.blk_N);
   // the views' offset tables, one pair of tables per operand block (every
   // pair reading the block shares them): all in one upload

@@ -1838,21 +1838,24 @@ SplitResult run_split(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::v
     }
   if (!shallow_ids.empty()) {
     const DigitPlan dp = choose_digits_for(pairs, grp, blk_M, blk_N, cplx ? 2 : 1, tol, forced_slices, forced_bits);
-    run_shallow(ctx, pairs, grp, blk_M, blk_N, c_off, blk_ldc, shallow_ids, A, B, C, cplx, va, vb);
     SplitResult res;
-    res.nslices = dp.nslices;
-    res.bits = dp.bits;
-    res.err_bound = dp.err_bound;
-    if (shallow_ids.size() == nb) return res;
-    const BlockList R = select_blocks(pairs, grp, blk_M, blk_N, c_off, blk_ldc, rest);
-    std::vector<OperandView> va2, vb2;
-    for (int32_t q : R.src) {
-      if (va) va2.push_back((*va)[q]);
-      if (vb) vb2.push_back((*vb)[q]);
+    if (shallow_ids.size() < nb) {
+      const BlockList R = select_blocks(pairs, grp, blk_M, blk_N, c_off, blk_ldc, rest);
+      std::vector<OperandView> va2, vb2;
+      for (int32_t q : R.src) {
+        if (va) va2.push_back((*va)[q]);
+        if (vb) vb2.push_back((*vb)[q]);
+      }
+      res = run_split(ctx, R.pairs, R.grp, R.bM, R.bN, R.coff, A, B, C, cplx, dp.nslices, tol, &R.bldc, dp.bits,
+                      va ? &va2 : nullptr, vb ? &vb2 : nullptr);
     }
-    SplitResult r2 = run_split(ctx, R.pairs, R.grp, R.bM, R.bN, R.coff, A, B, C, cplx, dp.nslices, tol, &R.bldc,
-                               dp.bits, va ? &va2 : nullptr, vb ? &vb2 : nullptr);
-    return r2.nslices ? r2 : res;
+    run_shallow(ctx, pairs, grp, blk_M, blk_N, c_off, blk_ldc, shallow_ids, A, B, C, cplx, va, vb);
+    if (!res.nslices) {
+      res.nslices = dp.nslices;
+      res.bits = dp.bits;
+      res.err_bound = dp.err_bound;
+    }
+    return res;
   }
   DeepSplit ds;
   if (reinterpret_cast<uintptr_t>(C) % eb == 0 &&
@@ -1879,6 +1882,7 @@ SplitResult run_split(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::v
           sel[g] = 0;
           small.push_back((int64_t)g);
         }
+      if (small.size() < ds.bM.size()) require_whole_elements(A, B, nullptr, cplx);
       run_dot(ctx, ds.pairs, ds.grp, ds.bM, ds.bN, ds.coff, &ds.bldc, small, A, B, C, cplx);
       SplitResult res;
       res.nslices = dp.nslices;
@@ -1919,6 +1923,7 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
   SplitResult res = plan_split(pairs, grp, blk_M, blk_N, c_off, cplx, forced_slices, tol, blk_ldc, w, forced_bits,
                                va, vb);
   if (w.tiles.empty()) return res;
+  require_whole_elements(A, B, nullptr, cplx);  // the products' stores are single doubles
   // the digit arena is pooled scratch
   SplitDev d;
   d.arena = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)std::max<int64_t>(w.arena, 256)));
@@ -1935,6 +1940,7 @@ SplitResult run_split_static(Ctx *ctx, const std::vector<PairDesc> &pairs, const
   SplitWork w;
   SplitResult res = plan_split(pairs, grp, blk_M, blk_N, c_off, cplx, forced_slices, tol, blk_ldc, w);
   if (w.tiles.empty()) return res;
+  require_whole_elements(A, B, nullptr, cplx);
   size_t used = 0;
   auto take = [&](size_t bytes) {
     const size_t o = used;
@@ -2021,11 +2027,6 @@ static bool f64_tensor_takes(const std::vector<PairDesc> &pairs, int64_t p0, int
   // either operand's real form may be the duplicated one
   bytes = (up(M * cm, TMS) + up(N * cm, TMS)) * kpad * (HP_DIGITS + 1) * 2;
   return bytes <= F64T_BLOCK_BYTES;
-}
-
-bool f64_direct(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int32_t M, int32_t N, bool cplx) {
-  int64_t bytes = 0;
-  return !f64_tensor_takes(pairs, p0, p1, M, N, cplx, bytes) || shallow_direct_wins(pairs, p0, p1, M, N, cplx);
 }
 
 F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,

@@ -102,19 +102,19 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
   std::vector<char> rest(bM.size(), 1);
   std::vector<int64_t> ids;
   for (size_t b = 0; b < bM.size(); ++b)
-    if (is_shallow(pairs, grp[b], grp[b + 1]) &&
-        f64_direct(pairs, grp[b], grp[b + 1], bM[b], bN[b], cplx)) {
+    if (is_shallow(pairs, grp[b], grp[b + 1])) {
       rest[b] = 0;
       ids.push_back((int64_t)b);
     }
   if (!ids.empty()) {
+    if (ids.size() < bM.size()) {
+      const BlockList R = select_blocks(pairs, grp, bM, bN, coff, bldc, rest);
+      for (int32_t q : R.src)
+        if ((va && (*va)[q].nl > 0) || (vb && (*vb)[q].nl > 0))
+          fail(QS_ERR_INTERNAL, "FP64 tiles of an operand read through a view");
+      run_f64(ctx, R.pairs, R.grp, R.bM, R.bN, R.coff, &R.bldc, A, B, C, cplx);
+    }
     run_shallow(ctx, pairs, grp, bM, bN, coff, bldc, ids, A, B, C, cplx, va, vb);
-    if (ids.size() == bM.size()) return;
-    const BlockList R = select_blocks(pairs, grp, bM, bN, coff, bldc, rest);
-    for (int32_t q : R.src)
-      if ((va && (*va)[q].nl > 0) || (vb && (*vb)[q].nl > 0))
-        fail(QS_ERR_INTERNAL, "FP64 tiles of an operand read through a view");
-    run_f64(ctx, R.pairs, R.grp, R.bM, R.bN, R.coff, &R.bldc, A, B, C, cplx);
     return;
   }
   DeepSplit ds;
@@ -142,6 +142,7 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
         skip[b] = 1;
         small.push_back((int64_t)b);
       }
+    if (small.size() < mm.size()) require_whole_elements(A, B, C, cplx);
     run_dot(ctx, pp, gg, mm, nn, cc, ll, small, A, B, C, cplx);
     const F64TensorList tl = plan_f64_tensor(pp, gg, mm, nn, cc, ll, cplx, skip);
     const std::vector<char> dots = skip;

@@ -304,6 +304,17 @@ bool ctx_alive(const Ctx *c);
 // qs_linalg.cu
 void destroy_solver(Ctx *ctx);
 
+// The tiled kernels move whole complex values (16 bytes at a time): buffers
+// at an odd multiple of 8 bytes are refused on the host, before a launch (a
+// misaligned access would end the context).  The direct kernels of shallow
+// blocks and of few-output deep sums take any 8-byte alignment.  C may be null.
+inline void require_whole_elements(const double *A, const double *B, const double *C, bool cplx) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C);
+  if (cplx && all % 16)
+    fail(QS_ERR_ARG, "complex buffers of blocks summed over more than %lld terms must be aligned to 16 bytes",
+         (long long)SHALLOW_K);
+}
+
 // ------------------------------------------------------ small utilities
 template <class T>
 T *dev_alloc(Ctx *ctx, size_t n) {

@@ -75,6 +75,8 @@ struct qs_grouped_plan {
 namespace {
 
 void launch_direct(qs_grouped_plan *p, const double *A, const double *B, double *C) {
+  if (!p->main.pairs.empty())
+    require_whole_elements(A, B, p->o.prec == QS_PREC_SPLIT ? nullptr : C, p->g.cplx);
   shallow_launch(p->ctx, p->shallow, A, B, C);
   if (p->main.pairs.empty()) return;
   if (p->o.prec == QS_PREC_SPLIT)
@@ -108,8 +110,7 @@ void split_shallow(qs_grouped_plan *p) {
   const bool split = p->o.prec == QS_PREC_SPLIT;
   for (size_t b = 0; b < g.bM.size(); ++b)
     if (is_shallow(g.pairs, g.grp[b], g.grp[b + 1]) &&
-        (split ? shallow_direct_wins(g.pairs, g.grp[b], g.grp[b + 1], g.bM[b], g.bN[b], g.cplx)
-               : f64_direct(g.pairs, g.grp[b], g.grp[b + 1], g.bM[b], g.bN[b], g.cplx))) {
+        (!split || shallow_direct_wins(g.pairs, g.grp[b], g.grp[b + 1], g.bM[b], g.bN[b], g.cplx))) {
       rest[b] = 0;
       ids.push_back((int64_t)b);
     }

@@ -67,14 +67,13 @@ struct F64TensorList {
   int64_t nflags = 0;
 };
 // The blocks of a list that the tensor-core launch takes (a property of the
-// block alone), except those marked in `skip`.
+// block alone), except those marked in `skip`.  The list holds no shallow
+// blocks: the FP64 path computes all of them directly (run_shallow), which
+// takes complex buffers aligned to 8 bytes.
 F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                               const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                               const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
                               const std::vector<char> &skip);
-// Whether the FP64 path computes a shallow block directly (run_shallow): it
-// does unless the tensor-core launch takes the block and is estimated faster.
-bool f64_direct(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int32_t M, int32_t N, bool cplx);
 // Runs them (strips and products); false when the device has no room for
 // their digits (nothing ran: the caller computes every tile in FP64).
 bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,

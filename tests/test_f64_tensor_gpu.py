@@ -8,6 +8,7 @@ the certificate are recomputed by the FP64 kernel and meet the same bound."""
 import numpy as np
 import pytest
 
+from qspace_gb300._capi import QSError
 from qspace_gb300.grouped import DeviceBatch, Packed
 
 U = 2.0 ** -53
@@ -230,3 +231,59 @@ def test_shallow_complex_alignment(shift):
     t.cuda.synchronize()
     db.run("fp64")
     _check(db.result(), want)
+
+
+def _shifted(db, shift):
+    t = db.torch
+    pad = lambda x: t.cat([t.zeros(shift, dtype=t.float64, device=x.device), x])[shift:]  # noqa: E731
+    db.dA, db.dB, db.dC = pad(db.dA), pad(db.dB), pad(db.dC)
+    t.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(64, 32, 8), (64, 64, 8), (256, 256, 8), (90, 130, 5), (33, 200, 6)])
+def test_large_shallow_blocks_take_any_alignment(shape):
+    """A block summed over at most 8 terms is computed directly on the FP64
+    path whatever its size: with the bits of the aligned call, from buffers at
+    an odd multiple of eight bytes too, alone, with others and from a plan."""
+    M, N, K = shape
+    rng = np.random.default_rng(7)
+    ops, afac, blk, trans = [_ops(rng, M, N, K, True), _ops(rng, 3, 5, 2, True)], [-0.7, 1.0], [0, 1], [5, 10]
+    db = _batch(ops, afac, blk, trans)
+    db.run("fp64")
+    want = [c.copy() for c in db.result()]
+    _check(want, _reference(ops, afac, blk))
+    _shifted(db, 1)
+    db.run("fp64")
+    for c, w in zip(db.result(), want):
+        assert np.array_equal(c, w)
+    plan = db.plan("fp64")
+    db.dC.fill_(float("nan"))
+    db.torch.cuda.synchronize()
+    db.run_plan(plan)
+    for c, w in zip(db.result(), want):
+        assert np.array_equal(c, w)
+    plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["fp64", "split"])
+def test_deeper_misaligned_blocks_are_refused_on_the_host(prec):
+    """Tiles move whole complex values: buffers that are not aligned to them
+    are an error, raised before anything is launched."""
+    rng = np.random.default_rng(8)
+    ops = [_ops(rng, 40, 40, 48, True), _ops(rng, 4, 6, 2, True)]
+    db = _batch(ops, [1.0, 1.0], [0, 1], [0, 0])
+    _shifted(db, 1)
+    db.dC.fill_(7.0)
+    db.torch.cuda.synchronize()
+    n0 = db.ctx.launches
+    with pytest.raises(QSError, match="aligned to 16"):
+        db.run(prec)
+    plan = db.plan(prec)
+    with pytest.raises(QSError, match="aligned to 16"):
+        db.run_plan(plan)
+    plan.close()
+    assert db.ctx.launches == n0
+    db.ctx.sync()
+    assert bool((db.dC == 7.0).all())
