@@ -296,6 +296,15 @@ __device__ __forceinline__ void digit_planes(unsigned long long w0, unsigned lon
   }
 }
 
+// max(|d_0| - 1/2, 0) of two leading digits (exact in FP16): d_0 is rounded, so
+// this, not |d_0|, stays below the entry's own magnitude (up to 0.4 %: the
+// other digits reach 128/255 of a unit, not a half).
+__device__ __forceinline__ uint32_t lower_magnitudes(uint32_t w) {
+  const uint32_t a = w & 0x7FFF7FFFu;
+  const __half2 m = __hmax2(__hsub2(*reinterpret_cast<const __half2 *>(&a), __float2half2_rn(0.5f)), __float2half2_rn(0.0f));
+  return *reinterpret_cast<const uint32_t *>(&m);
+}
+
 // L2 eviction priorities of the strip kernels (createpolicy, PTX ISA 7.4+):
 // the first read of an operand line is kept (evict_last) for the re-read of
 // phase 2, which is its last use (evict_first), and the digit stores stream
@@ -501,7 +510,7 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
                              fixed_word<S, B>(ca ? -a[j].y : a[j].y, Ei, ls, Fa), w2);
 #pragma unroll
           for (int t = 0; t < S; ++t) pw[t][j] = w2[t];
-          if constexpr (HP) pw[S][j] = w2[0] & 0x7FFF7FFFu;
+          if constexpr (HP) pw[S][j] = lower_magnitudes(w2[0]);
         }
         const int rr0 = rl + 2 * ml, rr1 = rr0 + 1;
         uint8_t *tile = tiles + (int64_t)kb * NP * A_DIGIT_BYTES;
@@ -565,7 +574,7 @@ __device__ __forceinline__ void strip_a(const SplitPair *__restrict__ pairs, con
         }
         if constexpr (HP) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) pk[S][j] = pk[0][j] & 0x7FFF7FFFu;
+          for (int j = 0; j < 4; ++j) pk[S][j] = lower_magnitudes(pk[0][j]);
         }
         const int rr = rl + rloc;
         uint8_t *dst = tiles + (int64_t)kb * NP * A_DIGIT_BYTES + ((rr >> 3) * KCM + q) * 128 + (rr & 7) * 16;
@@ -661,7 +670,7 @@ __device__ __forceinline__ void strip_b(const SplitPair *__restrict__ pairs, con
       }
       if constexpr (HP) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) pk[S][j] = pk[0][j] & 0x7FFF7FFFu;
+        for (int j = 0; j < 4; ++j) pk[S][j] = lower_magnitudes(pk[0][j]);
       }
       uint8_t *dst = tiles + (int64_t)kb * NP * B_DIGIT_BYTES + ((c >> 3) * KCM + q) * 128 + (c & 7) * 16;
 #pragma unroll
@@ -887,15 +896,20 @@ __device__ __forceinline__ void fold_groups(uint32_t set_base, int cbase, int b,
   }
 }
 
-// Smallest certificate of an output: sum_k |d_0(ik)| |d_0(kj)| in units of
-// 2^(E_i+F_j-2b), where 2^(2b) is the product of two full-scale entries.  The
-// truncations -- 2^-57 of full scale per operand entry and at most 6 2^-58 for
-// the digit products left out -- are below K 2^(E_i+F_j) 2^-54.9, so a sum of
-// at least full scale / 16 keeps them within 4.3 K u sum_k |a_ik b_kj|
-// (u = 2^-53; an FP64 dot product is bounded by K u of the same sum).
-// Normally distributed entries pass from nine terms on: 4e-6 of the outputs
-// miss it at nine terms, none of 10^7 at sixteen.
-constexpr float CERT_MIN = 65536.0f / 16.0f;
+// Smallest certificate of an output, sum_k m_ik m_kj in units of
+// 2^(E_i+F_j-16) with m = max(|d_0| - 1/2, 0) (lower_magnitudes).  It is a lower
+// bound of sum_k |a_ik b_kj| up to 0.8 % (m's 0.4 % twice; the FP32 sums add
+// 2^-10 at most).  What a term loses: 2^-57 of full scale per entry's rounding
+// and 6 2^-58 (a little more) for the digit products left out, together
+// 10.02 2^-58 2^(E_i+F_j).  A sum of at least a third of full scale keeps K terms
+// of that below 0.95 K u sum_k |a_ik b_kj|, u = 2^-53: the bound of an FP64 dot
+// product, K u of the same sum.  (The rounded magnitudes |d_0| with a sixteenth
+// of full scale had left 17 K u: |d_0| doubles an entry just above half a unit.)
+// Against sequential FP64 sums, root mean square error over outputs that pass,
+// in u sum |ab|: normal entries 0.16 to 0.47 at K = 32 and 0.03 to 0.48 at 1024;
+// log-normal (sigma 2) 0.37 to 1.3 at 32, 1.1 to 8.8 at 1024 (with a sixteenth:
+// 1.7 to 1.5 at 64, 16 to 9 at 4096); one dominant term 2.2 to 27 at 4096.
+constexpr float CERT_MIN = 65536.0f / 3.0f;
 
 // FP64-grade fold (S digits, two 64-bit words): the groups 0..HG-1 into Vh
 // with weights 2^(b(HG-1-g)), the others into Vl with 2^(b(S-1-g)), so that
@@ -958,9 +972,10 @@ __device__ __forceinline__ int kblock_depth(int Kr, int kb) { return min(TKS, Kr
 __device__ __forceinline__ int tile_of(int r, int c, int G) { return r * G + ((r & 1) ? (G - 1 - c) : c); }
 
 //
-// HP: the FP64-grade launch of the plain path (see split_f64_eligible): S
-// digits plus one plane of the leading digits' magnitudes per operand, whose
-// product (accumulator group S) bounds sum_k |a_ik b_kj| from below.  An
+// HP: the FP64-grade launch of the plain path (see f64_tensor_takes): S
+// digits plus one plane of the leading digits' magnitudes (lower_magnitudes)
+// per operand, whose product (accumulator group S) bounds sum_k |a_ik b_kj|
+// from below.  An
 // output whose bound is too small for the digits' truncation to stay at the
 // level of an FP64 sum, or whose row or column holds an infinity or NaN,
 // raises the flag of its FP64 tile, which the FP64 kernel then recomputes.
@@ -1995,14 +2010,16 @@ std::vector<int> split_candidate_bits(double tol, int forced_slices) {
 
 // ------------------------------------------- FP64-grade tensor-core products
 // Blocks the tensor-core launch takes: a summed real depth of at least
-// F64T_DEPTH (below it a sum of normally distributed terms often misses the
-// certificate) and at least F64T_WORK real multiply-adds, which take the
-// narrow FP64 pipe (about 2 multiply-adds per clock and SM) 9 us in one tile;
-// the three launches take about 25 us in sum whatever the block.  Measured, FP64 tiles against this path: 300
-// complex products of 8..1024 per side 23.1 -> 1.71 ms (15.6 TFLOP/s of FP64
-// work; error against a 64-bit product 1.2e-15 -> 6.7e-16), 64 real blocks of
+// F64T_DEPTH (below it nearly every tile of normally distributed operands holds
+// an output that misses the certificate: 99 % of the 32 x 32 tiles at depth 12,
+// 78 % at 16, 28 % at 20, 6 % at 24, 0.4 % at 32) and at least F64T_WORK real
+// multiply-adds, which take the narrow FP64 pipe (about 2 multiply-adds per
+// clock and SM) 9 us in one tile; the three launches take about 25 us in sum
+// whatever the block.  Measured, FP64 tiles against this path: 300 complex
+// products of 8..1024 per side 23.1 -> 1.71 ms (15.6 TFLOP/s of FP64 work;
+// error against a 64-bit product 1.2e-15 -> 6.7e-16), 64 real blocks of
 // 4..96 105 -> 77 us.
-constexpr int64_t F64T_DEPTH = 9, F64T_MAX_DEPTH = 1 << 20;
+constexpr int64_t F64T_DEPTH = 16, F64T_MAX_DEPTH = 1 << 20;
 constexpr double F64T_WORK = 32768.0;
 // Digit bytes of one launch (blocks above it get a launch of their own), and
 // of a block that still takes this path.

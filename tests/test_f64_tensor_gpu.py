@@ -287,3 +287,45 @@ def test_deeper_misaligned_blocks_are_refused_on_the_host(prec):
     assert db.ctx.launches == n0
     db.ctx.sync()
     assert bool((db.dC == 7.0).all())
+
+
+def _digits(d0, low):
+    """An entry below 1 whose 8-bit digits are d0 and then `low` six times."""
+    return d0 * 2.0 ** -8 + sum(low * 2.0 ** (-8 * t) for t in range(2, 8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K,d0,low", [(4103, 1, -128), (4103, 1, 127), (2050, 2, -128), (1030, 5, -128), (66, 20, -128),
+                                      (66, 19, -128), (66, 20, 127), (34, 28, -128), (34, 40, -128), (200, 12, -128)])
+@pytest.mark.parametrize("trans", [0, 3])
+def test_f64_tensor_bound_of_an_fp64_sum(K, d0, low, trans):
+    """Every digit product that is left out has the same sign, and the leading
+    digits overstate (or understate) the entries; one full-scale entry per line
+    faces a zero.  The bound is an FP64 dot product's own, n u sum |a_k b_k|, with
+    one rounding each for the factor and the result."""
+    M, N = 64, 40
+    a, b = np.full((M, K), _digits(d0, low)), np.full((K, N), _digits(d0, low))
+    a[:, 0], b[0, :] = 0.75, 0.0
+    a[:, 1], b[1, :] = 0.0, -0.875
+    ops, afac = [(a, b)], [1.0]
+    db = _batch(ops, afac, [0], [trans])
+    db.run("fp64")
+    (r, s, n), = _reference(ops, afac, [0])
+    err = np.abs(db.result()[0] - r).astype(float)
+    assert np.all(err <= n * U * s + 2 * U * np.abs(r).astype(float)), float(np.max(err / (n * U * s)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("K", [31, 32, 33, 64, 700])
+def test_f64_tensor_skewed_entries(K, cplx):
+    """Log-normal entries: many outputs are far below their lines' maxima."""
+    rng = np.random.default_rng(K)
+    a, b = _ops(rng, 70, 99, K, cplx)
+    a, b = a * np.exp(2 * rng.standard_normal(a.shape)), b * np.exp(2 * rng.standard_normal(b.shape))
+    db = _batch([(a, b)], [0.6], [0], [0])
+    db.run("fp64")
+    (r, s, n), = _reference([(a, b)], [0.6], [0])
+    d = db.result()[0] - r
+    err = np.maximum(np.abs(d.real), np.abs(d.imag)).astype(float)
+    assert np.all(err <= (n + 1) * U * s + 2 * U * np.abs(r).astype(float))
