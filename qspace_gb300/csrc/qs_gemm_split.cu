@@ -139,7 +139,8 @@ struct LineMax {
 };
 
 // A factor f (CG coefficient) as an exact integer mantissa and exponent,
-// f = fm * 2^fe; fm = 0 means "no factor" (f = 1); fe = -100000 means f = 0.
+// f = fm * 2^fe, 2^52 <= fm < 2^53; fm = 0 means "no factor" (f = 1); fe = -100000
+// means f = 0.
 struct Factor {
   unsigned long long fm;
   int fe;
@@ -154,8 +155,14 @@ __host__ __device__ inline Factor make_factor(double f) {
   memcpy(&bits, &f, 8);
   int be = (int)((bits >> 52) & 0x7ff);
   unsigned long long m = bits & 0xFFFFFFFFFFFFFull;
-  if (be == 0) be = 1; else m |= (1ull << 52);
-  r.fm = m ? m : 0ull;
+  if (be != 0) {
+    m |= 1ull << 52;
+  } else if (m) {
+    // a subnormal factor: normalised, since scaled_int keeps the upper bits of
+    // the product of the two mantissas
+    for (be = 1; !(m >> 52); --be) m <<= 1;
+  }
+  r.fm = m;
   r.fe = be - 1075;
   r.neg = (bits >> 63) != 0;
   if (!m) { r.fm = 0; r.fe = 0; r.neg = false; r.fe = -100000; }  // f == 0

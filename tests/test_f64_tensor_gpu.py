@@ -329,3 +329,24 @@ def test_f64_tensor_skewed_entries(K, cplx):
     d = db.result()[0] - r
     err = np.maximum(np.abs(d.real), np.abs(d.imag)).astype(float)
     assert np.all(err <= (n + 1) * U * s + 2 * U * np.abs(r).astype(float))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("f", [2.0 ** -1022, 1e-312, -1e-315, 3e-320, 2e-322, 2.0 ** -1074])
+def test_subnormal_factors(f):
+    """Large entries times a subnormal factor are ordinary numbers, exact to
+    one rounding of x f."""
+    rng = np.random.default_rng(13)
+    a, b = _ops(rng, 70, 60, 96, False)
+    a *= 1e290 if abs(f) > 1e-318 else 1e300
+    ops, afac = [(a, b)], [f]
+    db = _batch(ops, afac, [0], [0])
+    db.run("fp64")
+    ref = _reference(ops, afac, [0])
+    (r, s, n), = ref
+    err = np.abs(db.result()[0] - r).astype(float)
+    assert np.all(err <= (n + 1) * U * s + 2 * U * np.abs(r).astype(float))
+    for nslices in (0, 7):
+        db.run("split", nslices=nslices)
+        d = ((db.result()[0] - r) * 2.0 ** 60).astype(float)
+        assert np.linalg.norm(d) <= 1e-12 * np.linalg.norm((s * 2.0 ** 60).astype(float))
