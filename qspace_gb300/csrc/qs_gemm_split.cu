@@ -119,7 +119,7 @@ struct SplitTile {
   // C's columns); swapped: the block is computed as C^T; rdup / cdup: two
   // tile rows / columns per row / column of the computed block
   int32_t rs, splits;
-  int32_t fbase;           // FP64-grade launches: first FP64 tile flag of the block
+  int32_t fbase;           // FP64-grade launches: first FP64 tile of the block
 };
 constexpr int TILE_WORDS = (int)(sizeof(SplitTile) / 4);
 static_assert(sizeof(SplitTile) % 8 == 0 && TILE_WORDS <= 16, "tile descriptor fits one 64-byte slot");
@@ -985,13 +985,13 @@ __device__ __forceinline__ int tile_of(int r, int c, int G) { return r * G + ((r
 // from below.  An
 // output whose bound is too small for the digits' truncation to stay at the
 // level of an FP64 sum, or whose row or column holds an infinity or NaN,
-// raises the flag of its FP64 tile, which the FP64 kernel then recomputes.
+// has its FP64 cell listed (MissList), which the FP64 kernel then computes.
 template <int S, bool HP>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPair *__restrict__ pairs,
                   const uint8_t *__restrict__ arena, const int *__restrict__ E,
                   const int *__restrict__ F, double *__restrict__ C, int b, int nstages,
-                  int kchunk, int *err, int *__restrict__ flags) {
+                  int kchunk, int *err, MissList miss) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t *full = reinterpret_cast<uint64_t *>(smem);       // [MAX_STAGES]
   uint64_t *empty = full + MAX_STAGES;                        // [MAX_STAGES]
@@ -1243,6 +1243,7 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
       }
       if (!ok) break;
       if constexpr (HP) {
+        bool out = false;  // an output misses the certificate
         if (rv) {
           const int rsplit = T.splits & 1, csplit = (T.splits >> 1) & 1;
           double *crow = C + T.c_off + (int64_t)(i_glob >> rsplit) * T.rs + (i_glob & rsplit);
@@ -1254,15 +1255,20 @@ gemm_split_kernel(const SplitTile *__restrict__ tiles, int ntiles, const SplitPa
             crow[(int64_t)(j >> csplit) * T.ldc + (j & csplit)] =
                 wide_to_double((long long)Vh[jj], (long long)Vl[jj], b * (S - HG), Ei + Fj + scale_b);
             // a row or column of zeros (EMPTY_EXP) is exact
-            if (max(Ei, Fj) >= NONFINITE_EXP || (min(Ei, Fj) > EMPTY_EXP && cert[jj] < CERT_MIN)) {
-              const int rdup = (T.splits >> 3) & 1, cdup = (T.splits >> 4) & 1;
-              const int lr = i_glob >> rdup, lc = j >> cdup;
-              const bool sw = T.splits & 4;
-              const int rows = sw ? T.N >> cdup : T.Mr >> rdup;  // of C
-              flags[T.fbase + (sw ? lc : lr) / F64_TILE +
-                    (sw ? lr : lc) / F64_TILE * ((rows + F64_TILE - 1) / F64_TILE)] = 1;
-            }
+            out |= max(Ei, Fj) >= NONFINITE_EXP || (min(Ei, Fj) > EMPTY_EXP && cert[jj] < CERT_MIN);
           }
+        }
+        if (__any_sync(0xffffffffu, out)) {
+          // a thread's eight columns lie in one cell; one lane per cell lists it
+          static_assert(F64_CELL % CW == 0, "columns of a thread in one cell");
+          const int rdup = (T.splits >> 3) & 1, cdup = (T.splits >> 4) & 1;
+          const bool sw = T.splits & 4;
+          const int rows = sw ? T.N >> cdup : T.Mr >> rdup;  // of C
+          const int r = sw ? j0 >> cdup : i_glob >> rdup, c = sw ? i_glob >> rdup : j0 >> cdup;
+          const int tile = T.fbase + r / F64_TILE + c / F64_TILE * ((rows + F64_TILE - 1) / F64_TILE);
+          const int cell = (r / F64_CELL & 1) | (c / F64_CELL & 1) << 1;
+          const unsigned same = __match_any_sync(0xffffffffu, out ? tile * 4 + cell : -1);
+          if (out && lane == __ffs(same) - 1) miss.add(tile, cell);
         }
       } else {
         // the eight outputs side by side, then their stores (1024 x 1024 blocks
@@ -1317,7 +1323,7 @@ template <int S, bool HP>
 void launch_split_s(Ctx *ctx, bool cplx, const SplitPair *d_pairs, const OperandView *d_va, const OperandView *d_vb,
                     const int4 *d_sa, int nsa, const int4 *d_sb, int nsb, const SplitTile *d_tiles, int ntiles,
                     const double *A, const double *B, double *C, int *dE, int *dF, uint8_t *arena, int b,
-                    int kchunk, int *err, bool may_fork, int *flags, bool marks) {
+                    int kchunk, int *err, bool may_fork, const MissList &miss, bool marks) {
   if (b < 5 || b > 8 || b * S > 62 || (HP && (b != 8 || d_va || d_vb))) fail(QS_ERR_INTERNAL, "split: unsupported digit plan b=%d S=%d", b, S);
   cudaStream_t st = ctx->stream;
   if (marks) ctx->mark(0);
@@ -1363,7 +1369,7 @@ void launch_split_s(Ctx *ctx, bool cplx, const SplitPair *d_pairs, const Operand
   if (marks) ctx->mark(1);
   const int grid = std::min(ntiles, std::max(ctx->num_sms, 1));
   gemm_split_kernel<S, HP><<<grid, GEMM_THREADS, sm, st>>>(d_tiles, ntiles, d_pairs, arena, dE, dF, C, b, nst, kchunk,
-                                                           err, flags);
+                                                           err, miss);
   QS_LAUNCHED(ctx);
   if (marks) ctx->mark(2);
 }
@@ -1480,7 +1486,7 @@ constexpr int HP_BITS = 8, HP_DIGITS = 7;
 // Host-side work lists of one planned split product.
 struct SplitWork {
   int S = 0, b = 0, kchunk = 0;
-  bool hp = false;  // FP64-grade: one more plane per operand, tile flags
+  bool hp = false;  // FP64-grade: one more plane per operand, misses listed
   int64_t nE = 0, nF = 0, arena = 0;
   std::vector<SplitPair> sp;
   // strips of STRIP real lines: (first pair, end pair, first line, 0) of the
@@ -1499,7 +1505,7 @@ struct SplitDev {
   OperandView *va = nullptr, *vb = nullptr;
   int *E = nullptr, *F = nullptr;
   uint8_t *arena = nullptr;
-  int *flags = nullptr;  // FP64-grade: one flag per FP64 tile
+  MissList miss;  // FP64-grade
 };
 
 // Host half of the split path: digit plan, per-pair digit geometry and arena
@@ -1777,7 +1783,7 @@ static void launch_split(Ctx *ctx, const SplitWork &w, bool cplx, const SplitDev
   if (w.hp) {
     launch_split_s<HP_DIGITS, true>(ctx, cplx, d.pairs, nullptr, nullptr, d.sa, (int)w.sa.size(), d.sb,
                                     (int)w.sb.size(), d.tiles, (int)w.tiles.size(), A, B, C, d.E, d.F, d.arena, w.b,
-                                    w.kchunk, err, may_fork, d.flags, marks);
+                                    w.kchunk, err, may_fork, d.miss, marks);
     return;
   }
   switch (w.S) {
@@ -1785,7 +1791,7 @@ static void launch_split(Ctx *ctx, const SplitWork &w, bool cplx, const SplitDev
   case SS:                                                                                               \
     launch_split_s<SS, false>(ctx, cplx, d.pairs, d.va, d.vb, d.sa, (int)w.sa.size(), d.sb,               \
                               (int)w.sb.size(), d.tiles, (int)w.tiles.size(), A, B, C, d.E, d.F, d.arena, \
-                              w.b, w.kchunk, err, may_fork, nullptr, marks);                             \
+                              w.b, w.kchunk, err, may_fork, MissList{}, marks);                          \
     break;
     QS_CASE(2)
     QS_CASE(3)
@@ -1808,7 +1814,7 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
                                    const std::vector<OperandView> *vb);
 
 // Sends a planned product's work lists (one staging copy; L keeps them until
-// the launches are queued) and launches it; the arena and the flags are set.
+// the launches are queued) and launches it; the arena and the miss list are set.
 static void run_split_work(Ctx *ctx, const SplitWork &w, bool cplx, SplitDev d, DevLists &L, const double *A,
                            const double *B, double *C, bool marks) {
   const size_t sp = L.add(w.sp), sa = L.add(w.sa), sb = L.add(w.sb), st = L.add(w.tiles);
@@ -2066,10 +2072,10 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
     const int64_t M = bM[g], N = bN[g];
     int64_t bytes = 0;
     if ((!skip.empty() && skip[g]) || !f64_tensor_takes(pairs, grp[g], grp[g + 1], M, N, cplx, bytes)) continue;
-    const int64_t cells = ((M + F64_TILE - 1) / F64_TILE) * ((N + F64_TILE - 1) / F64_TILE);
-    if (tl.nflags + cells > INT32_MAX) continue;
+    const int64_t tiles = ((M + F64_TILE - 1) / F64_TILE) * ((N + F64_TILE - 1) / F64_TILE);
+    if (tl.ntiles + tiles > INT32_MAX / 4) continue;
     tl.on[g] = 1;
-    tl.fbase[g] = (int32_t)tl.nflags;
+    tl.fbase[g] = (int32_t)tl.ntiles;
     TileDesc t{};
     t.c_off = coff[g];
     t.p0 = (int32_t)grp[g];
@@ -2078,9 +2084,9 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
     t.N = bN[g];
     t.ldc = bldc ? (*bldc)[g] : std::max(bM[g], 1);
     t.cblk = (int32_t)g;
-    t.flag = tl.fbase[g];
+    t.first = tl.fbase[g];
     tl.checked.push_back(t);
-    tl.nflags += cells;
+    tl.ntiles += tiles;
     if (chunk_bytes && chunk_bytes + bytes > F64T_CHUNK_BYTES) {
       tl.chunks.push_back({chunk0, g});
       chunk0 = g;
@@ -2112,7 +2118,7 @@ static void plan_f64_chunk(const F64TensorList &tl, std::pair<int64_t, int64_t> 
 bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                     const std::vector<int64_t> &grp, const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                     const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, const double *A,
-                    const double *B, double *C, bool cplx, int *d_flags) {
+                    const double *B, double *C, bool cplx, const MissList &miss) {
   std::vector<SplitWork> ws(tl.chunks.size());
   int64_t arena = 256;
   for (size_t k = 0; k < ws.size(); ++k) {
@@ -2132,7 +2138,7 @@ bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDes
     if (w.tiles.empty()) continue;
     SplitDev d;
     d.arena = digits;
-    d.flags = d_flags;
+    d.miss = miss;
     DevLists L;
     run_split_work(ctx, w, cplx, d, L, A, B, C, k == 0);
   }
@@ -2147,7 +2153,7 @@ struct SplitPlanHandle {
   std::vector<SplitWork> w;
   std::vector<SplitDev> d;
   bool cplx = false;
-  int64_t flag_bytes = 0;  // cleared before the first launch
+  MissList miss;  // FP64-grade; the head is cleared before the first launch
   std::vector<void *> owned;
   ~SplitPlanHandle() {
     for (void *p : owned) cudaFree(p);
@@ -2206,7 +2212,7 @@ SplitPlanHandle *split_plan_create(const std::vector<PairDesc> &pairs, const std
 SplitPlanHandle *f64_tensor_plan_create(const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                                         const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
                                         const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
-                                        const std::vector<int32_t> &bldc, bool cplx, const int *&d_flags) {
+                                        const std::vector<int32_t> &bldc, bool cplx, MissList &miss) {
   std::unique_ptr<SplitPlanHandle> h(new SplitPlanHandle);
   h->cplx = cplx;
   h->w.resize(tl.chunks.size());
@@ -2214,10 +2220,12 @@ SplitPlanHandle *f64_tensor_plan_create(const F64TensorList &tl, const std::vect
     plan_f64_chunk(tl, tl.chunks[k], pairs, grp, bM, bN, coff, &bldc, cplx, h->w[k]);
   try {
     h->allocate();
-    h->flag_bytes = tl.nflags * (int64_t)sizeof(int);
-    int *flags = static_cast<int *>(h->own((size_t)h->flag_bytes));
-    for (SplitDev &v : h->d) v.flags = flags;
-    d_flags = flags;
+    MissList &c = h->miss;
+    c.n = tl.ntiles;
+    c.head = static_cast<int *>(h->own(c.head_bytes()));
+    c.list = static_cast<int *>(h->own(c.list_bytes()));
+    for (SplitDev &v : h->d) v.miss = c;
+    miss = c;
   } catch (const Error &e) {
     if (e.code != QS_ERR_OOM) throw;
     cudaGetLastError();
@@ -2227,7 +2235,7 @@ SplitPlanHandle *f64_tensor_plan_create(const F64TensorList &tl, const std::vect
 }
 
 void split_plan_launch(Ctx *ctx, SplitPlanHandle *h, const double *A, const double *B, double *C) {
-  if (h->flag_bytes) QS_CUDA(cudaMemsetAsync(h->d[0].flags, 0, (size_t)h->flag_bytes, ctx->stream));
+  if (h->miss.n) QS_CUDA(cudaMemsetAsync(h->miss.head, 0, h->miss.head_bytes(), ctx->stream));
   for (size_t k = 0; k < h->w.size(); ++k)
     if (!h->w[k].tiles.empty()) launch_split(ctx, h->w[k], h->cplx, h->d[k], A, B, C, ctx->d_err, true, k == 0);
 }

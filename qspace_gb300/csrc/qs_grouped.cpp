@@ -149,22 +149,26 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
     for (size_t b = 0; b < mm.size(); ++b) skip[b] |= tl.on[b];
     std::vector<TileDesc> tiles = make_tiles(gg, mm, nn, cc, F64_TILE, F64_TILE, ll, &pp, &skip);
     if (!tiles.empty() || !tl.checked.empty()) {
-      // the flags are cleared with the lists, before the launch that raises them
+      // the misses' head is cleared with the lists, before the launch that lists them
+      MissList miss;
+      miss.n = tl.ntiles;
       const size_t sp = lists.add(pp), st = lists.add(tiles), sc = lists.add(tl.checked),
-                   sf = lists.zeros((size_t)tl.nflags * sizeof(int));
+                   sh = lists.zeros(miss.head_bytes()), sl = lists.space(miss.list_bytes());
       lists.commit(ctx);
+      miss.head = lists.at<int>(sh);
+      miss.list = lists.at<int>(sl);
       int64_t nchecked = (int64_t)tl.checked.size();
-      if (nchecked && !run_f64_tensor(ctx, tl, pp, gg, mm, nn, cc, ll, A, B, C, cplx, lists.at<int>(sf))) {
+      if (nchecked && !run_f64_tensor(ctx, tl, pp, gg, mm, nn, cc, ll, A, B, C, cplx, miss)) {
         // no room for the digits: every tile in FP64
         tiles = make_tiles(gg, mm, nn, cc, F64_TILE, F64_TILE, ll, &pp, &dots);
         nchecked = 0;
         const size_t all = more.add(tiles);
         more.commit(ctx);
-        launch_gemm_f64(ctx, lists.at<PairDesc>(sp), more.at<TileDesc>(all), (int64_t)tiles.size(), nullptr, 0, 0,
-                        nullptr, A, B, C, cplx ? 1 : 0);
+        launch_gemm_f64(ctx, lists.at<PairDesc>(sp), more.at<TileDesc>(all), (int64_t)tiles.size(), nullptr, 0,
+                        MissList{}, A, B, C, cplx ? 1 : 0);
       } else {
         launch_gemm_f64(ctx, lists.at<PairDesc>(sp), lists.at<TileDesc>(st), (int64_t)tiles.size(),
-                        lists.at<TileDesc>(sc), nchecked, tl.nflags, lists.at<int>(sf), A, B, C, cplx ? 1 : 0);
+                        lists.at<TileDesc>(sc), nchecked, miss, A, B, C, cplx ? 1 : 0);
       }
     }
     if (deep) {

@@ -240,7 +240,7 @@ struct TileDesc {
   int32_t M, N;
   int32_t ldc;
   int32_t cblk;
-  int32_t flag;   // first tile flag of a checked block (launch_gemm_f64)
+  int32_t first;  // first tile of a checked block (launch_gemm_f64)
   int32_t pad_;
 };
 static_assert(sizeof(TileDesc) == 48, "TileDesc layout");
@@ -273,13 +273,31 @@ void launch_permute(Ctx *ctx, const PermDesc *d_desc, const int64_t *d_chunk_blk
                     const double *in, double *out, int is_complex, int chunk_elems);
 
 // qs_gemm_f64.cu -- plain FP64 grouped GEMM (deterministic: one CTA owns an
-// output tile, pairs summed in order) of the listed tiles, and of the tiles of
-// the blocks in d_checked whose flag is raised (each entry describes a block:
-// m0 = n0 = 0, `flag` the index of its first tile's flag; ascending)
+// output tile, pairs summed in order) of the listed tiles, and of the cells
+// that the tensor-core launch listed among the blocks in d_checked (each entry
+// describes a block: m0 = n0 = 0, `first` the index of its first tile, tiles
+// column by column; ascending)
 constexpr int F64_TILE = 32;
+constexpr int F64_CELL = 16;  // a quarter of a tile
+// What to compute again: head[0] tiles in `list`, each once, head[1] of them
+// taken so far; from head[2] on four bits per tile, one for each cell (row + 2
+// column) with a missed output.  The head is cleared before the launch that lists.
+struct MissList {
+  int *head = nullptr, *list = nullptr;
+  int64_t n = 0;  // tiles of the checked blocks
+  size_t head_bytes() const { return (size_t)(2 + (n + 7) / 8) * sizeof(int); }
+  size_t list_bytes() const { return (size_t)n * sizeof(int); }
+#ifdef __CUDACC__
+  __device__ __forceinline__ void add(int tile, int cell) const {
+    const int sh = (tile & 7) * 4, old = atomicOr(head + 2 + (tile >> 3), 1 << (sh + cell));
+    if (!((old >> sh) & 15)) list[atomicAdd(head, 1)] = tile;
+  }
+  __device__ __forceinline__ int cells(int tile) const { return (head[2 + (tile >> 3)] >> ((tile & 7) * 4)) & 15; }
+#endif
+};
 void launch_gemm_f64(Ctx *ctx, const PairDesc *d_pairs, const TileDesc *d_tiles, int64_t ntiles,
-                     const TileDesc *d_checked, int64_t nchecked, int64_t ncells, const int *d_flags,
-                     const double *A, const double *B, double *C, int is_complex);
+                     const TileDesc *d_checked, int64_t nchecked, const MissList &miss, const double *A,
+                     const double *B, double *C, int is_complex);
 
 // qs_permute.cu -- per-block "all zero" test for SkipZeroData, and the
 // real -> complex widening of an operand arena

@@ -58,10 +58,10 @@ struct qs_grouped_plan {
   PairDesc *d_pairs = nullptr;  // FP64 path
   TileDesc *d_tiles = nullptr;
   int64_t ntiles = 0;
-  // FP64 path: blocks of `split` whose tiles are recomputed when flagged
+  // FP64 path: blocks of `split` whose cells are computed again when listed
   TileDesc *d_checked = nullptr;
-  int64_t nchecked = 0, ncells = 0;
-  const int *d_flags = nullptr;
+  int64_t nchecked = 0;
+  MissList miss;
   // shallow output blocks run directly (as in the one-shot calls); `main`
   // holds the other blocks (all of them when none is shallow)
   ShallowPlan shallow;
@@ -83,8 +83,8 @@ void launch_direct(qs_grouped_plan *p, const double *A, const double *B, double 
     split_plan_launch(p->ctx, p->split, A, B, C);
   else {
     if (p->split) split_plan_launch(p->ctx, p->split, A, B, C);
-    launch_gemm_f64(p->ctx, p->d_pairs, p->d_tiles, p->ntiles, p->d_checked, p->nchecked, p->ncells, p->d_flags, A, B,
-                    C, p->g.cplx ? 1 : 0);
+    launch_gemm_f64(p->ctx, p->d_pairs, p->d_tiles, p->ntiles, p->d_checked, p->nchecked, p->miss, A, B, C,
+                    p->g.cplx ? 1 : 0);
   }
 }
 
@@ -266,7 +266,7 @@ qs_status qs_grouped_plan_create(qs_ctx *ctx, const qs_pair_list *pairs, const q
       const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.coff, &m.bldc, m.cplx, {});
       if (!tl.checked.empty()) {
         c->ensure_aux();
-        p->split = f64_tensor_plan_create(tl, m.pairs, m.grp, m.bM, m.bN, m.coff, m.bldc, m.cplx, p->d_flags);
+        p->split = f64_tensor_plan_create(tl, m.pairs, m.grp, m.bM, m.bN, m.coff, m.bldc, m.cplx, p->miss);
       }
       // every tile in FP64 when there is no room for the digits
       const std::vector<TileDesc> tiles =
@@ -281,7 +281,6 @@ qs_status qs_grouped_plan_create(qs_ctx *ctx, const qs_pair_list *pairs, const q
       put(p->d_tiles, tiles);
       if (p->split) {
         p->nchecked = (int64_t)tl.checked.size();
-        p->ncells = tl.nflags;
         put(p->d_checked, tl.checked);
       }
     }

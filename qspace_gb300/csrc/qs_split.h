@@ -57,14 +57,14 @@ SplitResult run_split_static(Ctx *ctx, const std::vector<PairDesc> &pairs,
 // FP64-grade products on the tensor cores, for the plain FP64 path: digits of
 // 56 bits per operand, summed without rounding, with a certificate per output
 // that the truncation stays at the level of an FP64 sum.  Where it does not
-// (and where a line holds an infinity or NaN) the launch raises the flag of
-// the output's FP64 tile (F64_TILE), and the FP64 kernel recomputes it.
+// (and where a line holds an infinity or NaN) the launch lists the output's
+// cell (MissList), and the FP64 kernel computes it.
 struct F64TensorList {
   std::vector<char> on;         // per block: computed by the tensor-core launch
-  std::vector<int32_t> fbase;   // per block: first tile flag
+  std::vector<int32_t> fbase;   // per block: first FP64 tile
   std::vector<std::pair<int64_t, int64_t>> chunks;  // block ranges of one launch each
   std::vector<TileDesc> checked;  // the blocks as launch_gemm_f64 takes them
-  int64_t nflags = 0;
+  int64_t ntiles = 0;  // FP64 tiles of the checked blocks
 };
 // The blocks of a list that the tensor-core launch takes (a property of the
 // block alone), except those marked in `skip`.  The list holds no shallow
@@ -79,7 +79,7 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
 bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                     const std::vector<int64_t> &grp, const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                     const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, const double *A,
-                    const double *B, double *C, bool cplx, int *d_flags);
+                    const double *B, double *C, bool cplx, const MissList &miss);
 
 // Reusable split plans (stable device addresses, for CUDA graph replay).
 struct SplitPlanHandle;
@@ -93,7 +93,7 @@ SplitPlanHandle *split_plan_create(const std::vector<PairDesc> &pairs, const std
 SplitPlanHandle *f64_tensor_plan_create(const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                                         const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
                                         const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
-                                        const std::vector<int32_t> &bldc, bool cplx, const int *&d_flags);
+                                        const std::vector<int32_t> &bldc, bool cplx, MissList &miss);
 void split_plan_launch(Ctx *ctx, SplitPlanHandle *h, const double *A, const double *B, double *C);
 void split_plan_destroy(SplitPlanHandle *h);
 

@@ -350,3 +350,43 @@ def test_subnormal_factors(f):
         db.run("split", nslices=nslices)
         d = ((db.result()[0] - r) * 2.0 ** 60).astype(float)
         assert np.linalg.norm(d) <= 1e-12 * np.linalg.norm((s * 2.0 ** 60).astype(float))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cplx", [False, True])
+def test_f64_cells_of_a_list(cplx):
+    """Blocks of which all, some or no outputs are computed again, depths far
+    apart, edges of the 16 x 16 cells; from a plan the cells are listed anew on
+    every run."""
+    rng = np.random.default_rng(17)
+    ops, trans = [], []
+    for M, N, K in [(16, 16, 2100), (17, 31, 640), (1, 513, 99), (513, 1, 99), (15, 90, 70), (160, 48, 33), (49, 64, 257),
+                    (300, 260, 40)]:
+        for kind in ("skew", "identity", "some", "none"):
+            a, b = _ops(rng, M, N, K, cplx)
+            if kind == "skew":
+                a = a * np.exp(3 * rng.standard_normal(a.shape))
+                b = b * np.exp(3 * rng.standard_normal(b.shape))
+            elif kind == "identity":
+                a = np.eye(M, K, dtype=a.dtype)
+            elif kind == "some":
+                a[M // 2, 1:] *= 1e-9
+            ops.append((a, b))
+            trans.append(int(rng.integers(0, 16 if cplx else 4)))
+    n = len(ops)
+    afac, blk = list(rng.uniform(0.5, 1.0, n)), list(range(n))
+    db = _batch(ops, afac, blk, trans)
+    db.run("fp64")
+    got = [c.copy() for c in db.result()]
+    for c, (r, s, k) in zip(got, _reference(ops, afac, blk)):
+        d = c - r
+        err = np.maximum(np.abs(d.real), np.abs(d.imag)).astype(float)
+        assert np.all(err <= (k + 1) * U * s + 2 * U * np.abs(r).astype(float))
+    plan = db.plan("fp64")
+    for _ in range(3):
+        db.dC.fill_(float("nan"))
+        db.torch.cuda.synchronize()
+        db.run_plan(plan)
+        for c, w in zip(db.result(), got):
+            assert np.array_equal(c, w)
+    plan.close()
