@@ -129,12 +129,22 @@ void DevLists::commit(Ctx *ctx) {
   ctx_ = ctx;
   base_ = dev_alloc<char>(ctx, sent_ + scratch_);
   if (!sent_) return;
-  char *h = ctx->stage_reserve(sent_);
-  for (const Span &s : spans_) {
-    if (s.src) std::memcpy(h + s.off, s.src, s.bytes);
-    else std::memset(h + s.off, 0, s.bytes);
-  }
+  pack(ctx->stage_reserve(sent_));
   ctx->stage_commit(base_, sent_);
+}
+
+void PlanLists::commit(Ctx *ctx) {
+  ctx_ = ctx;
+  base_ = dev_alloc<char>(ctx, sent_ + scratch_);
+  if (!sent_) return;
+  pack(ctx->stage_reserve(sent_));
+  ctx->stage_commit(base_, sent_);
+}
+
+PlanLists::~PlanLists() {
+  if (!base_) return;
+  if (ctx_alive(ctx_)) dev_free(ctx_, base_);
+  else cudaFree(base_);
 }
 
 void Ctx::ensure_ret(size_t bytes) {

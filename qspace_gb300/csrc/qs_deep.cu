@@ -477,25 +477,20 @@ void run_shallow(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector
                  cplx);
 }
 
-ShallowPlan shallow_prepare(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
-                            const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
-                            const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc,
-                            const std::vector<int64_t> &blocks, bool cplx) {
+ShallowPlan shallow_prepare(Ctx *ctx, PlanLists &mem, const std::vector<PairDesc> &pairs,
+                            const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
+                            const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
+                            const std::vector<int32_t> *bldc, const std::vector<int64_t> &blocks, bool cplx) {
   const std::vector<ShallowTask> tasks = shallow_tasks(grp, bM, bN, coff, bldc, blocks, cplx);
   const std::vector<PairDesc> pp = pairs_of(pairs, grp, blocks);
   ShallowPlan sp;
   sp.cplx = cplx;
   sp.ntasks = (int64_t)tasks.size();
   if (tasks.empty()) return sp;
-  try {
-    QS_CUDA(cudaMalloc(&sp.tasks, tasks.size() * sizeof(ShallowTask)));
-    QS_CUDA(cudaMemcpy(sp.tasks, tasks.data(), tasks.size() * sizeof(ShallowTask), cudaMemcpyHostToDevice));
-    QS_CUDA(cudaMalloc(&sp.pairs, std::max<size_t>(pp.size(), 1) * sizeof(PairDesc)));
-    if (!pp.empty()) QS_CUDA(cudaMemcpy(sp.pairs, pp.data(), pp.size() * sizeof(PairDesc), cudaMemcpyHostToDevice));
-  } catch (...) {
-    shallow_release(sp);
-    throw;
-  }
+  const size_t st = mem.add(tasks), so = mem.add(pp);
+  mem.commit(ctx);
+  sp.tasks = mem.at<ShallowTask>(st);
+  sp.pairs = mem.at<PairDesc>(so);
   return sp;
 }
 
@@ -503,13 +498,6 @@ void shallow_launch(Ctx *ctx, const ShallowPlan &sp, const double *A, const doub
   if (!sp.ntasks) return;
   launch_shallow(ctx, static_cast<const ShallowTask *>(sp.tasks), sp.ntasks, static_cast<const PairDesc *>(sp.pairs),
                  nullptr, nullptr, A, B, C, sp.cplx);
-}
-
-void shallow_release(ShallowPlan &sp) {
-  if (sp.tasks) cudaFree(sp.tasks);
-  if (sp.pairs) cudaFree(sp.pairs);
-  sp.tasks = sp.pairs = nullptr;
-  sp.ntasks = 0;
 }
 
 BlockList select_blocks(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,

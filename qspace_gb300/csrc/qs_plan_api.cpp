@@ -55,16 +55,18 @@ struct qs_grouped_plan {
   SplitResult sr;
   bool tune_pending = false;
   float tuned_ms = 0;
-  PairDesc *d_pairs = nullptr;  // FP64 path
-  TileDesc *d_tiles = nullptr;
+  PlanLists lists;  // FP64 path
+  const PairDesc *d_pairs = nullptr;
+  const TileDesc *d_tiles = nullptr;
   int64_t ntiles = 0;
   // FP64 path: blocks of `split` whose cells are computed again when listed
-  TileDesc *d_checked = nullptr;
+  const TileDesc *d_checked = nullptr;
   int64_t nchecked = 0;
   MissList miss;
   // shallow output blocks run directly (as in the one-shot calls); `main`
   // holds the other blocks (all of them when none is shallow)
   ShallowPlan shallow;
+  PlanLists shallow_lists;
   GroupedPlan main;
   cudaGraphExec_t exec = nullptr;
   const double *gA = nullptr, *gB = nullptr;
@@ -98,7 +100,7 @@ SplitPlanHandle *make_split(qs_grouped_plan *p, int bits, SplitResult *r) {
     bits = dp.bits;
     ns = dp.nslices;
   }
-  return split_plan_create(g.pairs, g.grp, g.bM, g.bN, g.coff, g.bldc, g.cplx, ns, p->o.tol, bits, r);
+  return split_plan_create(p->ctx, g.pairs, g.grp, g.bM, g.bN, g.coff, g.bldc, g.cplx, ns, p->o.tol, bits, r);
 }
 
 // Splits the plan's blocks into shallow ones (prepared for the direct
@@ -118,7 +120,7 @@ void split_shallow(qs_grouped_plan *p) {
     p->main = g;
     return;
   }
-  p->shallow = shallow_prepare(g.pairs, g.grp, g.bM, g.bN, g.coff, &g.bldc, ids, g.cplx);
+  p->shallow = shallow_prepare(p->ctx, p->shallow_lists, g.pairs, g.grp, g.bM, g.bN, g.coff, &g.bldc, ids, g.cplx);
   BlockList R = select_blocks(g.pairs, g.grp, g.bM, g.bN, g.coff, &g.bldc, rest);
   GroupedPlan &m = p->main;
   m.cplx = g.cplx;
@@ -266,23 +268,18 @@ qs_status qs_grouped_plan_create(qs_ctx *ctx, const qs_pair_list *pairs, const q
       const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.coff, &m.bldc, m.cplx, {});
       if (!tl.checked.empty()) {
         c->ensure_aux();
-        p->split = f64_tensor_plan_create(tl, m.pairs, m.grp, m.bM, m.bN, m.coff, m.bldc, m.cplx, p->miss);
+        p->split = f64_tensor_plan_create(c, tl, m.pairs, m.grp, m.bM, m.bN, m.coff, m.bldc, m.cplx, p->miss);
       }
       // every tile in FP64 when there is no room for the digits
       const std::vector<TileDesc> tiles =
           make_tiles(m.grp, m.bM, m.bN, m.coff, F64_TILE, F64_TILE, &m.bldc, &m.pairs, p->split ? &tl.on : nullptr);
-      auto put = [](auto *&d, const auto &v) {
-        if (v.empty()) return;
-        QS_CUDA(cudaMalloc(&d, v.size() * sizeof(v[0])));
-        QS_CUDA(cudaMemcpy(d, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice));
-      };
       p->ntiles = (int64_t)tiles.size();
-      put(p->d_pairs, m.pairs);
-      put(p->d_tiles, tiles);
-      if (p->split) {
-        p->nchecked = (int64_t)tl.checked.size();
-        put(p->d_checked, tl.checked);
-      }
+      if (p->split) p->nchecked = (int64_t)tl.checked.size();
+      const size_t op = p->lists.add(m.pairs), ot = p->lists.add(tiles), oc = p->lists.add(tl.checked);
+      p->lists.commit(c);
+      p->d_pairs = p->lists.at<PairDesc>(op);
+      p->d_tiles = p->lists.at<TileDesc>(ot);
+      p->d_checked = p->lists.at<TileDesc>(oc);
     }
   } else {
     fail(QS_ERR_ARG, "unknown precision mode %d", p->o.prec);
@@ -335,10 +332,6 @@ void qs_grouped_plan_destroy(qs_grouped_plan *p) {
   }
   if (p->exec) cudaGraphExecDestroy(p->exec);
   split_plan_destroy(p->split);
-  shallow_release(p->shallow);
-  if (p->d_pairs) cudaFree(p->d_pairs);
-  if (p->d_tiles) cudaFree(p->d_tiles);
-  if (p->d_checked) cudaFree(p->d_checked);
   delete p;
 }
 

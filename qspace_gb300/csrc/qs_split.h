@@ -85,12 +85,12 @@ bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDes
 struct SplitPlanHandle;
 std::vector<int> split_candidate_bits(double tol, int forced_slices);
 // bits = 0: the cost model picks the digit width
-SplitPlanHandle *split_plan_create(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
+SplitPlanHandle *split_plan_create(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                                    const std::vector<int32_t> &blk_M, const std::vector<int32_t> &blk_N,
                                    const std::vector<int64_t> &c_off, const std::vector<int32_t> &blk_ldc,
                                    bool cplx, int forced_slices, double tol, int bits, SplitResult *res);
 // The FP64-grade form; nullptr when the device has no room for the digits.
-SplitPlanHandle *f64_tensor_plan_create(const F64TensorList &tl, const std::vector<PairDesc> &pairs,
+SplitPlanHandle *f64_tensor_plan_create(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                                         const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
                                         const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
                                         const std::vector<int32_t> &bldc, bool cplx, MissList &miss);

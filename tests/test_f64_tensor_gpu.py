@@ -277,14 +277,14 @@ def test_deeper_misaligned_blocks_are_refused_on_the_host(prec):
     _shifted(db, 1)
     db.dC.fill_(7.0)
     db.torch.cuda.synchronize()
+    plan = db.plan(prec)
     n0 = db.ctx.launches
     with pytest.raises(QSError, match="aligned to 16"):
         db.run(prec)
-    plan = db.plan(prec)
     with pytest.raises(QSError, match="aligned to 16"):
         db.run_plan(plan)
-    plan.close()
     assert db.ctx.launches == n0
+    plan.close()
     db.ctx.sync()
     assert bool((db.dC == 7.0).all())
 
