@@ -1708,6 +1708,7 @@ static SplitResult plan_split(const std::vector<PairDesc> &pairs_in, const std::
     t.N = (int32_t)cols_r[g];
     // column stride of C in its elements, in the caller's orientation
     const int64_t ldc0 = blk_ldc ? (*blk_ldc)[g] : std::max(blk_M_in[g], 1);
+    if (ldc0 * cm > INT32_MAX) fail(QS_ERR_SHAPE, "split: leading dimension %lld of a complex C", (long long)ldc0);
     const bool swp = mode[g] & 1, dupb = mode[g] & 2;
     if (!swp && !dupb) {
       t.ldc = (int32_t)(ldc0 * cm);
@@ -2028,7 +2029,7 @@ constexpr int64_t F64T_CHUNK_BYTES = int64_t(2) << 30, F64T_BLOCK_BYTES = int64_
 
 // Whether the tensor-core launch takes a block; `bytes` its digits (at most).
 static bool f64_tensor_takes(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int64_t M, int64_t N,
-                             bool cplx, int64_t &bytes) {
+                             int64_t ldc, bool cplx, int64_t &bytes) {
   const int64_t cm = cplx ? 2 : 1;
   auto up = [](int64_t x, int64_t t) { return (x + t - 1) / t * t; };
   int64_t depth = 0, kpad = 0;
@@ -2039,7 +2040,8 @@ static bool f64_tensor_takes(const std::vector<PairDesc> &pairs, int64_t p0, int
     // a factor of 0 keeps the FP64 kernel's 0 * x (NaN for an infinite x)
     if (!std::isfinite(pairs[p].afac) || pairs[p].afac == 0.0) return false;
   }
-  if (depth < F64T_DEPTH || depth > F64T_MAX_DEPTH || M > (1 << 24) || N > (1 << 24) ||
+  // (the tiles' strides are 32-bit counts of doubles)
+  if (depth < F64T_DEPTH || depth > F64T_MAX_DEPTH || M > (1 << 24) || N > (1 << 24) || ldc * cm > INT32_MAX ||
       double(M) * double(N) * double(depth) * double(cm) < F64T_WORK)
     return false;
   // either operand's real form may be the duplicated one
@@ -2057,9 +2059,9 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
   tl.fbase.assign(nb, 0);
   int64_t chunk0 = 0, chunk_bytes = 0;
   for (int64_t g = 0; g < nb; ++g) {
-    const int64_t M = bM[g], N = bN[g];
+    const int64_t M = bM[g], N = bN[g], ldc = bldc ? (*bldc)[g] : std::max(bM[g], 1);
     int64_t bytes = 0;
-    if ((!skip.empty() && skip[g]) || !f64_tensor_takes(pairs, grp[g], grp[g + 1], M, N, cplx, bytes)) continue;
+    if ((!skip.empty() && skip[g]) || !f64_tensor_takes(pairs, grp[g], grp[g + 1], M, N, ldc, cplx, bytes)) continue;
     const int64_t tiles = ((M + F64_TILE - 1) / F64_TILE) * ((N + F64_TILE - 1) / F64_TILE);
     if (tl.ntiles + tiles > INT32_MAX / 4) continue;
     tl.on[g] = 1;
@@ -2070,7 +2072,7 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
     t.p1 = (int32_t)grp[g + 1];
     t.M = bM[g];
     t.N = bN[g];
-    t.ldc = bldc ? (*bldc)[g] : std::max(bM[g], 1);
+    t.ldc = (int32_t)ldc;
     t.cblk = (int32_t)g;
     t.first = tl.fbase[g];
     tl.checked.push_back(t);

@@ -390,3 +390,23 @@ def test_f64_cells_of_a_list(cplx):
         for c, w in zip(db.result(), got):
             assert np.array_equal(c, w)
     plan.close()
+
+
+@pytest.mark.gpu
+def test_long_columns_of_c():
+    """Complex columns 2^30 elements apart: in doubles the stride leaves 32
+    bits.  The FP64 path takes them, the split path refuses them on the host."""
+    rng = np.random.default_rng(4)
+    M, N, K, ldc = 64, 2, 256, 1 << 30
+    ops = [_ops(rng, M, N, K, True)]
+    db = _batch(ops, [1.0], [0], [0])
+    db.pk.ldc[:] = ldc
+    t = db.torch
+    db.dC = t.empty((2 * (ldc * (N - 1) + M),), dtype=t.float64, device="cuda")
+    t.cuda.synchronize()
+    with pytest.raises(QSError, match="leading dimension"):
+        db.run("split")
+    db.run("fp64")
+    db.ctx.sync()
+    got = t.stack([db.dC[:2 * M], db.dC[2 * ldc:]]).cpu().numpy().view(np.complex128).T
+    _check([got], _reference(ops, [1.0], [0]))
