@@ -2,6 +2,7 @@
 // contractQS / permuteQS drivers and the grouped block-product seam.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -30,14 +31,26 @@ void dev_free(Ctx *ctx, void *p) {
   if (p) cudaFreeAsync(p, ctx->stream);
 }
 
+cudaError_t pool_alloc(Ctx *ctx, void **p, size_t bytes) {
+  const char *limit = std::getenv("QS_ALLOC_LIMIT_MB");
+  if (limit && double(bytes) > std::atof(limit) * (1 << 20)) return cudaErrorMemoryAllocation;
+  return cudaMallocAsync(p, bytes, ctx->stream);
+}
+
 void *Ctx::ensure_scratch(size_t bytes) {
   if (bytes <= scratch_bytes) return scratch;
   if (scratch) QS_CUDA(cudaFreeAsync(scratch, stream));
   size_t nb = std::max(bytes, scratch_bytes * 3 / 2);
   scratch = nullptr;
-  cudaError_t e = cudaMallocAsync(&scratch, nb, stream);
+  scratch_bytes = 0;
+  cudaError_t e = pool_alloc(this, &scratch, nb);
+  if (e == cudaErrorMemoryAllocation && nb > bytes) {  // no room to grow ahead of the need
+    cudaGetLastError();
+    nb = bytes;
+    e = pool_alloc(this, &scratch, nb);
+  }
   if (e != cudaSuccess) {
-    scratch_bytes = 0;
+    scratch = nullptr;
     fail(e == cudaErrorMemoryAllocation ? QS_ERR_OOM : QS_ERR_CUDA, "scratch allocation of %zu bytes: %s", nb,
          cudaGetErrorString(e));
   }

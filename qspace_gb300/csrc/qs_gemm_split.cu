@@ -1802,10 +1802,10 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
                                    int forced_bits, const std::vector<OperandView> *va,
                                    const std::vector<OperandView> *vb);
 
-// Sends a planned product's work lists (one staging copy; L keeps them until
-// the launches are queued) and launches it; the arena and the miss list are set.
-static void run_split_work(Ctx *ctx, const SplitWork &w, bool cplx, SplitDev d, DevLists &L, const double *A,
-                           const double *B, double *C, bool marks) {
+// Sends a planned product's work lists (one staging copy; L keeps them until the
+// launches are queued); the arena and the miss list are the caller's.
+static SplitDev stage_split_work(Ctx *ctx, const SplitWork &w, DevLists &L) {
+  SplitDev d;
   const size_t sp = L.add(w.sp), sa = L.add(w.sa), sb = L.add(w.sb), st = L.add(w.tiles);
   const size_t va = L.add(w.va), vb = L.add(w.vb);
   const size_t se = L.space((size_t)w.nE * sizeof(int)), sf = L.space((size_t)w.nF * sizeof(int));
@@ -1818,7 +1818,7 @@ static void run_split_work(Ctx *ctx, const SplitWork &w, bool cplx, SplitDev d, 
   if (!w.vb.empty()) d.vb = L.at<OperandView>(vb);
   d.E = L.at<int>(se);
   d.F = L.at<int>(sf);
-  launch_split(ctx, w, cplx, d, A, B, C, ctx->d_err, true, marks);
+  return d;
 }
 
 // Shallow output blocks (summed depth <= SHALLOW_K) are computed directly in
@@ -1941,11 +1941,11 @@ static SplitResult run_split_lists(Ctx *ctx, const std::vector<PairDesc> &pairs,
                                va, vb);
   if (w.tiles.empty()) return res;
   require_whole_elements(A, B, nullptr, cplx);  // the products' stores are single doubles
-  // the digit arena is pooled scratch
-  SplitDev d;
-  d.arena = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)std::max<int64_t>(w.arena, 256)));
   DevLists L;
-  run_split_work(ctx, w, cplx, d, L, A, B, C, true);
+  SplitDev d = stage_split_work(ctx, w, L);
+  // the digit arena is pooled scratch
+  d.arena = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)std::max<int64_t>(w.arena, 256)));
+  launch_split(ctx, w, cplx, d, A, B, C, ctx->d_err, true, true);
   return res;
 }
 
@@ -2057,7 +2057,6 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
   const int64_t nb = (int64_t)bM.size();
   tl.on.assign(nb, 0);
   tl.fbase.assign(nb, 0);
-  int64_t chunk0 = 0, chunk_bytes = 0;
   for (int64_t g = 0; g < nb; ++g) {
     const int64_t M = bM[g], N = bN[g], ldc = bldc ? (*bldc)[g] : std::max(bM[g], 1);
     int64_t bytes = 0;
@@ -2077,15 +2076,26 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
     t.first = tl.fbase[g];
     tl.checked.push_back(t);
     tl.ntiles += tiles;
-    if (chunk_bytes && chunk_bytes + bytes > F64T_CHUNK_BYTES) {
-      tl.chunks.push_back({chunk0, g});
-      chunk0 = g;
-      chunk_bytes = 0;
-    }
-    chunk_bytes += bytes;
+    tl.bytes.push_back(bytes);
   }
-  if (!tl.checked.empty()) tl.chunks.push_back({chunk0, nb});
   return tl;
+}
+
+// The block ranges of launches that hold at most `limit` bytes of digits each
+// (a block above it gets a launch of its own).
+static std::vector<std::pair<int64_t, int64_t>> f64_chunks(const F64TensorList &tl, int64_t limit) {
+  std::vector<std::pair<int64_t, int64_t>> chunks;
+  int64_t held = 0;
+  for (size_t k = 0; k < tl.checked.size(); ++k) {
+    const int64_t g = tl.checked[k].cblk;
+    if (chunks.empty() || held + tl.bytes[k] > limit) {
+      chunks.push_back({g, g});
+      held = 0;
+    }
+    chunks.back().second = g + 1;
+    held += tl.bytes[k];
+  }
+  return chunks;
 }
 
 // Work lists of the launch of one block range of a list.
@@ -2105,33 +2115,58 @@ static void plan_f64_chunk(const F64TensorList &tl, std::pair<int64_t, int64_t> 
   plan_split(L.pairs, L.grp, L.bM, L.bN, L.coff, cplx, 0, 0, &L.bldc, w, 0, nullptr, nullptr, &fb);
 }
 
+// Plans the launches of a list and hands them to `allocate`, with fewer digits
+// a launch where that finds no room; false when the launches of single blocks
+// do not fit either.
+template <class F>
+static bool plan_f64_launches(const F64TensorList &tl, const std::vector<PairDesc> &pairs,
+                              const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
+                              const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
+                              const std::vector<int32_t> *bldc, bool cplx, std::vector<SplitWork> &ws, F allocate) {
+  size_t tried = 0;
+  for (int64_t limit = F64T_CHUNK_BYTES; tried < tl.checked.size(); limit /= 4) {
+    const auto chunks = f64_chunks(tl, limit);
+    if (chunks.size() == tried) continue;
+    tried = chunks.size();
+    ws.clear();
+    ws.resize(tried);
+    for (size_t k = 0; k < tried; ++k) plan_f64_chunk(tl, chunks[k], pairs, grp, bM, bN, coff, bldc, cplx, ws[k]);
+    try {
+      allocate();
+      return true;
+    } catch (const Error &e) {
+      if (e.code != QS_ERR_OOM) throw;
+      cudaGetLastError();
+    }
+  }
+  return false;
+}
+
 bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                     const std::vector<int64_t> &grp, const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                     const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, const double *A,
                     const double *B, double *C, bool cplx, const MissList &miss) {
-  std::vector<SplitWork> ws(tl.chunks.size());
-  int64_t arena = 256;
-  for (size_t k = 0; k < ws.size(); ++k) {
-    plan_f64_chunk(tl, tl.chunks[k], pairs, grp, bM, bN, coff, bldc, cplx, ws[k]);
-    arena = std::max(arena, ws[k].arena);
-  }
-  uint8_t *digits = nullptr;
-  try {
-    digits = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)arena));
-  } catch (const Error &e) {
-    if (e.code != QS_ERR_OOM) throw;
-    cudaGetLastError();
-    return false;
-  }
-  for (size_t k = 0; k < ws.size(); ++k) {
-    const SplitWork &w = ws[k];
-    if (w.tiles.empty()) continue;
-    SplitDev d;
-    d.arena = digits;
-    d.miss = miss;
-    DevLists L;
-    run_split_work(ctx, w, cplx, d, L, A, B, C, k == 0);
-  }
+  std::vector<SplitWork> ws;
+  std::vector<std::unique_ptr<DevLists>> lists;
+  std::vector<SplitDev> ds;
+  // every allocation before the first launch
+  auto allocate = [&] {
+    ds.clear();
+    lists.clear();
+    int64_t arena = 256;
+    for (const SplitWork &w : ws) {
+      lists.push_back(std::make_unique<DevLists>());
+      ds.push_back(stage_split_work(ctx, w, *lists.back()));
+      arena = std::max(arena, w.arena);
+    }
+    uint8_t *digits = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)arena));
+    for (SplitDev &d : ds) {
+      d.arena = digits;
+      d.miss = miss;
+    }
+  };
+  if (!plan_f64_launches(tl, pairs, grp, bM, bN, coff, bldc, cplx, ws, allocate)) return false;
+  for (size_t k = 0; k < ws.size(); ++k) launch_split(ctx, ws[k], cplx, ds[k], A, B, C, ctx->d_err, true, k == 0);
   return true;
 }
 
@@ -2144,10 +2179,13 @@ struct SplitPlanHandle {
   std::vector<SplitDev> d;
   bool cplx = false;
   MissList miss;  // FP64-grade; the head is cleared before the first launch
-  PlanLists mem;
+  std::unique_ptr<PlanLists> lists;
   // every launch's lists and exponent arrays, one arena, and the miss list of
   // `tiles` FP64 tiles
   void allocate(Ctx *ctx, int64_t tiles = 0) {
+    lists.reset(new PlanLists);
+    d.clear();
+    PlanLists &mem = *lists;
     int64_t arena = 0;
     struct At {
       size_t pairs, sa, sb, tiles, E, F;
@@ -2208,17 +2246,9 @@ SplitPlanHandle *f64_tensor_plan_create(Ctx *ctx, const F64TensorList &tl, const
                                         const std::vector<int32_t> &bldc, bool cplx, MissList &miss) {
   std::unique_ptr<SplitPlanHandle> h(new SplitPlanHandle);
   h->cplx = cplx;
-  h->w.resize(tl.chunks.size());
-  for (size_t k = 0; k < h->w.size(); ++k)
-    plan_f64_chunk(tl, tl.chunks[k], pairs, grp, bM, bN, coff, &bldc, cplx, h->w[k]);
-  try {
-    h->allocate(ctx, tl.ntiles);
-    miss = h->miss;
-  } catch (const Error &e) {
-    if (e.code != QS_ERR_OOM) throw;
-    cudaGetLastError();
+  if (!plan_f64_launches(tl, pairs, grp, bM, bN, coff, &bldc, cplx, h->w, [&] { h->allocate(ctx, tl.ntiles); }))
     return nullptr;
-  }
+  miss = h->miss;
   return h.release();
 }
 

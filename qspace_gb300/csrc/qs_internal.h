@@ -335,11 +335,15 @@ inline void require_whole_elements(const double *A, const double *B, const doubl
 }
 
 // ------------------------------------------------------ small utilities
+// Stream-ordered memory from the device's pool (qs_capi.cpp).
+// QS_ALLOC_LIMIT_MB in the environment refuses larger single allocations as if
+// the device had no room for them.
+cudaError_t pool_alloc(Ctx *ctx, void **p, size_t bytes);
 template <class T>
 T *dev_alloc(Ctx *ctx, size_t n) {
   void *p = nullptr;
   if (n == 0) n = 1;
-  cudaError_t e = cudaMallocAsync(&p, n * sizeof(T), ctx->stream);
+  cudaError_t e = pool_alloc(ctx, &p, n * sizeof(T));
   if (e != cudaSuccess)
     fail(e == cudaErrorMemoryAllocation ? QS_ERR_OOM : QS_ERR_CUDA,
          "cudaMallocAsync(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));

@@ -55,7 +55,7 @@ struct qs_grouped_plan {
   SplitResult sr;
   bool tune_pending = false;
   float tuned_ms = 0;
-  PlanLists lists;  // FP64 path
+  std::unique_ptr<PlanLists> lists;  // FP64 path
   const PairDesc *d_pairs = nullptr;
   const TileDesc *d_tiles = nullptr;
   int64_t ntiles = 0;
@@ -72,6 +72,11 @@ struct qs_grouped_plan {
   const double *gA = nullptr, *gB = nullptr;
   double *gC = nullptr;
   int64_t graph_launches = 0;  // kernels in the recorded graph
+  // also where creation fails; the caller makes sure that no run is in flight
+  ~qs_grouped_plan() {
+    if (exec) cudaGraphExecDestroy(exec);
+    split_plan_destroy(split);
+  }
 };
 
 namespace {
@@ -266,20 +271,25 @@ qs_status qs_grouped_plan_create(qs_ctx *ctx, const qs_pair_list *pairs, const q
     if (!p->main.pairs.empty()) {
       const GroupedPlan &m = p->main;
       const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.coff, &m.bldc, m.cplx, {});
+      // the lists before the digits, which may take what memory there is
+      auto lists = [&](bool tensor) {
+        const std::vector<TileDesc> tiles =
+            make_tiles(m.grp, m.bM, m.bN, m.coff, F64_TILE, F64_TILE, &m.bldc, &m.pairs, tensor ? &tl.on : nullptr);
+        p->lists.reset(new PlanLists);
+        const size_t op = p->lists->add(m.pairs), ot = p->lists->add(tiles), oc = p->lists->add(tl.checked);
+        p->lists->commit(c);
+        p->d_pairs = p->lists->at<PairDesc>(op);
+        p->d_tiles = p->lists->at<TileDesc>(ot);
+        p->d_checked = p->lists->at<TileDesc>(oc);
+        p->ntiles = (int64_t)tiles.size();
+        p->nchecked = tensor ? (int64_t)tl.checked.size() : 0;
+      };
+      lists(true);
       if (!tl.checked.empty()) {
         c->ensure_aux();
         p->split = f64_tensor_plan_create(c, tl, m.pairs, m.grp, m.bM, m.bN, m.coff, m.bldc, m.cplx, p->miss);
+        if (!p->split) lists(false);  // no room for the digits: every tile in FP64
       }
-      // every tile in FP64 when there is no room for the digits
-      const std::vector<TileDesc> tiles =
-          make_tiles(m.grp, m.bM, m.bN, m.coff, F64_TILE, F64_TILE, &m.bldc, &m.pairs, p->split ? &tl.on : nullptr);
-      p->ntiles = (int64_t)tiles.size();
-      if (p->split) p->nchecked = (int64_t)tl.checked.size();
-      const size_t op = p->lists.add(m.pairs), ot = p->lists.add(tiles), oc = p->lists.add(tl.checked);
-      p->lists.commit(c);
-      p->d_pairs = p->lists.at<PairDesc>(op);
-      p->d_tiles = p->lists.at<TileDesc>(ot);
-      p->d_checked = p->lists.at<TileDesc>(oc);
     }
   } else {
     fail(QS_ERR_ARG, "unknown precision mode %d", p->o.prec);
@@ -330,8 +340,6 @@ void qs_grouped_plan_destroy(qs_grouped_plan *p) {
     cudaSetDevice(p->ctx->device);
     cudaStreamSynchronize(p->ctx->stream);
   }
-  if (p->exec) cudaGraphExecDestroy(p->exec);
-  split_plan_destroy(p->split);
   delete p;
 }
 

@@ -62,8 +62,8 @@ SplitResult run_split_static(Ctx *ctx, const std::vector<PairDesc> &pairs,
 struct F64TensorList {
   std::vector<char> on;         // per block: computed by the tensor-core launch
   std::vector<int32_t> fbase;   // per block: first FP64 tile
-  std::vector<std::pair<int64_t, int64_t>> chunks;  // block ranges of one launch each
   std::vector<TileDesc> checked;  // the blocks as launch_gemm_f64 takes them
+  std::vector<int64_t> bytes;     // their digits (at most)
   int64_t ntiles = 0;  // FP64 tiles of the checked blocks
 };
 // The blocks of a list that the tensor-core launch takes (a property of the
@@ -74,8 +74,9 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
                               const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                               const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
                               const std::vector<char> &skip);
-// Runs them (strips and products); false when the device has no room for
-// their digits (nothing ran: the caller computes every tile in FP64).
+// Runs them (strips and products), in several launches where the digits are
+// many or room is short; false when the device has no room for the digits of one
+// block or for the lists (nothing ran: the caller computes every tile in FP64).
 bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                     const std::vector<int64_t> &grp, const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                     const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, const double *A,

@@ -1,0 +1,62 @@
+"""The plain FP64 path where device memory is short.  QS_ALLOC_LIMIT_MB refuses
+larger single allocations as if the device had no room for them."""
+import numpy as np
+import pytest
+
+from qspace_gb300.grouped import DeviceBatch, Packed
+
+U = 2.0 ** -53
+
+
+def _batch(sizes, seed=0):
+    rng = np.random.default_rng(seed)
+    m = lambda r, c: rng.standard_normal((r, c)) + 1j * rng.standard_normal((r, c))  # noqa: E731
+    A, B = [m(M, K) for M, N, K in sizes], [m(K, N) for M, N, K in sizes]
+    return DeviceBatch(Packed(A, B, rng.uniform(0.5, 1.0, len(sizes)))), A, B
+
+
+def _runs(db):
+    """Results of the one-shot call and of a plan's first and replayed run."""
+    db.run("fp64")
+    out = [[c.copy() for c in db.result()]]
+    plan = db.plan("fp64")
+    for _ in range(2):
+        db.dC.fill_(float("nan"))
+        db.torch.cuda.synchronize()
+        db.run_plan(plan)
+        out.append([c.copy() for c in db.result()])
+    plan.close()
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit", ["64", "16", "7"])
+def test_several_launches_give_the_same_bits(limit, monkeypatch):
+    """Digits of eight blocks, 6.3 MB each: in one launch where there is room,
+    else in several that share the memory."""
+    db, _, _ = _batch([(256, 256, 256)] * 8 + [(40, 50, 60), (5, 6, 7), (8, 8, 400)])
+    want = _runs(db)[0]
+    monkeypatch.setenv("QS_ALLOC_LIMIT_MB", limit)
+    from qspace_gb300 import Context
+    ctx = Context(0)  # no scratch of earlier calls
+    db.ctx = ctx
+    for got in _runs(db):
+        assert all(np.array_equal(c, w) for c, w in zip(got, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit", ["3", "0.2"])
+def test_no_room_for_a_block(limit, monkeypatch):
+    """Where one block's digits do not fit, the FP64 tiles compute the list, in
+    the one-shot call and from a plan."""
+    db, A, B = _batch([(256, 256, 256), (300, 40, 64), (70, 80, 90), (3, 4, 5)])
+    monkeypatch.setenv("QS_ALLOC_LIMIT_MB", limit)
+    from qspace_gb300 import Context
+    db.ctx = Context(0)
+    runs = _runs(db)
+    for a, b, f, *cs in zip(A, B, db.pk.afac, *runs):
+        r = (a * f).astype(np.clongdouble) @ b.astype(np.clongdouble)
+        s = (np.abs(a.real) + np.abs(a.imag)) @ (np.abs(b.real) + np.abs(b.imag))
+        for c in cs:
+            assert np.all(np.abs(c - r).astype(float) <= (2 * a.shape[1] + 2) * U * s)
+            assert np.array_equal(c, cs[0])
