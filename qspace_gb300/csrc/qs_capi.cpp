@@ -32,9 +32,12 @@ void dev_free(Ctx *ctx, void *p) {
 }
 
 cudaError_t pool_alloc(Ctx *ctx, void **p, size_t bytes) {
-  const char *limit = std::getenv("QS_ALLOC_LIMIT_MB");
-  if (limit && double(bytes) > std::atof(limit) * (1 << 20)) return cudaErrorMemoryAllocation;
+  if (bytes > ctx->alloc_limit) return cudaErrorMemoryAllocation;
   return cudaMallocAsync(p, bytes, ctx->stream);
+}
+
+Ctx::Ctx() {
+  if (const char *mb = std::getenv("QS_ALLOC_LIMIT_MB")) alloc_limit = (size_t)(std::atof(mb) * (1 << 20));
 }
 
 void *Ctx::ensure_scratch(size_t bytes) {

@@ -2026,6 +2026,10 @@ constexpr double F64T_WORK = 32768.0;
 // Digit bytes of one launch (blocks above it get a launch of their own), and
 // of a block that still takes this path.
 constexpr int64_t F64T_CHUNK_BYTES = int64_t(2) << 30, F64T_BLOCK_BYTES = int64_t(8) << 30;
+// Digits that a call leaves as the context's scratch for the next one; more go
+// back to the pool at its end (about 3 us a call), where every allocation of the
+// library finds them.
+constexpr int64_t F64T_KEEP_BYTES = int64_t(16) << 20;
 
 // Whether the tensor-core launch takes a block; `bytes` its digits (at most).
 static bool f64_tensor_takes(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1, int64_t M, int64_t N,
@@ -2149,6 +2153,7 @@ bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDes
   std::vector<SplitWork> ws;
   std::vector<std::unique_ptr<DevLists>> lists;
   std::vector<SplitDev> ds;
+  std::unique_ptr<DevLists> own;
   // every allocation before the first launch
   auto allocate = [&] {
     ds.clear();
@@ -2159,7 +2164,15 @@ bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDes
       ds.push_back(stage_split_work(ctx, w, *lists.back()));
       arena = std::max(arena, w.arena);
     }
-    uint8_t *digits = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)arena));
+    uint8_t *digits;
+    if (arena <= F64T_KEEP_BYTES || (size_t)arena <= ctx->scratch_bytes) {
+      digits = static_cast<uint8_t *>(ctx->ensure_scratch((size_t)arena));
+    } else {
+      own = std::make_unique<DevLists>();
+      const size_t o = own->space((size_t)arena);
+      own->commit(ctx);
+      digits = own->at<uint8_t>(o);
+    }
     for (SplitDev &d : ds) {
       d.arena = digits;
       d.miss = miss;

@@ -55,6 +55,10 @@ struct Ctx {
   int64_t launches = 0;
   // device error word for bounded waits inside kernels (0 = ok)
   int *d_err = nullptr;
+  Ctx();
+  // larger single allocations are refused as if the device had no room for them
+  // (QS_ALLOC_LIMIT_MB in the environment when the context is created)
+  size_t alloc_limit = SIZE_MAX;
   // pooled scratch (grown on demand, stream ordered)
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
@@ -336,8 +340,6 @@ inline void require_whole_elements(const double *A, const double *B, const doubl
 
 // ------------------------------------------------------ small utilities
 // Stream-ordered memory from the device's pool (qs_capi.cpp).
-// QS_ALLOC_LIMIT_MB in the environment refuses larger single allocations as if
-// the device had no room for them.
 cudaError_t pool_alloc(Ctx *ctx, void **p, size_t bytes);
 template <class T>
 T *dev_alloc(Ctx *ctx, size_t n) {

@@ -60,3 +60,47 @@ def test_no_room_for_a_block(limit, monkeypatch):
         for c in cs:
             assert np.all(np.abs(c - r).astype(float) <= (2 * a.shape[1] + 2) * U * s)
             assert np.array_equal(c, cs[0])
+
+
+def _pool_used(high=False):
+    """Bytes of the device's default pool in use (now, or at most since the
+    last call with high=True)."""
+    import ctypes
+    import glob
+    import os
+    import torch
+    torch.cuda.synchronize()
+    names = ["libcudart.so.13", "libcudart.so.12", "libcudart.so"]
+    names += glob.glob(os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "*", "lib", "libcudart.so*"))
+    names += glob.glob("/usr/local/cuda/lib64/libcudart.so*")
+    for n in names:
+        try:
+            rt = ctypes.CDLL(n)
+            break
+        except OSError:
+            pass
+    else:
+        pytest.skip("no CUDA runtime library")
+    pool, v = ctypes.c_void_p(), ctypes.c_uint64()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    # cudaMemPoolAttrUsedMemCurrent = 7, cudaMemPoolAttrUsedMemHigh = 8
+    assert rt.cudaMemPoolGetAttribute(pool, 8 if high else 7, ctypes.byref(v)) == 0
+    used = v.value
+    if high:
+        zero = ctypes.c_uint64(0)
+        assert rt.cudaMemPoolSetAttribute(pool, 8, ctypes.byref(zero)) == 0
+    return used
+
+
+@pytest.mark.gpu
+def test_digits_go_back_to_the_pool():
+    """A plain FP64 call leaves at most 16 MB of its digits with the context."""
+    from qspace_gb300 import Context
+    db, _, _ = _batch([(700, 600, 500), (900, 800, 300)])
+    db.ctx = Context(0)
+    db.ctx.sync()
+    before = _pool_used()
+    for _ in range(2):
+        db.run("fp64")
+        db.ctx.sync()
+        assert _pool_used() - before <= 17 << 20
