@@ -493,7 +493,12 @@ typedef struct {
   int32_t nslots;          /* concurrent requests on the device               */
   int32_t max_batch;       /* requests one slot runs in one grouped launch
                               (continuous batching); 0 = 16                  */
-  int64_t hbm_budget;      /* bytes of scratch+output the server may hold      */
+  int64_t hbm_budget;      /* bytes of scratch+output the server may hold,
+                              digits of plain FP64 requests included.  One
+                              whose output and copies fit but not all of its
+                              digits runs alone, with the digits that fit:
+                              in several launches, and blocks that do not fit
+                              by themselves through the FP64 tiles           */
 } qs_server_cfg;
 QS_EXPORT qs_status qs_server_create(qs_ctx *ctx, const qs_server_cfg *cfg, qs_server **out);
 QS_EXPORT void qs_server_destroy(qs_server *s);

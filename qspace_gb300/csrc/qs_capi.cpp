@@ -846,7 +846,8 @@ void contract_batch_core(Ctx *ctx, int n, const QMeta *const *Am, const double *
 }
 
 int64_t contract_footprint(const QMeta &Am, const QMeta &Bm, const char *ia, const char *ib,
-                           const qs_opts *opts) {
+                           const qs_opts *opts, int64_t *f64_digits) {
+  *f64_digits = 0;
   ContractPlan pl = plan_contract(Am, ia, Bm, ib, nullptr, 0);
   const int64_t es = pl.C.cplx ? 16 : 8;
   int64_t fp = pl.C.nelem * es * 2;  // result, and its permuted copy
@@ -861,6 +862,8 @@ int64_t contract_footprint(const QMeta &Am, const QMeta &Bm, const char *ia, con
       const int64_t rows = (d.M * cm + 127) / 128 * 128 + (d.N + 31) / 32 * 32;
       fp += rows * ((Kr + 31) / 32 * 32) * 2 * 8;
     }
+  } else if (!opts || opts->prec == QS_PREC_FP64) {
+    *f64_digits = f64_digit_bytes(pl.pairs, pl.grp, pl.blk_M, pl.blk_N, pl.C.offs, pl.C.cplx);
   }
   return fp;
 }

@@ -2056,7 +2056,7 @@ static bool f64_tensor_takes(const std::vector<PairDesc> &pairs, int64_t p0, int
 F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                               const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                               const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
-                              const std::vector<char> &skip) {
+                              const std::vector<char> &skip, int64_t limit) {
   F64TensorList tl;
   const int64_t nb = (int64_t)bM.size();
   tl.on.assign(nb, 0);
@@ -2064,7 +2064,9 @@ F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vec
   for (int64_t g = 0; g < nb; ++g) {
     const int64_t M = bM[g], N = bN[g], ldc = bldc ? (*bldc)[g] : std::max(bM[g], 1);
     int64_t bytes = 0;
-    if ((!skip.empty() && skip[g]) || !f64_tensor_takes(pairs, grp[g], grp[g + 1], M, N, ldc, cplx, bytes)) continue;
+    if ((!skip.empty() && skip[g]) || !f64_tensor_takes(pairs, grp[g], grp[g + 1], M, N, ldc, cplx, bytes) ||
+        bytes > limit)
+      continue;
     const int64_t tiles = ((M + F64_TILE - 1) / F64_TILE) * ((N + F64_TILE - 1) / F64_TILE);
     if (tl.ntiles + tiles > INT32_MAX / 4) continue;
     tl.on[g] = 1;
@@ -2119,16 +2121,40 @@ static void plan_f64_chunk(const F64TensorList &tl, std::pair<int64_t, int64_t> 
   plan_split(L.pairs, L.grp, L.bM, L.bN, L.coff, cplx, 0, 0, &L.bldc, w, 0, nullptr, nullptr, &fb);
 }
 
+int64_t f64_digit_bytes(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
+                        const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
+                        const std::vector<int64_t> &coff, bool cplx) {
+  // the blocks as run_f64 has them: no shallow ones, deep ones cut into parts,
+  // of which those with a few outputs have no digits
+  std::vector<char> rest(bM.size(), 1);
+  for (size_t b = 0; b < bM.size(); ++b) rest[b] = !is_shallow(pairs, grp[b], grp[b + 1]);
+  const BlockList R = select_blocks(pairs, grp, bM, bN, coff, nullptr, rest);
+  DeepSplit ds;
+  const bool deep = split_deep(R.pairs, R.grp, R.bM, R.bN, R.coff, &R.bldc, ds);
+  std::vector<char> skip(deep ? ds.bM.size() : R.bM.size(), 0);
+  if (deep)
+    for (size_t b = 0; b < skip.size(); ++b) skip[b] = ds.part[b] && (int64_t)ds.bM[b] * ds.bN[b] <= DOT_OUTPUTS;
+  const F64TensorList tl = deep ? plan_f64_tensor(ds.pairs, ds.grp, ds.bM, ds.bN, ds.coff, &ds.bldc, cplx, skip)
+                                : plan_f64_tensor(R.pairs, R.grp, R.bM, R.bN, R.coff, &R.bldc, cplx, skip);
+  int64_t sum = 0, most = 0;
+  for (int64_t x : tl.bytes) {
+    sum += x;
+    most = std::max(most, x);
+  }
+  return std::min(sum, std::max(most, F64T_CHUNK_BYTES));
+}
+
 // Plans the launches of a list and hands them to `allocate`, with fewer digits
-// a launch where that finds no room; false when the launches of single blocks
+// (at first `most`) a launch where that finds no room; false when the launches of single blocks
 // do not fit either.
 template <class F>
 static bool plan_f64_launches(const F64TensorList &tl, const std::vector<PairDesc> &pairs,
                               const std::vector<int64_t> &grp, const std::vector<int32_t> &bM,
                               const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,
-                              const std::vector<int32_t> *bldc, bool cplx, std::vector<SplitWork> &ws, F allocate) {
+                              const std::vector<int32_t> *bldc, bool cplx, int64_t most,
+                              std::vector<SplitWork> &ws, F allocate) {
   size_t tried = 0;
-  for (int64_t limit = F64T_CHUNK_BYTES; tried < tl.checked.size(); limit /= 4) {
+  for (int64_t limit = std::min(F64T_CHUNK_BYTES, most); tried < tl.checked.size(); limit /= 4) {
     const auto chunks = f64_chunks(tl, limit);
     if (chunks.size() == tried) continue;
     tried = chunks.size();
@@ -2178,7 +2204,7 @@ bool run_f64_tensor(Ctx *ctx, const F64TensorList &tl, const std::vector<PairDes
       d.miss = miss;
     }
   };
-  if (!plan_f64_launches(tl, pairs, grp, bM, bN, coff, bldc, cplx, ws, allocate)) return false;
+  if (!plan_f64_launches(tl, pairs, grp, bM, bN, coff, bldc, cplx, ctx->f64_digits, ws, allocate)) return false;
   for (size_t k = 0; k < ws.size(); ++k) launch_split(ctx, ws[k], cplx, ds[k], A, B, C, ctx->d_err, true, k == 0);
   return true;
 }
@@ -2259,7 +2285,7 @@ SplitPlanHandle *f64_tensor_plan_create(Ctx *ctx, const F64TensorList &tl, const
                                         const std::vector<int32_t> &bldc, bool cplx, MissList &miss) {
   std::unique_ptr<SplitPlanHandle> h(new SplitPlanHandle);
   h->cplx = cplx;
-  if (!plan_f64_launches(tl, pairs, grp, bM, bN, coff, &bldc, cplx, h->w, [&] { h->allocate(ctx, tl.ntiles); }))
+  if (!plan_f64_launches(tl, pairs, grp, bM, bN, coff, &bldc, cplx, ctx->f64_digits, h->w, [&] { h->allocate(ctx, tl.ntiles); }))
     return nullptr;
   miss = h->miss;
   return h.release();

@@ -144,7 +144,7 @@ void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int
       }
     if (small.size() < mm.size()) require_whole_elements(A, B, C, cplx);
     run_dot(ctx, pp, gg, mm, nn, cc, ll, small, A, B, C, cplx);
-    const F64TensorList tl = plan_f64_tensor(pp, gg, mm, nn, cc, ll, cplx, skip);
+    const F64TensorList tl = plan_f64_tensor(pp, gg, mm, nn, cc, ll, cplx, skip, ctx->f64_digits);
     const std::vector<char> dots = skip;
     for (size_t b = 0; b < mm.size(); ++b) skip[b] |= tl.on[b];
     std::vector<TileDesc> tiles = make_tiles(gg, mm, nn, cc, F64_TILE, F64_TILE, ll, &pp, &skip);

@@ -59,6 +59,9 @@ struct Ctx {
   // larger single allocations are refused as if the device had no room for them
   // (QS_ALLOC_LIMIT_MB in the environment when the context is created)
   size_t alloc_limit = SIZE_MAX;
+  // most digits that a plain FP64 launch may hold (the serving loop's budget);
+  // blocks with more are computed by the FP64 tiles
+  int64_t f64_digits = INT64_MAX;
   // pooled scratch (grown on demand, stream ordered)
   void *scratch = nullptr;
   size_t scratch_bytes = 0;

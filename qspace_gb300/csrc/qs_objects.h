@@ -40,9 +40,10 @@ void contract_batch_core(Ctx *ctx, int n, const QMeta *const *Am, const double *
                          const char *const *ib, const int32_t *const *perm, const int32_t *nperm,
                          const qs_opts *opts, std::vector<std::unique_ptr<qs_tensor>> &out);
 // Device bytes a contraction will hold while it runs (output, operand
-// copies, digit arena): the admission footprint of the serving loop.
+// copies, digit arena): the admission footprint of the serving loop.  The
+// digits of the plain FP64 path come in *f64_digits: it can do with fewer.
 int64_t contract_footprint(const QMeta &Am, const QMeta &Bm, const char *ia, const char *ib,
-                           const qs_opts *opts);
+                           const qs_opts *opts, int64_t *f64_digits);
 // eigQS of a device-resident rank-2 QSpace on ctx's stream: kept and
 // discarded eigenvectors as new tensors, optional host copies of the
 // eigenvalues / keep flags (sum of block sizes each), NK and Etrunc.

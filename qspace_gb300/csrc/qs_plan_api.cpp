@@ -270,7 +270,7 @@ qs_status qs_grouped_plan_create(qs_ctx *ctx, const qs_pair_list *pairs, const q
   } else if (p->o.prec == QS_PREC_FP64) {
     if (!p->main.pairs.empty()) {
       const GroupedPlan &m = p->main;
-      const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.coff, &m.bldc, m.cplx, {});
+      const F64TensorList tl = plan_f64_tensor(m.pairs, m.grp, m.bM, m.bN, m.coff, &m.bldc, m.cplx, {}, c->f64_digits);
       // the lists before the digits, which may take what memory there is
       auto lists = [&](bool tensor) {
         const std::vector<TileDesc> tiles =

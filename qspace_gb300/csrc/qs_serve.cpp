@@ -53,6 +53,7 @@ struct Request {
   cudaEvent_t ready = nullptr;
   Ctx *owner = nullptr;            // context whose stream orders the request and frees its results
   int64_t footprint = 0;
+  int64_t f64_digits = INT64_MAX;  // most digits a plain FP64 request may hold
   clk::time_point t_submit;
   enum State { QUEUED, RUNNING, DONE, FAILED, CANCELLED } state = QUEUED;
   qs_status status = QS_OK;
@@ -87,6 +88,7 @@ struct qs_server {
 
   static bool same_opts(const Request &a, const Request &b) {
     if (a.kind != Request::CONTRACT || b.kind != Request::CONTRACT) return false;  // eig requests run alone
+    if (a.f64_digits != INT64_MAX || b.f64_digits != INT64_MAX) return false;  // these too
     if (a.has_opts != b.has_opts) return false;
     if (!a.has_opts) return true;
     return a.opts.prec == b.opts.prec && a.opts.nslices == b.opts.nslices && a.opts.tol == b.opts.tol;
@@ -133,6 +135,7 @@ struct qs_server {
         for (auto &r : batch) r->state = Request::RUNNING;
       }
       const int n = (int)batch.size();
+      slot->f64_digits = batch[0]->f64_digits;
       std::vector<qs_status> st(n, QS_OK);
       std::vector<std::string> msg(n);
       std::vector<qs_tensor *> C(n, nullptr);
@@ -297,11 +300,20 @@ qs_status qs_server_submit_from(qs_server *s, qs_ctx *client, const qs_tensor *A
   // not in a worker
   (void)parse_ctr_idx(ia);
   (void)parse_ctr_idx(ib);
-  const int64_t fp = contract_footprint(A->meta, B->meta, ia, ib, opts);
+  int64_t digits = 0;
+  int64_t fp = contract_footprint(A->meta, B->meta, ia, ib, opts, &digits);
   if (fp > s->budget)
     fail(QS_ERR_OOM, "admission refused: request needs %lld bytes, budget is %lld", (long long)fp,
          (long long)s->budget);
   auto r = std::make_shared<Request>();
+  // the digits of a plain FP64 request count too; one that does not fit with all
+  // of them takes the whole budget and does with what is left of it
+  if (fp + digits > s->budget) {
+    r->f64_digits = s->budget - fp;
+    fp = s->budget;
+  } else {
+    fp += digits;
+  }
   r->A = A;
   r->B = B;
   r->ia = ia;

@@ -67,13 +67,18 @@ struct F64TensorList {
   int64_t ntiles = 0;  // FP64 tiles of the checked blocks
 };
 // The blocks of a list that the tensor-core launch takes (a property of the
-// block alone), except those marked in `skip`.  The list holds no shallow
-// blocks: the FP64 path computes all of them directly (run_shallow), which
-// takes complex buffers aligned to 8 bytes.
+// block and of `limit`, the most digits a launch may hold), except those marked
+// in `skip`.  The list holds no shallow blocks: the FP64 path computes all of
+// them directly (run_shallow), which takes complex buffers aligned to 8 bytes.
 F64TensorList plan_f64_tensor(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
                               const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
                               const std::vector<int64_t> &coff, const std::vector<int32_t> *bldc, bool cplx,
-                              const std::vector<char> &skip);
+                              const std::vector<char> &skip, int64_t limit = INT64_MAX);
+// Bytes of digits that the plain FP64 path holds at a time for a list (at
+// most), alone or as part of a longer one.
+int64_t f64_digit_bytes(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
+                        const std::vector<int32_t> &bM, const std::vector<int32_t> &bN,
+                        const std::vector<int64_t> &coff, bool cplx);
 // Runs them (strips and products), in several launches where the digits are
 // many or room is short; false when the device has no room for the digits of one
 // block or for the lists (nothing ran: the caller computes every tile in FP64).

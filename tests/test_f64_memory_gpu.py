@@ -104,3 +104,35 @@ def test_digits_go_back_to_the_pool():
         db.run("fp64")
         db.ctx.sync()
         assert _pool_used() - before <= 17 << 20
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("budget", [9, 14, 20, 40])
+@pytest.mark.parametrize("nblk,n", [(1, 700), (4, 350)])
+def test_serving_budget_covers_fp64_digits(nblk, n, budget):
+    """Plain FP64 requests whose result and copies fit the budget are served
+    within it: with all of their digits (17 MB here), with fewer at a time, or
+    by the FP64 tiles."""
+    from qspace_gb300 import Context, QSpace, contract_dev, upload
+    from qspace_gb300.serve import Server
+    rng = np.random.default_rng(5)
+    q = np.arange(nblk, dtype=np.int32).reshape(-1, 1)
+    a, b = ([rng.standard_normal((n, n)) for _ in range(nblk)] for _ in range(2))
+    ctx = Context(0)
+    A, B = upload(QSpace([q, q.copy()], a), ctx), upload(QSpace([q, q.copy()], b), ctx)
+    want = contract_dev(A, "2", B, "1", prec="fp64").download().data
+    ctx.sync()
+    with Server(nslots=2, hbm_budget=budget << 20, ctx=ctx) as srv:
+        before = _pool_used()
+        _pool_used(high=True)
+        tickets = [srv.submit(A, "2", B, "1") for _ in range(4)]
+        for t in tickets:
+            c, _ = srv.wait(t)
+            got = c.download().data
+            for x, y, r in zip(a, b, got):
+                assert np.all(np.abs(r - x @ y) <= 2 * n * U * (np.abs(x) @ np.abs(y)))
+            if budget == 40 or nblk == 4 and budget >= 14:
+                assert all(np.array_equal(r, w) for r, w in zip(got, want))
+            c.free()
+        results = 4 * 8 * nblk * n * n  # of requests that are done, not yet collected
+        assert _pool_used(high=True) - before <= (budget + 1 << 20) + results
