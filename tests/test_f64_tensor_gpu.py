@@ -410,3 +410,46 @@ def test_long_columns_of_c():
     db.ctx.sync()
     got = t.stack([db.dC[:2 * M], db.dC[2 * ldc:]]).cpu().numpy().view(np.complex128).T
     _check([got], _reference(ops, [1.0], [0]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("scale", [(1e200, 1e200, 1e-300), (1e-300, 1e200, 1e200), (1e-200, 1e-200, 1e250),
+                                   (1e250, 1e-200, 1e-200), (1.0, 1e-315, 1e300), (1e300, 1e-315, 1.0)])
+def test_shallow_factors_scale_the_sum(scale, cplx):
+    """x f leaves the normal numbers, on some lines or all, where f (x y) does
+    not: either side long, lines past the first of a thread, plans."""
+    rng = np.random.default_rng(23)
+    sa, f, sb = scale
+    ops, afac, blk, trans = [], [], [], []
+    for g, (M, N, K) in enumerate([(1, 1, 1), (700, 3, 4), (3, 700, 4), (5, 600, 1), (300, 33, 5), (129, 2, 3)]):
+        a, b = _ops(rng, M, N, K, cplx)
+        a[::3] *= sa
+        b[:, ::2] *= sb
+        ops += [(a, b), tuple(x * 1e-140 for x in _ops(rng, M, N, 2, cplx))]
+        afac += [f, -0.31]
+        blk += [g, g]
+        trans += [int(t) for t in rng.integers(0, 16 if cplx else 4, 2)]
+    db = _batch(ops, afac, blk, trans)
+    db.run("fp64")
+    got = [c.copy() for c in db.result()]
+    wide = np.clongdouble if cplx else np.longdouble
+    for g, c in enumerate(got):
+        r, s, n = 0, 0, 1
+        for (a, b), w in zip(ops[2 * g:2 * g + 2], afac[2 * g:2 * g + 2]):
+            w = np.longdouble(w)
+            r = r + w * (a.astype(wide) @ b.astype(wide))
+            m = [np.abs(x).astype(np.longdouble) for x in (a.real, a.imag, b.real, b.imag)]
+            s = s + abs(w) * ((m[0] + m[1]) @ (m[2] + m[3]))
+            n += a.shape[1] * (2 if cplx else 1) + 1
+        d = c - r
+        err = np.maximum(np.abs(d.real), np.abs(d.imag))
+        fits = s < 1e307  # others overflow
+        assert np.all((err <= n * U * s + 1e-320)[fits]), float(np.max((err / s)[fits]))
+    plan = db.plan("fp64")
+    db.dC.fill_(float("nan"))
+    db.torch.cuda.synchronize()
+    db.run_plan(plan)
+    for c, w in zip(db.result(), got):
+        assert np.array_equal(c, w)
+    plan.close()
