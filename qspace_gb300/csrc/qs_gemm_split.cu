@@ -821,14 +821,6 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
                    smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
-  uint32_t r[4];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
-}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
   uint32_t r[8];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -1469,14 +1461,6 @@ DigitPlan choose_digits_for(const std::vector<PairDesc> &pairs, const std::vecto
   }
   if (!best.nslices) fail(QS_ERR_NUMERIC, "no digit plan for tol=%g, slices=%d", tol, forced_slices);
   return best;
-}
-
-DigitPlan choose_digits(int64_t kreal, double tol, int forced_slices) {
-  std::vector<PairDesc> one(1);
-  one[0].M = TMS;
-  one[0].N = TNS;
-  one[0].K = (int32_t)std::max<int64_t>(kreal, 1);
-  return choose_digits_for(one, {0, 1}, {TMS}, {TNS}, 1, tol, forced_slices);
 }
 
 // Digits of the FP64-grade launches: 7 x 8 bits and the magnitude plane fill

@@ -17,14 +17,11 @@ struct SplitResult {
   int64_t ntiles = 0;
 };
 
-// Digit plan for a maximal accumulated depth `kreal` (real terms summed into
-// one output element) and a target relative error.
 struct DigitPlan {
   int bits;    // bits per digit (the leading digit carries bits+1)
   int nslices; // digits per operand
   double err_bound;
 };
-DigitPlan choose_digits(int64_t kreal, double tol, int forced_slices);
 // The digit plan the split path picks for a grouped product (cm = 2 for
 // complex), optionally with the digit count and/or width forced.
 DigitPlan choose_digits_for(const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
