@@ -10,7 +10,7 @@ the persistent grouped launch replayed as a CUDA graph -- the way a DMRG
 or NRG driver repeats products over one block structure.  The one-shot call
 (qs_grouped_gemm, planned every call) is reported beside it.  Metric:
 FP64-equivalent TFLOP/s (8 M N K per complex pair) at <= 1e-12 relative
-error; the split BF16 path is the headline, the plain FP64 path is reported
+error; the split FP16 path is the headline, the plain FP64 path is reported
 beside it; per-step latency p50/p99.  Inputs (2.8 GB) are larger than L2,
 so no flush is needed.
 
@@ -170,7 +170,7 @@ GEMM_DRAM_WRITE_PER_OUTPUT_BYTE = 175.655168e6 / 231684512
 
 
 def split_arena_bytes(pk, S: int) -> float:
-    """Bytes of the BF16 digit arena of the batch: 128 x 32 A tiles and 32 x 32
+    """Bytes of the FP16 digit arena of the batch: 128 x 32 A tiles and 32 x 32
     B tiles of the real form (2M x 2K and 2K x N per complex pair with A
     duplicated, M x 2K and 2K x 2N with B duplicated), S digits, after the
     planner's choice of layout per output block (plain, C^T, and for complex
@@ -528,7 +528,7 @@ def main():
     bf16_peak, hbm_peak, peak_kind = measured_peaks()
     if a.prec == "split":
         S = st.get("nslices", 0)
-        # BF16 digit products actually required (no tile padding): S(S+1)/2
+        # FP16 digit products actually required (no tile padding): S(S+1)/2
         # real products of (2M) x (2K) x N per complex pair
         digit_flops = S * (S + 1) / 2 * float(np.sum(2.0 * (2 * pk.M.astype(float)) * pk.N * (2 * pk.K.astype(float))))
         achieved = digit_flops / (gemm_ms * 1e-3) / 1e12
@@ -538,7 +538,7 @@ def main():
                 "unit": "TFLOP/s", "frac": achieved / bf16_peak, "traffic": traffic,
                 "traffic_note": "bytes per launch, scaled from an ncu capture of the 300-pair case",
                 "peak_kind": f"bf16 dense, {peak_kind}", "kernel_ms": gemm_ms, "prep_ms": prep_ms,
-                "algorithmic": f"{S}x{S + 1}/2 BF16 digit products of the real 2M x 2K x N form per pair"}
+                "algorithmic": f"{S}x{S + 1}/2 FP16 digit products of the real 2M x 2K x N form per pair"}
     else:
         achieved = flops / (gemm_ms * 1e-3) / 1e12
         roof = {"bound": "fp64", "kernel": "gemm_f64_kernel", "achieved": achieved, "peak": None,
@@ -864,7 +864,7 @@ def main():
                 "unit": "TFLOP/s", "n_gpus": ws, "steps": a.steps,
                 "warmup": a.warmup, "ms_per_step": ms, "higher_is_better": True,
                 "scaling": "strong" if a.shard else "weak",
-                "vs_baseline": None, "dtype": "f64 (split: bf16 digits, fp32 exact accumulation)",
+                "vs_baseline": None, "dtype": "f64 (split: fp16 digits, fp32 exact accumulation)",
                 "data": "synthetic (seeded normal)",
                 "config": {"workload": WORKLOAD, "npairs": a.npairs, "seed": a.seed, "prec": a.prec,
                            "nslices": st.get("nslices"), "digit_bits": st.get("digit_bits"),

@@ -58,7 +58,15 @@ typedef enum {
 } qs_status;
 
 typedef enum {
-  QS_PREC_FP64 = 0,   /* plain FP64 (DFMA) path: the drop-in                   */
+  QS_PREC_FP64 = 0,   /* plain FP64 path, the drop-in: every output within the
+                         error bound of an FP64 dot product, K u sum |f a b|
+                         (u = 2^-53, K real terms; one rounding more for the
+                         factor f), whatever the operands hold.
+                         Larger blocks run on the tensor cores with 56-bit
+                         digits (fixed point below the largest entry of a row
+                         of op(A) or column of op(B)); outputs that this does
+                         not serve, by a bound per output, and all other
+                         blocks by FP64 multiply-adds                          */
   QS_PREC_SPLIT = 1   /* FP64 sliced into FP16 digits, tcgen05 products with
                          exact FP32 accumulation, compensated recombination   */
 } qs_prec;
@@ -255,7 +263,14 @@ QS_EXPORT qs_status qs_permute_dev(qs_ctx *ctx, const qs_tensor *A, const int32_
  * tiles would mostly be padding, e.g. M = 1); a block with a summed depth of
  * thousands and few output tiles is cut along its depth into parts summed in
  * a fixed order (parts of at most 64 outputs reduced in FP64); every other
- * block runs through the grouped tiles of the chosen precision. */
+ * block runs through the grouped tiles of the chosen precision.  One thing
+ * else can change an FP64 result's last bits: where the device has no room
+ * for the digits of a list's largest block by itself (up to 8 GiB; lists with
+ * more digits than that, or than there is room for, run in several launches
+ * with the same bits), FP64 tiles compute the whole list, more slowly and
+ * within the same error bound.
+ * Complex buffers start at a multiple of 16 bytes; blocks computed directly
+ * take any multiple of 8, others are refused (QS_ERR_ARG) before a launch. */
 typedef struct {
   int64_t npairs;
   const int32_t *M, *N, *K;
@@ -282,8 +297,8 @@ QS_EXPORT qs_status qs_grouped_gemm_host(qs_ctx *ctx, const qs_pair_list *pairs,
 
 /* ------------------------------------------------ reusable grouped plans
  * No reference counterpart (the reference plans every contraction anew).  A
- * plan validates a pair list once, keeps its work lists and digit arena on
- * the device, and records its launch sequence as a CUDA graph on the first
+ * plan validates a pair list once, keeps its work lists and digits (split and
+ * FP64 plans) on the device until it is destroyed, and records its launch sequence as a CUDA graph on the first
  * run; later runs with the same A, B, C replay the graph (other pointers
  * record it again).  Repeated products over one block structure -- the
  * Davidson iterations of a DMRG site update, the steps of an NRG run --

@@ -2,7 +2,7 @@
 
 A drop-in for QSpace's contractQS / permuteQS numerical core (block-sparse
 contraction with exact label bookkeeping) with a plain FP64 path and a
-split-precision BF16 tensor-core path; eigQS / svdQS / orthoQS over block
+split-precision FP16 tensor-core path; eigQS / svdQS / orthoQS over block
 eig/SVD on the GPU; a serving loop.
 The numerical work runs in libqsgpu.so (CUDA for sm_103a) behind the C-ABI
 of include/qsgpu.h.

@@ -854,7 +854,7 @@ int64_t contract_footprint(const QMeta &Am, const QMeta &Bm, const char *ia, con
   if (pl.la.permute || (pl.C.cplx && !Am.cplx)) fp += Am.nelem * es * 2;
   if (pl.lb.permute || (pl.C.cplx && !Bm.cplx)) fp += Bm.nelem * es * 2;
   if (opts && opts->prec == QS_PREC_SPLIT) {
-    // at most 8 BF16 digits of every pair operand in the real form (2M x 2K
+    // at most 8 FP16 digits of every pair operand in the real form (2M x 2K
     // and 2K x N when complex), padded to 128 x 32 / 32 x 32 tiles
     const int64_t cm = pl.C.cplx ? 2 : 1;
     for (const PairDesc &d : pl.pairs) {

@@ -12,7 +12,8 @@
 //    and cut into S balanced signed digits of b bits,
 //    N = sum_t d_t 2^(b(S-1-t)), |d_0| <= 2^b, |d_t| <= 2^(b-1).
 //    The digits are small integers, exact in FP16.  The cut uses integer
-//    operations on the FP64 bit pattern only (GB300's FP64 pipe is narrow).
+//    operations on the FP64 bit pattern, and one FP64 multiply-add an entry
+//    for 8-bit digits of at most 48 bits.
 //  * The product of the two digit expansions is
 //      sum_k x_ik y_kj = 2^(E_i+F_j-2b) sum_g 2^(-bg) acc_g,
 //      acc_g = sum_k sum_{t+u=g} d_t(ik) d'_u(kj),   g = 0..S-1
@@ -30,12 +31,12 @@
 //    integer product (53 x 53 bits) before rounding, so pairs with different
 //    factors share the accumulators.
 //  * The epilogue reads the S accumulators from TMEM, combines them in int64
-//    fixed point, and assembles the FP64 result with integer bit operations
-//    (scale 2^(E_i+F_j-2b), round to nearest even): no FP64 instruction, as
-//    the FP64 pipe of GB300 is narrow.  Partial sums of later accumulator
-//    chunks are added exactly as int64 in the output slot.  One CTA owns one
-//    128x32 output tile at a time and sums the block pairs in plan order:
-//    deterministic, no atomics.
+//    fixed point over all accumulator chunks of the block, and converts the
+//    sum once (int64 to FP64, round to nearest even) with an integer exponent
+//    add for the scale 2^(E_i+F_j-2b): GB300's FP64 pipe is narrow.  One CTA
+//    owns one 128x32 output tile at a time and sums the block pairs in plan
+//    order: the result is deterministic (atomics only list outputs that the
+//    FP64-grade launch leaves to the FP64 kernel, not their values).
 //
 // Data movement: a slicing kernel writes the digits of every pair operand once
 // into an HBM arena, pre-tiled in the tcgen05 K-major, no-swizzle core-matrix
@@ -831,13 +832,12 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Recombination without the FP64 pipe.  The S accumulators hold exact
+// Recombination.  The S accumulators hold exact
 // integers (|acc_g| <= 2^24); their weighted sum
 //   V = sum_g acc_g 2^(b(S-1-g) - r)
 // is formed in 64-bit fixed point (r low bits of the smallest groups are
 // rounded away so that V and the sum over accumulator chunks keep headroom),
-// then turned into an FP64 value V * 2^scale by integer bit assembly (round
-// to nearest even).
+// then turned into an FP64 value V * 2^scale (fixed_to_double).
 // Wrapping 32 x 32 -> 64-bit multiply-add: acc + (int64)a * m (mod 2^64).
 __device__ __forceinline__ unsigned long long mad_wide(int a, int m, unsigned long long acc) {
   unsigned long long d;
@@ -1874,7 +1874,7 @@ SplitResult run_split(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::v
       ds.place((int64_t)(reinterpret_cast<intptr_t>(T) - reinterpret_cast<intptr_t>(C)) / eb);
       d_red = dev_upload(ctx, ds.red);
       // parts with a few outputs: one CTA per output element in FP64
-      // (run_dot; the tiles would compute 4096 outputs for each); the rest
+      // (run_dot; a tile would compute 4096 outputs for each); the rest
       // through the split path
       std::vector<char> sel(ds.bM.size(), 1);
       std::vector<int64_t> small;

@@ -25,9 +25,9 @@ struct GroupedPlan {
 // access is checked against them.
 GroupedPlan grouped_plan(const qs_pair_list *pl, int64_t a_elems, int64_t b_elems, int64_t c_elems);
 
-// The plain FP64 grouped product of a list (tensor cores with an FP64 net, FP64 tiles): shallow output
-// blocks computed directly (run_shallow), deep ones cut along their depth and
-// summed in part order (split_deep).  Pairs of blocks computed directly may
+// The plain FP64 grouped product of a list (tensor cores with an FP64 net, FP64
+// tiles): shallow output blocks computed directly (run_shallow), deep ones cut
+// along their depth and summed in part order (split_deep).  Pairs of blocks computed directly may
 // read their operands through views (va / vb, one per pair).
 void run_f64(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,
              const std::vector<int32_t> &bM, const std::vector<int32_t> &bN, const std::vector<int64_t> &coff,

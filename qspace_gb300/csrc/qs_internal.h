@@ -189,8 +189,8 @@ void launch_reduce_parts(Ctx *ctx, const DeepReduce *d_red, int64_t nred, const 
 // Shallow output blocks: a summed depth of at most SHALLOW_K (applying a
 // site operator over a leg of dimension 1 or 2, an outer product).  Tiled
 // products would pad the depth to a full k-block and pay the epilogue per
-// tile; these blocks are computed directly, one thread per output element,
-// in FP64 (exact products, summed in pair and k order).
+// tile; these blocks are computed directly in FP64 (exact products, summed in
+// pair and k order).
 constexpr int64_t SHALLOW_K = 8;
 bool is_shallow(const std::vector<PairDesc> &pairs, int64_t p0, int64_t p1);
 // Whether the direct FP64 computation of a shallow block is estimated to be
@@ -207,9 +207,8 @@ void run_shallow(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector
                  const std::vector<int32_t> *bldc, const std::vector<int64_t> &blocks, const double *A,
                  const double *B, double *C, bool cplx, const std::vector<OperandView> *va = nullptr,
                  const std::vector<OperandView> *vb = nullptr);
-// Parts of deep output blocks with at most DOT_OUTPUTS elements on the FP64
-// path: one CTA per output element reduces over the part's pairs and depth
-// (a fixed partition and tree order); 64 x 64 tiles would compute 4096
+// Parts of deep output blocks with at most DOT_OUTPUTS elements: one CTA per output element reduces over the part's pairs and depth
+// (a fixed partition and tree order); 32 x 32 tiles would compute 1024
 // outputs for each of them.
 constexpr int64_t DOT_OUTPUTS = 64;
 void run_dot(Ctx *ctx, const std::vector<PairDesc> &pairs, const std::vector<int64_t> &grp,

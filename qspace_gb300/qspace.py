@@ -252,7 +252,7 @@ def contractQS(A, ia=None, B: QSpace | None = None, ib=None, perm=None, *, prec:
     """C = contractQS(A, ia, B, ib [,perm]) on the GPU (host buffers in/out).
 
     ``ia``/``ib``: '12*' style strings or 1-based sequences; ``perm`` 1-based.
-    ``prec``: 'fp64' (plain drop-in) or 'split' (BF16 digits on tcgen05).
+    ``prec``: 'fp64' (plain drop-in) or 'split' (FP16 digits on tcgen05).
 
     Cell form ``contractQS([X0, X1, '*', X2, ...] [, perm])``: contraction
     over matching itags, right to left (Source/contractQS.cc:634-808); a '*'
