@@ -74,8 +74,8 @@ __global__ void reduce_parts_kernel(const DeepReduce *__restrict__ red, const do
 // the terms in shared memory, once per CTA (4 blocks of 900 x 900 x 8 with
 // factors: 72 us when it scaled each thread's elements, 56 us here).  Applying an MPO tensor
 // over a leg of dimension 3 (12 million outputs, up to 3 terms of 3): 190 us
-// with one thread per output and a permuted copy, 140 us here, 73 us of it the
-// FP64 pipe's.
+// with one thread per output and a permuted copy, 144 us here (caches cold), 73 us
+// of it the FP64 pipe's.
 struct ShallowTask {
   int64_t c_off;
   int32_t p0, p1, M, N, ldc;

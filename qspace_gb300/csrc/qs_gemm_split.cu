@@ -2002,9 +2002,9 @@ std::vector<int> split_candidate_bits(double tol, int forced_slices) {
 // multiply-adds, which take the narrow FP64 pipe (about 2 multiply-adds per
 // clock and SM) 9 us in one tile; the three launches take about 25 us in sum
 // whatever the block.  Measured, FP64 tiles against this path: 300 complex
-// products of 8..1024 per side 23.1 -> 1.71 ms (15.6 TFLOP/s of FP64 work;
-// error against a 64-bit product 1.2e-15 -> 6.7e-16), 64 real blocks of
-// 4..96 105 -> 77 us.
+// products of 8..1024 per side 23.1 -> 1.25 ms (21.4 TFLOP/s of FP64 work;
+// error against a 64-bit product 1.2e-15 -> 7.0e-16), 64 real blocks of
+// 4..96 105 -> 53..60 us.
 constexpr int64_t F64T_DEPTH = 16, F64T_MAX_DEPTH = 1 << 20;
 constexpr double F64T_WORK = 32768.0;
 // Digit bytes of one launch (blocks above it get a launch of their own), and
