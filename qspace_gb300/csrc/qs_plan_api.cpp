@@ -82,8 +82,6 @@ struct qs_grouped_plan {
 namespace {
 
 void launch_direct(qs_grouped_plan *p, const double *A, const double *B, double *C) {
-  if (!p->main.pairs.empty())
-    require_whole_elements(A, B, p->o.prec == QS_PREC_SPLIT ? nullptr : C, p->g.cplx);
   shallow_launch(p->ctx, p->shallow, A, B, C);
   if (p->main.pairs.empty()) return;
   if (p->o.prec == QS_PREC_SPLIT)
@@ -306,6 +304,8 @@ qs_status qs_grouped_plan_run(qs_grouped_plan *p, const double *A, const double 
   QS_CUDA(cudaSetDevice(c->device));
   const int64_t l0 = c->launches;
   if (!p->g.pairs.empty()) {
+    if (!p->main.pairs.empty())
+      require_whole_elements(A, B, p->o.prec == QS_PREC_SPLIT ? nullptr : C, p->g.cplx);
     if (p->tune_pending) autotune(p, A, B, C);
     if (p->o.flags & QS_FLAG_NO_GRAPH) {
       launch_direct(p, A, B, C);

@@ -453,3 +453,24 @@ def test_shallow_factors_scale_the_sum(scale, cplx):
     for c, w in zip(db.result(), got):
         assert np.array_equal(c, w)
     plan.close()
+
+
+@pytest.mark.gpu
+def test_misaligned_blocks_are_refused_before_tuning():
+    """A plan that times its digit widths on the first run looks at the buffers
+    before that, and runs once they are aligned."""
+    rng = np.random.default_rng(31)
+    ops = [_ops(rng, 43, 41, 59, True), _ops(rng, 4, 6, 2, True)]
+    db = _batch(ops, [1.0, 0.5], [0, 1], [0, 0])
+    aligned = db.dA, db.dB, db.dC
+    plan = db.plan("split", autotune=True)
+    _shifted(db, 1)
+    n0 = db.ctx.launches
+    with pytest.raises(QSError, match="aligned to 16"):
+        db.run_plan(plan)
+    assert db.ctx.launches == n0
+    db.dA, db.dB, db.dC = aligned
+    db.run_plan(plan)
+    for c, (r, s, n) in zip(db.result(), _reference(ops, [1.0, 0.5], [0, 1])):
+        assert np.linalg.norm((c - r).astype(complex)) <= 1e-12 * np.linalg.norm(s)
+    plan.close()
