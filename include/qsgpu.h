@@ -61,7 +61,8 @@ typedef enum {
   QS_PREC_FP64 = 0,   /* plain FP64 path, the drop-in: every output within the
                          error bound of an FP64 dot product, K u sum |f a b|
                          (u = 2^-53, K real terms; one rounding more for the
-                         factor f), whatever the operands hold.
+                         factor f), whatever the operands hold, as long as f a
+                         is an ordinary number.
                          Larger blocks run on the tensor cores with 56-bit
                          digits (fixed point below the largest entry of a row
                          of op(A) or column of op(B)); outputs that this does
